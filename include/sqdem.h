@@ -104,15 +104,16 @@ typedef struct {
   long long steps;            /* timesteps executed */
   long long evals_fp32;       /* Disfunction evaluations on the FP32 pipes (double-float, mixed form) */
   long long evals_fp64;       /* Disfunction evaluations in FP64 */
-  long long lm_rounds_max;    /* longest contact, in evaluation rounds of the LM kernel
-                                 (the critical path of the contact stage), max over steps */
+  long long lm_rounds_max;    /* longest contact among those searched one per warp, in its rounds of up
+                                 to six evaluations (the critical path of the contact stage), max over
+                                 steps */
   long long fallback_fp64;    /* mixed form: searches deferred to the FP64 kernel (a decision
                                  inside its rounding band, itmax reached, or an evaluation it does
                                  not reproduce) */
   long long lm_rounds_max_ff; /* mixed form: longest search in rounds of the double-float kernel
                                  (lm_rounds_max: of the FP64 kernel) */
-  long long long_queue;       /* searches of 32+ iterations at the previous step, queued for the
-                                 FP64 kernel's long-search handling (both forms) */
+  long long long_queue;       /* searches that ran long at the previous step (mixed form: 32+
+                                 iterations; FP64 form: 8+, in a batch 16+), run one per warp in FP64 */
 } sqdem_report;
 
 /* Record layouts shared with the CPU oracle (doubles per record). */
@@ -208,11 +209,12 @@ sqdem_status sqdem_put_scalars(sqdem_ctx* ctx, const double* in9);
  * the step then writes only the history the next step needs. */
 sqdem_status sqdem_set_record_full(sqdem_ctx* ctx, int on);
 
-/* Schedule of the Levenberg-Marquardt evaluations (no counterpart in the reference, which
- * runs one search per thread).  on = 1 (default): once the contact queue is drained, lanes
- * without a contact evaluate the points the searches still running in their warp will ask
- * for next; on = 0: every lane evaluates only its own search's point.  Results are identical
- * bit for bit; only the time of the longest searches changes. */
+/* Schedule of the search evaluations of the double-float and Nelder-Mead kernels (no counterpart
+ * in the reference, which runs one search per thread).  on = 1 (default): once the contact queue is
+ * drained, lanes without a contact evaluate the points the searches still running in their warp
+ * will ask for next; on = 0: every lane evaluates only its own search's point.  Results are
+ * identical bit for bit; only the time of the longest searches changes.  (The FP64
+ * Levenberg-Marquardt searches have one schedule.) */
 sqdem_status sqdem_set_lm_spread(sqdem_ctx* ctx, int on);
 
 /* Periodic-boundary correction, off by default (the reference's behaviour).  For a contact
@@ -225,9 +227,9 @@ sqdem_status sqdem_set_lm_spread(sqdem_ctx* ctx, int on);
 sqdem_status sqdem_set_periodic_fix(sqdem_ctx* ctx, int on);
 
 /* Device time (ms, summed over the steps of the last sqdem_step call made with use_graph = 0,
- * CUDA events on the context stream) of the contact search kernel (k_contacts_lm, or the mixed
- * form's double-float k_contacts_lm_ff) and of the mixed form's FP64 fallback kernel (0 for the
- * FP64 form).  Linear contact model only (0, 0 otherwise).  No counterpart in the reference
+ * CUDA events on the context stream) of the contact searches (the FP64 form's launches, or the mixed
+ * form's double-float ones) and of what the mixed form then waits for in FP64, the long searches
+ * that run beside them and the deferred ones (0 for the FP64 form).  Linear contact model only (0, 0 otherwise).  No counterpart in the reference
  * (per-kernel timing of what the reference times per engine with timing.stats). */
 sqdem_status sqdem_search_times(sqdem_ctx* ctx, double* out2);
 

@@ -64,7 +64,14 @@ enum : unsigned {
 // that took at least 4 iterations first, so that the longest searches start first.
 static const unsigned F_ITERS_SHIFT = 20, F_ITERS_MASK = 15u << 20;
 static const unsigned LONG_ITERS_BUCKET = 3;   // iterations >= 4
-static const unsigned VLONG_ITERS_BUCKET = 6;  // iterations >= 32: the searches that bound the kernel
+// Iterations at the last step (as bit length) from which a search goes to the long-search queue, and
+// from which it goes to that queue's front.  Mixed form: 32 and 64 (restarted) iterations: these run
+// in FP64, where the results are held to FP64's own.  FP64 form: 8 and 32: a warp each beside the
+// rounds (43,011 particles: 6.3 ms a step from 8, 6.6 from 16, 7.1 from 32); in a batch 16, since the
+// other specimens fill the FP64 pipe and a warp per search is three times the work of the rounds
+// (32 specimens of 300-4,000 particles: 13.6 ms for two steps from 16, 14.8 from 8).
+static const int LONG_BUCKET_MIXED = 6, LONG_BUCKET_FP64 = 4, LONG_BUCKET_BATCH = 5;
+static const int LONG_FRONT_MIXED = 7, LONG_FRONT_FP64 = 6;
 __device__ __forceinline__ unsigned itersBucket(int iters) { return iters > 0 ? min(15u, 32u - __clz((unsigned)iters)) : 0u; }
 enum { KIND_SQ = 0, KIND_WALL = 1 };
 static const unsigned DOF_ALL = 63u;
@@ -76,6 +83,7 @@ struct Params {
   int contactModel;   // SQDEM_CONTACT_LINEAR or SQDEM_CONTACT_HERTZ_MINDLIN
   int periodicFix;    // sqdem_set_periodic_fix: torque arm and relative velocity of image contacts
   int vlongBucket;    // iteration bucket from which a search goes to the long-search queue
+  int vlongFront;     // and from which to that queue's front
 };
 
 enum { E_NAN_NORMAL = 0, E_NAN_FORCE, E_LM_CALLS, E_LM_ITERS, E_LM_MAX, E_OVERFLOW, E_COLLIDER_RUNS, E_STEPS, E_EVAL32, E_EVAL64, E_ROUNDS_MAX,
@@ -107,8 +115,8 @@ struct SceneState {
   int runCollider, initSort, newtonRan, maxDispCode;
   int P, Pnew, nWW, overflowRun;
   int lmCount, lmHead;
-  int vlCount, vlHead;   // long-search queue: fbQueue[0, vlCount), filled by pass 1
-  int fbCount, fbHead;   // searches the mixed form deferred to FP64: fbQueue[vlCount, vlCount + fbCount)
+  int vlCount, vlHead;   // long-search queue, from the front of fbQueue: the longest at the last step
+  int fbCount, fbHead;   // searches the mixed form deferred to FP64 (deferQueue)
   int nmFin;   // Hertz-Mindlin searches that ended touching, for the finish pass
   int nmShort; // searches queued from the back of the queue (expected short)
   int numReinit; long long colliderRuns;
@@ -119,6 +127,14 @@ struct SceneState {
   double hSize[9], trsf[9], velGrad[9], nextVelGrad[9], prevVelGrad[9], dVelGrad[9], dtPrevVelGrad[9];
   double cellSize[3], prevCellSize[3], prevRunCellSize[3], cellTerm;
   unsigned long long err[E_NUM];
+};
+
+// Queue counters outside SceneState, whose layout the snapshots hold.
+static const int WAVE_MAX_ROUNDS = 32;
+struct QueueState {
+  int vl2Count;   // long-search queue, from the back of fbQueue: fewer iterations than those at its front
+  // FP64 rounds: entries of each round's lists, of the finish list, and the last list's head
+  int nT[WAVE_MAX_ROUNDS + 1], nP[WAVE_MAX_ROUNDS + 1], nF, tailHead;
 };
 
 // Contact table, structure of arrays (one set per buffer).
@@ -137,7 +153,7 @@ struct Table {
 
 struct Dev {
   int N, W, Pcap, Gmax, MAXC, NP;   // NP = particles
-  Params* prm; SceneState* S;
+  Params* prm; SceneState* S; QueueState* Q;
   // bodies
   double4 *pos, *ori, *vel, *angVel, *angMom, *inertia, *shpA, *shpB;   // shpA (rx,ry,rz,rmax) shpB (e1,e2,-,-)
   double* mass; int4* info;  // info: kind, mat, isSphere, wall axis | (sense+1)<<4
@@ -156,7 +172,9 @@ struct Dev {
   int* wCount; int* wList; int* wBlk;
   int2* ww;
   int* lmQueue; int qCap;   // work queue of the contact searches and its capacity
-  int* fbQueue;             // mixed form: searches deferred to the FP64 kernel (capacity Pcap)
+  int* fbQueue;             // long-search queue, two-ended (capacity Pcap)
+  int* deferQueue;          // mixed form: searches deferred to FP64 (capacity Pcap)
+  int *waveT0, *waveT1, *waveP, *waveF;   // FP64 rounds: lists of table-B slots (capacity Pcap)
   FFShape* bodyFF;          // mixed form: double-float shape and rotation of each body, this step
   // grid
   int* bodyCell; int* cellCount; int* cellStart; int* cellFill; int* cellBodies;
@@ -295,7 +313,7 @@ __global__ void k_scan_apply(const int* __restrict__ in, int n, const int* __res
 __global__ void k_gate(Dev d) {
   SceneState& S = *d.S;
   S.skip = (S.haltAt >= 0 && S.iter >= S.haltAt) ? 1 : 0;
-  if (S.skip) { S.runCollider = 0; S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0; return; }
+  if (S.skip) { S.runCollider = 0; S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0; *d.Q = QueueState(); return; }
   if (S.newtonRan) {
     const double code = S.maxDispCode == 2 ? 2.0 : (S.maxDispCode == 1 ? 0.5 : 0.0);
     S.maxVelocitySq = fmax_ref(S.cellTerm, code);
@@ -324,7 +342,7 @@ __global__ void k_gate(Dev d) {
     else run = 0;
   }
   S.runCollider = run;
-  S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0;
+  S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0; *d.Q = QueueState();
   if (run) {
     int init = 0;
     if (S.doSort) { init = 1; S.doSort = 0; }
@@ -1439,16 +1457,15 @@ __global__ void __launch_bounds__(128, 3) k_contacts_pre(Dev d) {
           shortq = d.prm->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN
                        ? (!isNew && prevDepth > 0)
                        : (!isNew && ((fl & F_ITERS_MASK) >> F_ITERS_SHIFT) < LONG_ITERS_BUCKET);
-          // Levenberg-Marquardt searches that took 32 or more iterations at the last step go to
-          // the long-search queue (fbQueue): the FP64 kernel spreads them over its warps, at
-          // most LONG_PER_WARP per warp, and gives them the spare evaluation slots, so that the
-          // chains of dependent evaluations that bound the stage advance an iteration per round;
-          // the mixed form runs them in FP64 (a double-float search that long would be deferred)
-          if (d.prm->contactModel != SQDEM_CONTACT_HERTZ_MINDLIN && !isNew &&
-              (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT) >= d.prm->vlongBucket) {
+          // Levenberg-Marquardt searches that ran long at the last step go to the long-search queue
+          // (fbQueue, the longest from its front): a warp each (k_search_warp), in FP64 in both forms
+          // (a double-float search that long would be deferred)
+          const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
+          if (d.prm->contactModel != SQDEM_CONTACT_HERTZ_MINDLIN && !isNew && bucket >= d.prm->vlongBucket) {
             queue = false;
-            const int k = atomicAdd(&d.S->vlCount, 1);
-            d.fbQueue[k] = e;
+            shortq = false;
+            if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
+            else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
             atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
           }
         }
@@ -1476,26 +1493,11 @@ __global__ void __launch_bounds__(128, 3) k_contacts_pre(Dev d) {
   flushCounters(d, cnt);
 }
 
-// Pass 2: the Levenberg-Marquardt searches of lmder2 (Superquadrics_Ig2.cpp:1057-1354),
-// restated as a per-lane state machine.  Every round each lane of a warp evaluates exactly
-// one Disfunction (Superquadrics_Ig2.cpp:622-687) at the point its state asks for, so the
-// warp stays converged on the expensive evaluation while lanes sit at different iterations
-// of different contacts; a lane that finishes a contact takes the next one from the queue.
-// The sequence of evaluations, decisions and results per contact is that of the reference:
-// only JacfunctionApp's re-evaluation at the current point is skipped, whose outputs equal
-// the stored ones bit for bit and are overwritten by the two probes that follow.
-enum { ST_INIT = 1, ST_PROBE0 = 2, ST_PROBE1 = 3, ST_TRIAL = 4 };
-
-struct LMLane {
-  int e, st, phase, k, stop, nu;
-  bool stopFlag, touching, isNew, fromCenter;
-  double p0, p1, q0, q1, mu, Dp0, Dp1, pfL2, pL2;
-  double j00, j01, j11, diag0, diag1, jt0, jt1;
-  D3 pf, f1, contact, P1, P2, C;
-  unsigned calls, iters, maxit, rounds;
-  bool isLong;   // taken from the long-search queue: first claim on the spare slots
-};
-
+// Pass 2: the Levenberg-Marquardt searches of lmder2 (Superquadrics_Ig2.cpp:1057-1354), restated as
+// a sequence of Disfunction evaluations (Superquadrics_Ig2.cpp:622-687) and the decisions between
+// them.  The sequence of evaluations, decisions and results per contact is that of the reference:
+// only JacfunctionApp's re-evaluation at the current point is skipped, whose outputs equal the
+// stored ones bit for bit and are overwritten by the two probes that follow.
 static const int LM_BS = 128;
 
 // x^3 for the damping update of lmder2 (pow(2*tmp - 1., 3.), Superquadrics_Ig2.cpp:1299): x^2
@@ -1508,207 +1510,40 @@ __device__ __forceinline__ double cube(double x) {
   return fma(h, x, l * x);
 }
 
-__device__ __forceinline__ void lmStartSolve(LMLane& L) {
-  L.touching = true; L.stopFlag = false; L.stop = 0;
-  L.q0 = L.p0; L.q1 = L.p1; L.st = ST_INIT;
-}
-
-// top of lmder2's for-loop: loop condition, then the checks before the Jacobian
-__device__ __forceinline__ bool lmOuter(LMLane& L) {
-  if (!(L.k < 50 && !L.stop)) { if (L.k >= 50) L.stop = 3; return false; }
-  if (L.pfL2 <= 1e-20) { L.stop = 6; return false; }
-  if (L.stopFlag) { L.stop = 9; L.touching = false; return false; }
-  double s0, c0, s1, c1;
-  sincos(L.p0, &s0, &c0);
-  sincos(L.p1, &s1, &c1);
-  L.contact = d3(c0 * c1, s0 * c1, s1);
-  double angle = dot(L.pf, L.contact) / (nrm(L.pf) * nrm(L.contact));
-  if (fabs(angle) > 0.95) { L.stop = 8; return false; }
-  L.q0 = L.p0 + L.Dp0; L.q1 = L.p1; L.st = ST_PROBE0;
-  return true;
-}
-// top of the damping while-loop
-__device__ __forceinline__ bool lmInner(LMLane& L) {
-  L.j00 += L.mu;
-  L.j11 += L.mu;
-  const double n_a = L.j00 * L.j11 - L.j01 * L.j01;
-  L.Dp0 = (L.jt0 * L.j11 - L.jt1 * L.j01) / n_a;
-  L.Dp1 = (L.jt1 * L.j00 - L.jt0 * L.j01) / n_a;
-  const double Dp_L2 = sqrt(L.Dp0 * L.Dp0 + L.Dp1 * L.Dp1);
-  if (Dp_L2 < 1e-5) { L.stop = 2; L.k++; return lmOuter(L); }
-  L.q0 = L.p0 + L.Dp0; L.q1 = L.p1 + L.Dp1;
-  if (Dp_L2 >= (L.pL2 + 1e-3) / (1e-12 * 1e-12)) { L.stop = 4; L.k++; return lmOuter(L); }
-  L.st = ST_TRIAL;
-  return true;
-}
-// consume the evaluation the lane asked for; returns true while the solve continues
-__device__ __forceinline__ bool lmConsume(LMLane& L) {
-  switch (L.st) {
-    case ST_INIT:
-      L.pf = L.P2 - L.P1;
-      L.pfL2 = nrm(L.pf);
-      L.stop = isfinite(L.pfL2) ? 0 : 7;
-      L.k = 0; L.mu = 0; L.nu = 2; L.Dp0 = 1e-7; L.Dp1 = 1e-7;
-      return lmOuter(L);
-    case ST_PROBE0:
-      L.f1 = L.P2 - L.P1;
-      L.q0 = L.p0; L.q1 = L.p1 + L.Dp1; L.st = ST_PROBE1;
-      return true;
-    case ST_PROBE1: {
-      const D3 f2 = L.P2 - L.P1, f0 = L.pf;
-      const double J00 = (L.f1.x - f0.x) / L.Dp0, J10 = (L.f1.y - f0.y) / L.Dp0, J20 = (L.f1.z - f0.z) / L.Dp0;
-      const double J01 = (f2.x - f0.x) / L.Dp1, J11 = (f2.y - f0.y) / L.Dp1, J21 = (f2.z - f0.z) / L.Dp1;
-      L.j00 = J00 * J00 + (J10 * J10 + J20 * J20);
-      L.j01 = J00 * J01 + (J10 * J11 + J20 * J21);
-      L.j11 = J01 * J01 + (J11 * J11 + J21 * J21);
-      L.jt0 = J00 * (-1.0 * f0.x) + (J10 * (-1.0 * f0.y) + J20 * (-1.0 * f0.z));
-      L.jt1 = J01 * (-1.0 * f0.x) + (J11 * (-1.0 * f0.y) + J21 * (-1.0 * f0.z));
-      const double jinf = (fabs(L.jt0) > fabs(L.jt1) ? fabs(L.jt0) : fabs(L.jt1));
-      L.pL2 = sqrt(L.p0 * L.p0 + L.p1 * L.p1);
-      if (jinf <= 1e-15) { L.stop = 1; return false; }
-      if (L.k == 0) L.mu = 1.0 * (L.j00 > L.j11 ? L.j00 : L.j11);
-      L.diag0 = L.j00; L.diag1 = L.j11;
-      return lmInner(L);
-    }
-    default: {  // ST_TRIAL
-      const D3 pDp_f = L.P2 - L.P1;
-      const double pDp_fL2 = nrm(pDp_f);
-      if (!isfinite(pDp_fL2)) { L.stop = 7; L.k++; return lmOuter(L); }
-      const double dL = L.Dp0 * (L.mu * L.Dp0 + L.jt0) + L.Dp1 * (L.mu * L.Dp1 + L.jt1);
-      const double dF = L.pfL2 - pDp_fL2;
-      double tmp = dF / dL;
-      if (tmp > 0.0) {
-        tmp = 1.0 - cube(2 * tmp - 1.);
-        L.mu = L.mu * ((tmp >= 0.3333333333333334) ? tmp : 0.3333333333333334);
-        L.nu = 2;
-        L.p0 = L.q0; L.p1 = L.q1;
-        L.pf = pDp_f; L.pfL2 = pDp_fL2;
-        L.k++;
-        return lmOuter(L);
-      }
-      L.mu *= L.nu;
-      const int nu2 = (int)((unsigned)L.nu << 1);
-      if (nu2 <= L.nu) { L.stop = 5; L.k++; return lmOuter(L); }
-      L.nu = nu2;
-      L.j00 = L.diag0; L.j11 = L.diag1;
-      return lmInner(L);
-    }
-  }
-}
-
-// Points lmder2 evaluates next: the requested one in slot 0, then the points that follow it
-// under each outcome of the requested evaluation: after INIT the two probes at the start
-// point; after PROBE0 the second probe; after a TRIAL the two probes at the trial point
-// (accepted), then the next trial with mu*nu (rejected) and its probes, and so on.  Along
-// every outcome the points asked for appear in increasing slot order (the order of the
-// consume pass).  Every point is computed with the operations the state machine itself
-// uses, so a point it later asks for matches bit for bit.  (Ordering the trials first when
-// the last iteration had rejections was measured slower.)  Writes q[i] and own[i] = lane
-// for each planned slot i < S.
-__device__ __forceinline__ void lmPlan(const LMLane& L, double2* q, int* own, int S, int lane) {
-  int n = 0;
-  q[n] = make_double2(L.q0, L.q1); own[n++] = lane;
-  if (L.st == ST_INIT) {
-    if (n < S) { q[n] = make_double2(L.p0 + 1e-7, L.p1); own[n++] = lane; }
-    if (n < S) { q[n] = make_double2(L.p0, L.p1 + 1e-7); own[n++] = lane; }
-  } else if (L.st == ST_PROBE0) {
-    if (n < S) { q[n] = make_double2(L.p0, L.p1 + L.Dp1); own[n++] = lane; }
-  } else if (L.st == ST_TRIAL) {
-    double mu = L.mu, t0 = L.q0, t1 = L.q1, d0 = L.Dp0, d1 = L.Dp1;
-    int nu = L.nu;
-    while (n < S) {
-      q[n] = make_double2(t0 + d0, t1); own[n++] = lane;
-      if (n >= S) break;
-      q[n] = make_double2(t0, t1 + d1); own[n++] = lane;
-      if (n >= S) break;
-      // the trial after a rejection of this one (lmConsume's rejection branch, then lmInner)
-      mu *= nu;
-      const int nu2 = (int)((unsigned)nu << 1);
-      if (nu2 <= nu) break;
-      nu = nu2;
-      const double j00 = L.diag0 + mu, j11 = L.diag1 + mu;
-      const double n_a = j00 * j11 - L.j01 * L.j01;
-      d0 = (L.jt0 * j11 - L.jt1 * L.j01) / n_a;
-      d1 = (L.jt1 * j00 - L.jt0 * L.j01) / n_a;
-      const double Dp_L2 = sqrt(d0 * d0 + d1 * d1);
-      if (Dp_L2 < 1e-5) break;
-      t0 = L.p0 + d0; t1 = L.p1 + d1;
-      if (Dp_L2 >= (L.pL2 + 1e-3) / (1e-12 * 1e-12)) break;
-      q[n] = make_double2(t0, t1); own[n++] = lane;
-    }
-  }
-}
-
 __device__ __forceinline__ bool sameBits(double2 a, double q0, double q1) {
   return __double_as_longlong(a.x) == __double_as_longlong(q0) && __double_as_longlong(a.y) == __double_as_longlong(q1);
 }
 
-// One lmder2 call finished: the restart rules of Superquadrics_Ig2.cpp:2013-2053, and when no
-// restart follows, the end of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go, Ip2 and
-// the law.  Returns true when the contact is finished.
-__device__ __forceinline__ bool lmCallEnd(const Dev& d, LMLane& L, const SqShape& A, const SqShape& B, Counters& cnt) {
+// End of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go (Superquadrics_Ig2.cpp:2054-2095)
+// for a search that ended at angles (p0, p1), then Ip2 and the law.
+__device__ __forceinline__ void finishSearch(const Dev& d, int e, unsigned fl, int id1, int id2, bool isNew, double p0,
+                                             double p1, bool touching, D3 P1, D3 P2, D3 contact, unsigned calls,
+                                             unsigned iters, unsigned maxit, Counters& cnt) {
   const SceneState& S = *d.S;
-  for (;;) {
-    L.calls++; L.iters += L.k; L.maxit += (L.stop == 3);
-    bool restart = false;
-    if (L.phase == 0) {
-      L.phase = 1;
-      if ((isnan(L.p0) || isnan(L.p1) || 7 == L.stop) && L.touching) restart = true;
-    } else if (L.phase == 1) {
-      L.phase = 3;
-      if (L.touching && 10.0 * nrm(L.P2 - L.P1) > A.rmax && (!isInside(A, L.P2 - A.pos) || !isInside(B, L.P1 - B.pos))) {
-        L.phase = 2; restart = true;
-      }
-    } else L.phase = 3;
-    if (!restart && L.phase == 1) {  // no NaN restart: continue with the local-minimum check
-      L.phase = 3;
-      if (L.touching && 10.0 * nrm(L.P2 - L.P1) > A.rmax && (!isInside(A, L.P2 - A.pos) || !isInside(B, L.P1 - B.pos))) {
-        L.phase = 2; restart = true;
-      }
-    }
-    if (!restart) break;
-    if (!L.fromCenter) {
-      double para[2];
-      centerLine(A.pos, B.pos, para);
-      L.p0 = para[0]; L.p1 = para[1];
-      L.fromCenter = true;
-      lmStartSolve(L);
-      return false;
-    }
-    // The restarted call would start where the call that just ended started (the centre
-    // line), from the state lmStartSolve sets: it is the same computation, and its outcome
-    // is the one at hand.  It is counted as run, and the restart rules go on from there.
-  }
-  // end of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go, then Ip2 + law
-  const int e = L.e;
-  const unsigned fl = d.A.flags[e];
-  int id1, id2;
-  entryIds(d, e, fl, id1, id2);
   const BodyView b1 = loadBody(d, id1), b2 = loadBody(d, id2);
   GeomOut g;
-  g.lmCalls = L.calls; g.lmIters = L.iters; g.lmStop = 0; g.nanNormal = false;
-  g.isShearNew = L.isNew ? true : (d.A.depth[e] <= 0);
-  g.cp = L.isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]);
-  g.ang0 = L.p0; g.ang1 = L.p1; g.angSet = true;
-  if (!L.touching) {
+  g.lmCalls = calls; g.lmIters = iters; g.lmStop = 0; g.nanNormal = false;
+  g.isShearNew = isNew ? true : (d.A.depth[e] <= 0);
+  g.cp = isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]);
+  g.ang0 = p0; g.ang1 = p1; g.angSet = true;
+  if (!touching) {
     g.precomputed = false; g.depth = 0; g.isShearNew = true;
   } else {
-    const double pDepth = dot(L.P1 - L.P2, L.contact);
-    g.p1 = L.P1; g.p2 = L.P2;
-    if (isnan(L.contact.x)) g.nanNormal = true;
-    g.cp = L.C;
+    const double pDepth = dot(P1 - P2, contact);
+    g.p1 = P1; g.p2 = P2;
+    if (isnan(contact.x)) g.nanNormal = true;
+    g.cp = 0.5 * (P1 + P2);
     g.depth = pDepth;
-    D3 cn = L.contact;
+    D3 cn = contact;
     normalize(cn);
-    const D3 oldNormal = L.isNew ? d3(0, 0, 0) : xyz(d.A.normal[e]);
+    const D3 oldNormal = isNew ? d3(0, 0, 0) : xyz(d.A.normal[e]);
     g.precomputed = true;
-    precomputeD(g, oldNormal, b1, b2, d.prm->dt, cn, g.isShearNew, cellShift(S, d.A.cd[e]),
-                shiftVelOf(S, *d.prm, cellShift(S, d.A.cd[e])));
+    const D3 shift2 = cellShift(S, d.A.cd[e]);
+    precomputeD(g, oldNormal, b1, b2, d.prm->dt, cn, g.isShearNew, shift2, shiftVelOf(S, *d.prm, shift2));
     g.normal = cn;
   }
-  cnt.lmCalls += L.calls; cnt.lmIters += L.iters; cnt.lmMax += L.maxit;
-  finishEntry(d, e, fl, L.isNew, id1, b1, b2, g, cnt);
-  return true;
+  cnt.lmCalls += calls; cnt.lmIters += iters; cnt.lmMax += maxit;
+  finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
 }
 
 // One Disfunction evaluation (Superquadrics_Ig2.cpp:622-687) by a group of six lanes:
@@ -1721,10 +1556,6 @@ __device__ __forceinline__ bool lmCallEnd(const Dev& d, LMLane& L, const SqShape
 // first lane, sub the lane's place in it.  (Four-lane groups, eight points per round, were
 // measured slower: one more pow on the chain.)
 static const int COOP_LANES = 6, COOP_POINTS = 5;
-// FP64 search kernel: searches a warp holds while its queues have work, long-queue searches
-// per warp, and the spare slots one search may take in a round (trial, two probes, the next
-// trials after rejections)
-static const int LONG_PER_WARP = 2, MAX_EXTRA = 4;
 __device__ __forceinline__ void coopEval(const SqShape& A, const SqShape& B, double q0, double q1, int g0, int sub,
                                          D3& p1, D3& p2, bool& flag, const Rot* G = nullptr, double* dist = nullptr) {
   const unsigned FULL = 0xffffffffu;
@@ -1792,187 +1623,33 @@ __device__ __forceinline__ void allocSlots(bool in, unsigned prio, int budget, i
   jmax = share + min(maxExtra, extra);
 }
 
-// Pass 2, FP64.  Rounds of one Disfunction evaluation per lane.  While the queue has work,
-// every lane evaluates the point its own search asks for.  Once the queue is drained, the
-// lanes left without a contact evaluate, for the searches still running in their warp, the
-// points those searches will ask for next (lmPlan); each search then consumes, in its own
-// order, every evaluation whose point is the one it asks for.  A search with 31 idle lanes
-// beside it thus advances one whole iteration (trial + two probes, or a run of rejected
-// trials) per round instead of one evaluation, which shortens the dependency chain of the
-// longest searches that bound the kernel.  While at most COOP_POINTS searches run in the
-// warp, each point is evaluated by a group of six lanes (coopEval), which shortens each
-// round as well.  Results are those of the one-point rounds: an evaluation depends only on
-// its point and the two shapes.
-// Two builds: MINB = 1 keeps every lane's state in registers (222, two blocks per SM); MINB =
-// 3 caps registers at 168 for three blocks per SM (more warps to hide FP64 latency, at the cost
-// of a few hundred bytes of spills per thread).  The launch shape (search blocks per SM)
-// selects one; the autotuner times both.
-// mode: LM_FP64 the FP64 form (main queue and long-search queue); LM_DEFERRED the mixed form's
-// FP64 pass: its long-search queue and the searches the double-float kernels deferred.  (Running
-// the long-search queue on a second stream beside the double-float kernel was measured slower:
-// its blocks take the SM resources the double-float kernel's warps need.)
-enum { LM_FP64 = 0, LM_DEFERRED = 2 };
-template <int MINB>
-__global__ void __launch_bounds__(LM_BS, MINB) k_contacts_lm(Dev d, int mode) {
-  __shared__ SqShape shA[LM_BS], shB[LM_BS];
-  __shared__ double2 slotQ[LM_BS];
-  __shared__ int slotOwner[LM_BS];
-  const SceneState& S = *d.S;
-  // the main queue (lmQueue: long searches first, then the short ones from its back) and the
-  // long-search queue in fbQueue: the searches of 32+ iterations at the last step
-  // ([0, vlCount)), in the mixed form's FP64 pass followed by the deferred searches
-  // ([vlCount, vlCount + fbCount))
-  const int fallback = mode != LM_FP64;   // no main queue: the long-search queue alone
-  const int nFront = S.lmCount, count = S.lmCount + S.nmShort;
-  const int longBase = 0;
-  const int nLongQ = mode == LM_DEFERRED ? S.vlCount + S.fbCount : S.vlCount;
-  int* longHead = mode == LM_DEFERRED ? &d.S->fbHead : &d.S->vlHead;
-  const int lane = threadIdx.x & 31;
-  const int wbase = threadIdx.x & ~31;
-  const bool spread = d.prm->lmSpread != 0;
-  // searches a warp holds: in the main pass at most LONG_PER_WARP from the long queue, and in
-  // all 32 less MAX_EXTRA per long search held while the main queue has work (those slots go
-  // to the long searches); in the second pass of the mixed form as many as spread the queue
-  // over all warps, at most COOP_POINTS
-  const int warps = gridDim.x * (LM_BS / 32);
-  const int cap = !spread ? 32 : fallback ? min(COOP_POINTS, max(1, (nLongQ + warps - 1) / warps)) : 32;
-  Counters cnt = {0, 0, 0, 0, 0};
-  unsigned long long ev64 = 0;
-  unsigned roundsMax = 0;
-  LMLane L;
-  L.isLong = false;
-  bool active = false;
-  bool mainDone = fallback != 0, longDone = false;   // warp-uniform: the queues this warp found empty
-  auto start = [&](int e) {
-    // start a contact: Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go up to lmder2
-    SqShape& A = shA[threadIdx.x];
-    SqShape& B = shB[threadIdx.x];
-    L.e = e;
-    const unsigned fl = d.A.flags[L.e];
-    int id1, id2;
-    entryIds(d, L.e, fl, id1, id2);
-    const double4 o1 = d.ori[id1], o2 = d.ori[id2];
-    const double4 a1 = d.shpA[id1], a2 = d.shpA[id2], e1 = d.shpB[id1], e2 = d.shpB[id2];
-    shapeInit(A, a1.x, a1.y, a1.z, e1.x, e1.y, a1.w); A.R = quatToRot(o1.x, o1.y, o1.z, o1.w); A.pos = xyz(d.pos[id1]);
-    shapeInit(B, a2.x, a2.y, a2.z, e2.x, e2.y, a2.w); B.R = quatToRot(o2.x, o2.y, o2.z, o2.w);
-    B.pos = xyz(d.pos[id2]) + cellShift(S, d.A.cd[L.e]);
-    L.isNew = !(fl & F_GEOM);
-    if (L.isNew) { double para[2]; centerLine(A.pos, B.pos, para); L.p0 = para[0]; L.p1 = para[1]; }
-    else { const double2 an = d.A.angle[L.e]; L.p0 = an.x; L.p1 = an.y; }
-    L.fromCenter = L.isNew;
-    L.contact = d3(0, 0, 0); L.P1 = d3(0, 0, 0); L.P2 = d3(0, 0, 0); L.C = d3(0, 0, 0);
-    L.phase = 0; L.calls = 0; L.iters = 0; L.maxit = 0; L.rounds = 0;
-    lmStartSolve(L);
-    active = true;
-  };
-  while (true) {
-    // take work: idle lanes claim entries with one atomic per warp and queue, up to the caps
-    const unsigned below = (1u << lane) - 1;
-    if (!longDone) {
-      const unsigned idle = __ballot_sync(0xffffffffu, !active);
-      const int nAct = 32 - __popc(idle);
-      const int held = __popc(__ballot_sync(0xffffffffu, active && L.isLong));
-      const int perWarp = (fallback || !spread) ? cap : LONG_PER_WARP;
-      const int want = min(__popc(idle), min(perWarp - held, cap - nAct));
-      if (want > 0) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(longHead, want);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        const int r = __popc(idle & below);
-        if (!active && r < want && base + r < nLongQ) { start(d.fbQueue[longBase + base + r]); L.isLong = true; }
-        if (base + want >= nLongQ) longDone = true;
-      }
-    }
-    if (!mainDone) {
-      const unsigned idle = __ballot_sync(0xffffffffu, !active);
-      const int held = spread ? __popc(__ballot_sync(0xffffffffu, active && L.isLong)) : 0;
-      const int room = cap - MAX_EXTRA * held - (32 - __popc(idle));
-      const int want = min(__popc(idle), room);
-      if (want > 0) {
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&d.S->lmHead, want);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        const int r = __popc(idle & below);
-        if (!active && r < want) {
-          const int idx = base + r;
-          if (idx < count) { start(idx < nFront ? d.lmQueue[idx] : d.lmQueue[d.qCap - 1 - (idx - nFront)]); L.isLong = false; }
-        }
-        if (base + want >= count) mainDone = true;
-      }
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (!act && mainDone && longDone) break;
-    if (!act) continue;
-    // Points per running search: 1 while the queues have work and the warp holds 32 searches.
-    // Otherwise the warp's evaluation slots (five groups of six lanes, coopEval, while at most
-    // COOP_POINTS searches run, else 32 single lanes) are shared out: one each, the rest to the
-    // long searches first, then to those that have run the most rounds.
-    const int nA = __popc(act);
-    const bool drained = spread && mainDone && longDone;
-    const bool capped = spread && !drained && (cap < 32 || __any_sync(0xffffffffu, active && L.isLong));
-    const bool coop = (drained || capped) && nA <= COOP_POINTS;
-    const unsigned prio = (L.isLong ? 0x80000000u : 0u) | min(L.rounds, 0x7fffffffu);
-    int spc, base, jmax;
-    allocSlots(active, prio, (drained || capped) ? (coop ? COOP_POINTS : 32) : nA, drained ? 1 : MAX_EXTRA, spc, base,
-               jmax);
-    slotOwner[threadIdx.x] = -1;
-    __syncwarp();
-    if (active) lmPlan(L, &slotQ[wbase + base], &slotOwner[wbase + base], spc, lane);
-    __syncwarp();
-    D3 P1 = d3(0, 0, 0), P2 = d3(0, 0, 0);
-    bool flag = false;
-    if (coop) {
-      // group g of six lanes evaluates slot g; lanes 30-31 and groups without a point mirror
-      // slot 0 (its owner always exists) so that every lane computes on valid inputs
-      const int graw = lane / COOP_LANES;
-      const int grp = graw < COOP_POINTS ? graw : 0;
-      const int sub = graw < COOP_POINTS ? lane - grp * COOP_LANES : lane - COOP_POINTS * COOP_LANES;
-      const int o = slotOwner[wbase + grp];
-      const bool has = graw < COOP_POINTS && o >= 0;
-      const int slot = has ? grp : 0;
-      const int src = wbase + slotOwner[wbase + slot];
-      const double2 q = slotQ[wbase + slot];
-      coopEval(shA[src], shB[src], q.x, q.y, grp * COOP_LANES, sub, P1, P2, flag);
-      if (has && sub == 0) ev64++;
-    } else {
-      const int own = slotOwner[threadIdx.x];
-      if (own >= 0) {
-        const double2 q = slotQ[threadIdx.x];
-        D3 C;
-        disfunction(shA[wbase + own], shB[wbase + own], q.x, q.y, C, P1, P2, flag);
-        ev64++;
-      }
-    }
-    if (active) L.rounds++;
-    for (int j = 0; j < jmax; j++) {
-      const int si = base + j;
-      const bool mine = j < spc;
-      const int src = mine ? (coop ? si * COOP_LANES : si) : lane;
-      const double x1 = __shfl_sync(0xffffffffu, P1.x, src), y1 = __shfl_sync(0xffffffffu, P1.y, src),
-                   z1 = __shfl_sync(0xffffffffu, P1.z, src);
-      const double x2 = __shfl_sync(0xffffffffu, P2.x, src), y2 = __shfl_sync(0xffffffffu, P2.y, src),
-                   z2 = __shfl_sync(0xffffffffu, P2.z, src);
-      const bool f = __shfl_sync(0xffffffffu, (int)flag, src) != 0;
-      if (mine && active && slotOwner[wbase + si] == lane && sameBits(slotQ[wbase + si], L.q0, L.q1)) {
-        L.P1 = d3(x1, y1, z1);
-        L.P2 = d3(x2, y2, z2);
-        L.C = 0.5 * (L.P1 + L.P2);
-        if (f) L.stopFlag = true;
-        if (!lmConsume(L) && lmCallEnd(d, L, shA[threadIdx.x], shB[threadIdx.x], cnt)) {
-          active = false;
-          roundsMax = max(roundsMax, L.rounds);
-        }
-      }
-    }
-    __syncwarp();
-  }
-  flushCounters(d, cnt);
-  for (int o = 16; o > 0; o >>= 1) {
-    ev64 += __shfl_down_sync(0xffffffffu, ev64, o);
-    roundsMax = max(roundsMax, __shfl_down_sync(0xffffffffu, roundsMax, o));
-  }
-  if (lane == 0) { atomicAdd(&d.S->err[E_EVAL64], ev64); atomicMax(&d.S->err[E_ROUNDS_MAX], (unsigned long long)roundsMax); }
+// c.(p2 - p1) against |p2 - p1| |c|: |cos(f, c)| > 0.95 as lmder2 tests it
+// (Superquadrics_Ig2.cpp:1144-1154).  |c| is 1 to a few ulps, so that outside a band of 1e-9 around
+// the threshold the test needs neither |c| nor the division.
+__device__ __forceinline__ bool angleTest(double sep, double nrmf, const D3& c) {
+  const double a = fabs(sep), t = 0.95 * nrmf;
+  if (a > t * (1.0 + 1e-9)) return true;
+  if (a < t * (1.0 - 1e-9)) return false;
+  return fabs(sep / (nrmf * nrm(c))) > 0.95;
 }
+
+// isInside (Superquadrics.cpp:103-108) of p relative to the centre, decided in FP32 where it is far
+// from its threshold: 1 inside, 0 outside, -1 for the FP64 test (six pow).  The FP32 value is off by
+// some 1e-6 times its exponents (2/eps1, 2/eps2 up to 200 here); a point is decided outside [0.9, 1.1].
+__device__ __forceinline__ int insideFast(const SqShape& s, D3 p) {
+  const float e1 = (float)s.e1, e2 = (float)s.e2;
+  if (!(e1 >= 0.01f && e2 >= 0.01f)) return -1;
+  const float px = (float)p.x, py = (float)p.y, pz = (float)p.z;
+  const float x = (float)s.R.m[0] * px + (float)s.R.m[3] * py + (float)s.R.m[6] * pz;
+  const float y = (float)s.R.m[1] * px + (float)s.R.m[4] * py + (float)s.R.m[7] * pz;
+  const float z = (float)s.R.m[2] * px + (float)s.R.m[5] * py + (float)s.R.m[8] * pz;
+  const float v = powf(powf(fabsf(x / (float)s.rx), 2.f / e1) + powf(fabsf(y / (float)s.ry), 2.f / e1), e1 / e2) +
+                  powf(fabsf(z / (float)s.rz), 2.f / e2);
+  return v < 0.9f ? 1 : v > 1.1f ? 0 : -1;   // NaN: the FP64 test
+}
+
+#include "sq_wave_search.cuh"
+#include "sq_warp_search.cuh"
 
 // ---------------------------------------------------------------------------
 // Pass 2 of the Hertz-Mindlin model: the Nelder-Mead searches of
@@ -2425,8 +2102,7 @@ __global__ void __launch_bounds__(LM_BS) k_contacts_lm_ff(Dev d) {
           d.B.normal[i] = make_double4(ffToD(L.c[0]), ffToD(L.c[1]), ffToD(L.c[2]), 0);
           d.B.cd[i] = make_int4((int)L.calls, (int)L.iters, (int)L.maxit, L.touching ? 1 : 0);
         } else if (r == LMF_DEFER) {
-          const int k = atomicAdd(&d.S->fbCount, 1);
-          d.fbQueue[d.S->vlCount + k] = L.e;
+          d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = L.e;
           deferred++;
         }
         if (r != LMF_MORE) {
@@ -2501,8 +2177,7 @@ __global__ void __launch_bounds__(128) k_contacts_lm_ff_finish(Dev d) {
       cnt.lmCalls += info.x; cnt.lmIters += info.y; cnt.lmMax += info.z;
       finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
     } else {
-      const int k = atomicAdd(&d.S->fbCount, 1);
-      d.fbQueue[d.S->vlCount + k] = e;
+      d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = e;
       deferred++;
     }
   }
@@ -2995,7 +2670,7 @@ __global__ void __launch_bounds__(256) k_integrate(Dev d) {
 
 __global__ void k_reset_queue(Dev d) {
   d.S->lmCount = 0; d.S->lmHead = 0; d.S->fbCount = 0; d.S->fbHead = 0; d.S->vlCount = 0; d.S->vlHead = 0;
-  d.S->nmFin = 0; d.S->nmShort = 0;
+  d.S->nmFin = 0; d.S->nmShort = 0; *d.Q = QueueState();
 }
 
 // Start of NewtonIntegrator::action (NewtonIntegrator.cpp:107-117): pending velGrad, the
@@ -3044,6 +2719,8 @@ struct sqdem_ctx {
   int lmBlocksPerSM = 4, lmBlocksPerSMmixed = 4, nmBlocksPerSM = 4;
   int shapeSearch = 0, shapePass1 = 0;   // launch shapes set by the caller or the autotuner (0: defaults)
   cudaStream_t stream = nullptr;
+  cudaStream_t stream2 = nullptr;   // the long searches, beside the rest of the contact stage
+  cudaEvent_t fork = nullptr, join = nullptr;
   Dev d;
   bool haveBodies = false, haveMats = false, haveParams = false;
   cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr; bool graphValid = false;
@@ -3055,6 +2732,8 @@ struct sqdem_ctx {
   int lmSpread = 1;
   int periodicFix = 0;   // sqdem_set_periodic_fix
   int contactModel = SQDEM_CONTACT_LINEAR;
+  bool inBatch = false;
+  int load = 0;          // particles of the batch the context steps in (0: none): what the launch shapes go by
   bool servoOn = false;
   std::vector<int> kind, wallIds, matIds, isSphere, axisSense;
   std::vector<double> shape5;
@@ -3116,6 +2795,10 @@ static void launchScan(sqdem_ctx* c, const int* in, int n, int* out, const int* 
   c->launches += 3;
 }
 
+// resident blocks per SM of the rounds: two keep the FP64 pipe busy, a third slows the long searches
+// that run beside them (200,000 particles: 20.6 ms a step with two, 21.3 with three, 23 with one)
+static const int WAVE_BLOCKS_PER_SM = 2;
+
 // Resident blocks per SM of the search kernel the context launches.
 static int maxSearchBlocksPerSM(const sqdem_ctx* c) {
   if (c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) return c->nmBlocksPerSM;
@@ -3123,15 +2806,22 @@ static int maxSearchBlocksPerSM(const sqdem_ctx* c) {
 }
 static int searchBlocksPerSM(const sqdem_ctx* c) {
   const int mx = maxSearchBlocksPerSM(c);
-  return c->shapeSearch > 0 ? std::min(c->shapeSearch, mx) : mx;
+  if (c->shapeSearch > 0) return std::min(c->shapeSearch, mx);
+  return c->contactModel != SQDEM_CONTACT_HERTZ_MINDLIN && c->precision == SQDEM_FP64 ? std::min(WAVE_BLOCKS_PER_SM, mx) : mx;
 }
 static const int PASS1_BLOCKS_PER_SM = 16;   // grid-stride blocks of pass 1 per SM (default)
 
-// the FP64 search kernel build for a grid of `grid` blocks: the three-blocks-per-SM build when
-// the grid asks for more than two blocks per SM
-static void launchLmFP64(const sqdem_ctx* c, int grid, cudaStream_t s, const Dev& d, int mode) {
-  if (grid > 2 * c->numSMs) k_contacts_lm<3><<<grid, LM_BS, 0, s>>>(d, mode);
-  else k_contacts_lm<1><<<grid, LM_BS, 0, s>>>(d, mode);
+// FP64 form, where each search goes.  Up to WARP_SEARCH_MAX particles (of the scene, or of the batch
+// it steps in) every search takes a warp: 608 warps then run the stage in about the time of its
+// longest search (a jammed cell of 1,583 particles: 2.9 ms a step, 3.2 in rounds; of 9,000: 1.7
+// against 2.3).  Above it the rounds' full lanes win (43,011 particles: 6.3 ms against 15.5), until
+// few searches are left: a trial and a probe launch take 0.2 ms for up to some 3,500 searches, one
+// warp each 0.24 ms per iteration of those, and their number falls with the iterations, so that
+// the number of rounds grows with the logarithm of the scene (43,011 particles: 6 rounds, 200,000:
+// 13; one third more or fewer rounds cost at most 2% there).
+static const int WARP_SEARCH_MAX = 16000;
+static int waveRounds(const sqdem_ctx* c, const Dev& d) {
+  return std::max(4, std::min(WAVE_MAX_ROUNDS, (int)std::lround(3.0 * std::log2(std::max(c->load, d.NP) / 1e4))));
 }
 
 // The contact stage on c->stream: pass 1, then the searches of the selected contact model
@@ -3145,25 +2835,49 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
     k_contacts_nm_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
     c->launches += 3;
   } else {
+    // one block per SM for the warp searches: one warp per scheduler, whose FP64 pipe serves its
+    // chain alone
+    const int ws = std::min(c->numSMs, nblk(d.Pcap, LM_BS / 32));
     if (c->precision == SQDEM_MIXED) {
-      // double-float searches, then the FP64 kernel on the long-search queue and the searches
-      // the double-float kernels deferred
-      k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
+      // the long searches in FP64 beside the double-float searches, then the searches the
+      // double-float kernels deferred
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
+      cudaEventRecord(c->fork, s);
+      cudaStreamWaitEvent(c->stream2, c->fork, 0);
+      k_search_warp<<<ws, LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
+      cudaEventRecord(c->join, c->stream2);
+      k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
       k_contacts_lm_ff<<<grid, LM_BS, 0, s>>>(d);
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
       k_contacts_lm_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      // one block per SM: one warp per scheduler, so that the FP64 pipe serves each warp's
-      // chain of dependent evaluations alone (these searches are long; more warps per
-      // scheduler lengthen every round of the longest one)
-      launchLmFP64(c, c->numSMs, s, d, LM_DEFERRED);
+      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_DEFERRED, 0);
+      cudaStreamWaitEvent(s, c->join, 0);
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
-      c->launches += 5;
-    } else {
+      c->launches += 6;
+    } else if (std::max(c->load, d.NP) <= WARP_SEARCH_MAX) {
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
-      launchLmFP64(c, grid, s, d, LM_FP64);
+      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_ALL, 0);
       if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
       c->launches += 2;
+    } else {
+      if (c->timingSearch) cudaEventRecord(c->ev[4], s);
+      cudaEventRecord(c->fork, s);
+      cudaStreamWaitEvent(c->stream2, c->fork, 0);
+      k_search_warp<<<ws, LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
+      cudaEventRecord(c->join, c->stream2);
+      const int wave = c->numSMs * searchBlocksPerSM(c);
+      k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
+      k_wave_probe<<<wave, LM_BS, 0, s>>>(d, 0);
+      const int rounds = waveRounds(c, d);
+      for (int r = 1; r < rounds; r++) {
+        k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
+        k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
+      }
+      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_TAIL, rounds);
+      k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
+      cudaStreamWaitEvent(s, c->join, 0);
+      if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
+      c->launches += 4 + 2 * rounds;
     }
   }
 }
@@ -3262,9 +2976,10 @@ static sqdem_status uploadParams(sqdem_ctx* c) {
   P.lmSpread = c->lmSpread;
   P.contactModel = c->contactModel;
   P.periodicFix = c->periodicFix;
-  // 32+ iterations in both forms (from 64 in the mixed form was measured no faster: the
-  // double-float kernel then deferred more searches past 50 iterations, run again in FP64)
-  P.vlongBucket = (int)VLONG_ITERS_BUCKET;
+  // (from 64 in the mixed form was measured no faster: the double-float kernel then deferred more
+  // searches past 50 iterations, run again in FP64)
+  P.vlongBucket = c->precision == SQDEM_MIXED ? LONG_BUCKET_MIXED : c->inBatch ? LONG_BUCKET_BATCH : LONG_BUCKET_FP64;
+  P.vlongFront = c->precision == SQDEM_MIXED ? LONG_FRONT_MIXED : LONG_FRONT_FP64;
   P.h0 = hostH0(c);
   CK(cudaMemcpyAsync(c->d.prm, &P, sizeof(P), cudaMemcpyHostToDevice, c->stream));
   return SQDEM_OK;
@@ -3324,10 +3039,13 @@ sqdem_status sqdem_create(sqdem_ctx** out, const sqdem_config* cfg) {
   if (c->precision != SQDEM_FP64 && c->precision != SQDEM_MIXED) return fail(c, SQDEM_ERR_ARG, "unknown precision");
   CK(cudaSetDevice(c->device));
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
   CK(cudaDeviceGetAttribute(&c->numSMs, cudaDevAttrMultiProcessorCount, c->device));
   {
     int nb = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_contacts_lm<3>, LM_BS, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_wave_trial<false>, LM_BS, 0));
     c->lmBlocksPerSM = nb > 0 ? nb : 1;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_contacts_lm_ff, LM_BS, 0));
     c->lmBlocksPerSMmixed = nb > 0 ? nb : 1;
@@ -3349,6 +3067,9 @@ void sqdem_destroy(sqdem_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   freeAll(c);
   for (int i = 0; i < 7; i++) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
+  if (c->fork) cudaEventDestroy(c->fork);
+  if (c->join) cudaEventDestroy(c->join);
+  if (c->stream2) cudaStreamDestroy(c->stream2);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -3452,7 +3173,7 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* c, int n, const int* kind, const double
   d.MAXC = c->maxCand;
   d.Pcap = (int)std::min<long long>((long long)c->contactsPerBody * NP + 64, 0x7fffffffLL - 1024);
   d.Gmax = std::max(8 * NP, 1 << 12);
-  CK(dalloc(c, &d.prm, 1)); CK(dalloc(c, &d.S, 1));
+  CK(dalloc(c, &d.prm, 1)); CK(dalloc(c, &d.S, 1)); CK(dalloc(c, &d.Q, 1));
   CK(dalloc(c, &d.pos, n)); CK(dalloc(c, &d.ori, n)); CK(dalloc(c, &d.vel, n)); CK(dalloc(c, &d.angVel, n));
   CK(dalloc(c, &d.angMom, n)); CK(dalloc(c, &d.inertia, n)); CK(dalloc(c, &d.shpA, n)); CK(dalloc(c, &d.shpB, n));
   CK(dalloc(c, &d.mass, n)); CK(dalloc(c, &d.info, n)); CK(dalloc(c, &d.blocked, n)); CK(dalloc(c, &d.damped, n));
@@ -3475,7 +3196,8 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* c, int n, const int* kind, const double
   c->servoOn = false;
   CK(dalloc(c, &d.ww, std::max(d.W * d.W, 1)));
   CK(dalloc(c, &d.lmQueue, d.Pcap));
-  CK(dalloc(c, &d.fbQueue, d.Pcap));
+  CK(dalloc(c, &d.fbQueue, d.Pcap)); CK(dalloc(c, &d.deferQueue, d.Pcap));
+  CK(dalloc(c, &d.waveT0, d.Pcap)); CK(dalloc(c, &d.waveT1, d.Pcap)); CK(dalloc(c, &d.waveP, d.Pcap)); CK(dalloc(c, &d.waveF, d.Pcap));
   CK(dalloc(c, &d.bodyFF, d.N));
   d.qCap = d.Pcap;
   CK(dalloc(c, &d.bodyCell, n)); CK(dalloc(c, &d.cellCount, d.Gmax + 1)); CK(dalloc(c, &d.cellStart, d.Gmax + 1));
@@ -4557,12 +4279,15 @@ static sqdem_status batchReady(sqdem_batch* B) {
   BK(cudaSetDevice(B->device));
   BK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
   BK(cudaEventRecord(B->fork, B->stream));
-  long long l = 0;
+  long long l = 0, load = 0;
+  for (const sqdem_ctx* c : B->scenes) load += c->d.NP;
   for (size_t i = 0; i < B->scenes.size(); i++) {
     sqdem_ctx* c = B->scenes[i];
     BK(cudaStreamWaitEvent(c->stream, B->fork, 0));
     const long long l0 = c->launches;
+    c->load = (int)std::min(load, 0x7fffffffLL);
     enqueueStep(c, false);
+    c->load = 0;
     l += c->launches - l0;
     c->launches = l0;
     BK(cudaEventRecord(B->join[i], c->stream));
@@ -4592,6 +4317,7 @@ sqdem_status sqdem_batch_create(sqdem_batch** out, int n_scenes, const sqdem_con
     sqdem_ctx* c = nullptr;
     sqdem_status s = sqdem_create(&c, cfg);
     B->scenes.push_back(c);
+    if (c) c->inBatch = true;
     if (s) return bfail(B, s, "scene " + std::to_string(i) + ": " + (c ? c->err : std::string("create failed")));
     if (c->device != B->device) return bfail(B, SQDEM_ERR_ARG, "all scenes of a batch share one device");
   }
