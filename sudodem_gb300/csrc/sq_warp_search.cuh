@@ -9,16 +9,17 @@
 // iterations, each a trial evaluation, 0.9 rejected trials on average, and two
 // finite-difference probes, all dependent on one another.  So the 32 lanes of a warp serve one
 // search: six points per round, five lanes a point (two lanes per body, the fifth takes the ninth
-// pow of both), which makes a round 4 pow + 2 atan2 + 3 sincos long, and the six points are the
-// pending trial with the two probes that follow if it is accepted, and the trial that follows if it
-// is rejected with its two probes: a round is an iteration unless two trials in a row are
-// rejected.  The state machine's own arithmetic (the Jacobian's six divisions, the normal
-// equations, the step for both trials, gain ratio and damping) is spread over the lanes
-// as well; it took a third of a round when the owning lane did it alone.
+// pow of both), which makes a round's evaluation 4 pow + 2 atan2 + 3 sincos long: the pending trial,
+// those that follow if it is rejected, and the probes of the one likely to be accepted (1.3 rounds
+// an iteration; 1.4 with always two trials).  The state machine's own arithmetic (the Jacobian's six divisions, the normal equations, the
+// steps, gain ratios and damping of all trials) is spread over the lanes as well; it took a third
+// of a round when the owning lane did it alone.  A round takes 21-23 us (26-29 before, of one third
+// of an iteration while four searches shared a warp).  Longest searches of a jammed cell of 12,800
+// particles: FP64 pass 5.3 -> 3.4 ms; a servo specimen of 2,197: 3.1 -> 1.6 ms.
 //
-// Every value is computed by the operations of k_contacts_lm's state machine on the same operands,
-// in the same order, so that the results are the same bit for bit: speculative points that a search
-// does not come to are dropped.
+// Every value is computed by lmder2's operations on the same operands, in the same order, so that a
+// search's results do not depend on the schedule: speculative points that it does not come to are
+// dropped.
 
 static const int WS_LANES = 5, WS_POINTS = 6;
 

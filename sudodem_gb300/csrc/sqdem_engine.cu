@@ -1382,7 +1382,7 @@ __device__ int screenSeparatedNM(const BodyView& b1, const BodyView& b2, double 
 
 // Pass 1 over the table: every entry that needs no Levenberg-Marquardt iteration is finished
 // here (bound-separated pairs, wall contacts, sphere pairs, bounding-sphere rejections, pairs the
-// FP32 screen proves separated at the LM start point); the rest is queued for k_contacts_lm.
+// FP32 screen proves separated at the LM start point); the rest is queued for pass 2.
 __global__ void __launch_bounds__(128, 3) k_contacts_pre(Dev d) {
   const SceneState& S = *d.S;
   if (S.skip) return;
@@ -1900,7 +1900,7 @@ __global__ void __launch_bounds__(LM_BS) k_contacts_nm(Dev d) {
 // A search that meets a decision inside its band, or an evaluation the double-float routines
 // do not reproduce (ill: exactly axis-aligned normals, non-finite values), is deferred whole:
 // the lane drops it without writing anything and appends it to the fallback queue, which the
-// FP64 kernel (k_contacts_lm on that queue) then runs from the same inputs.  The starting
+// FP64 kernel (k_search_warp on that queue) then runs from the same inputs.  The starting
 // angles (table or centre line, FP64), the contact points, depth, normal, precompute, Ip2 and
 // the law stay FP64.
 
@@ -1938,7 +1938,7 @@ __device__ __forceinline__ void shapeFromGlobal(SqShape& s, const Dev& d, int b)
 // One lmder2 call ended: the restart rules of Superquadrics_Ig2.cpp:2013-2053 (as lmCallEnd).
 // Returns LMF_MORE when a restarted call begins, LMF_END when the contact's geometry is final,
 // LMF_DEFER when a restart decision falls inside its band.
-__device__ __noinline__ int lmfCallEnd(const Dev& d, LMF& L, int id1, int id2, D3 pB) {
+__device__ __noinline__ int lmfCallEnd(const Dev& d, LMF& L, int id1, int id2, const ff* pB) {
   for (;;) {
     L.calls++; L.iters += L.k; L.maxit += (L.stop == 3);
     bool restart = false;
@@ -1957,7 +1957,7 @@ __device__ __noinline__ int lmfCallEnd(const Dev& d, LMF& L, int id1, int id2, D
           shapeFromGlobal(A, d, id1);
           shapeFromGlobal(B, d, id2);
           const D3 p2a = d3(ffToD(L.P2[0]), ffToD(L.P2[1]), ffToD(L.P2[2]));
-          const D3 p1b = d3(ffToD(L.P1[0]), ffToD(L.P1[1]), ffToD(L.P1[2])) - pB;
+          const D3 p1b = d3(ffToD(L.P1[0]), ffToD(L.P1[1]), ffToD(L.P1[2])) - d3(ffToD(pB[0]), ffToD(pB[1]), ffToD(pB[2]));
           const double va = insideValue(A, p2a), vb = insideValue(B, p1b);
           if (!(fabs(va - 1.0) >= 1e-9) || !(fabs(vb - 1.0) >= 1e-9)) return LMF_DEFER;
           if (!(1 > va) || !(1 > vb)) { L.phase = 2; restart = true; }
@@ -1978,168 +1978,22 @@ __device__ __noinline__ int lmfCallEnd(const Dev& d, LMF& L, int id1, int id2, D
   }
 }
 
-// Pass 2, mixed form (see the section comment).  Rounds of one double-float evaluation per
-// lane; once the queue is drained, the lanes without a contact evaluate the points the running
-// searches of their warp ask for next (lmfPlan), as in k_contacts_lm.  Each lane's search state
-// and each round's evaluation results live in shared memory and the bodies' double-float shapes
-// are read from bodyFF, so that the registers serve the evaluation (more resident warps hide
-// the latency of its dependent FP32 chains).  A finished search's geometry goes to a compact
-// list in the merge buffer (table B); k_contacts_lm_ff_finish completes it in FP64.
-static const int FFEV_WORDS = 27;   // c, p1, p2, d (ff, 3 each), sep (ff), ill
-__global__ void __launch_bounds__(LM_BS) k_contacts_lm_ff(Dev d) {
-  __shared__ LMF sL[LM_BS];
-  __shared__ float sEv[FFEV_WORDS][LM_BS];
-  __shared__ int sId[2][LM_BS];
-  __shared__ float sPB[6][LM_BS];
-  __shared__ float4 slotQ[LM_BS];
-  __shared__ int slotOwner[LM_BS];
-  const SceneState& S = *d.S;
-  const int nFront = S.lmCount, count = S.lmCount + S.nmShort;   // long searches first
-  const int t = threadIdx.x;
-  const int lane = t & 31;
-  const int wbase = t & ~31;
-  const bool spread = d.prm->lmSpread != 0;
-  unsigned long long ev32 = 0, deferred = 0;
-  unsigned roundsMax = 0;
-  LMF& L = sL[t];
-  // a warp holds 32 searches while the queue has work (capping it to leave spare slots for the
-  // longest searches, as the FP64 kernel does for its long-search queue, was measured slower
-  // here: the double-float rounds are short and the bulk throughput dominates)
-  const int cap = 32;
-  bool active = false, done = false;   // done: warp-uniform, the queue is empty
-  while (true) {
-    const unsigned idleAll = __ballot_sync(0xffffffffu, !active);
-    const int want = done ? 0 : min(__popc(idleAll), cap - (32 - __popc(idleAll)));
-    if (want > 0) {
-      int base = 0;
-      if (lane == 0) base = atomicAdd(&d.S->lmHead, want);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      const int r = __popc(idleAll & ((1u << lane) - 1));
-      if (base + want >= count) done = true;
-      if (!active && r < want) {
-        const int idx = base + r;
-        if (idx < count) {
-          const int e = idx < nFront ? d.lmQueue[idx] : d.lmQueue[d.qCap - 1 - (idx - nFront)];
-          const unsigned fl = d.A.flags[e];
-          int id1, id2;
-          entryIds(d, e, fl, id1, id2);
-          const D3 shift2 = cellShift(S, d.A.cd[e]);
-          const D3 pa = xyz(d.pos[id1]), pb = xyz(d.pos[id2]) + shift2;
-          sId[0][t] = id1; sId[1][t] = id2;
-          const ff px = ffFromD(pb.x - pa.x), py = ffFromD(pb.y - pa.y), pz = ffFromD(pb.z - pa.z);
-          sPB[0][t] = px.hi; sPB[1][t] = px.lo; sPB[2][t] = py.hi; sPB[3][t] = py.lo; sPB[4][t] = pz.hi; sPB[5][t] = pz.lo;
-          L.e = e;
-          L.E = 4e-13f * (d.bodyFF[id1].rmax + d.bodyFF[id2].rmax);
-          L.isNew = !(fl & F_GEOM);
-          if (L.isNew) { double para[2]; centerLine(pa, pb, para); L.p0 = ffFromD(para[0]); L.p1 = ffFromD(para[1]); }
-          else { const double2 an = d.A.angle[e]; L.p0 = ffFromD(an.x); L.p1 = ffFromD(an.y); }
-          L.fromCenter = L.isNew;
-          L.phase = 0; L.calls = 0; L.iters = 0; L.maxit = 0; L.rounds = 0;
-          lmfStartSolve(L);
-          active = true;
-        }
-      }
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (!act) {
-      if (done) break;
-      continue;
-    }
-    const int nA = __popc(act);
-    const bool drained = spread && done;
-    int spc, base, jmax;
-    allocSlots(active, active ? L.rounds : 0u, drained ? 32 : nA, 1, spc, base, jmax);
-    slotOwner[t] = -1;
-    __syncwarp();
-    if (active) lmfPlan(L, &slotQ[wbase + base], &slotOwner[wbase + base], spc, lane);
-    __syncwarp();
-    {
-      // lanes without a slot evaluate the warp's first slot (whose owner always exists) so that
-      // every lane computes on valid inputs
-      const int own = slotOwner[t];
-      const int slot = own >= 0 ? t : wbase;
-      const int src = wbase + slotOwner[slot];
-      const float4 q = slotQ[slot];
-      const ff pB[3] = {mkff(sPB[0][src], sPB[1][src]), mkff(sPB[2][src], sPB[3][src]), mkff(sPB[4][src], sPB[5][src])};
-      FFEval v;
-      ffDisfunction(d.bodyFF[sId[0][src]], d.bodyFF[sId[1][src]], pB, mkff(q.x, q.y), mkff(q.z, q.w), v);
-      for (int i = 0; i < 3; i++) {
-        sEv[2 * i][t] = v.c[i].hi; sEv[2 * i + 1][t] = v.c[i].lo;
-        sEv[6 + 2 * i][t] = v.p1[i].hi; sEv[7 + 2 * i][t] = v.p1[i].lo;
-        sEv[12 + 2 * i][t] = v.p2[i].hi; sEv[13 + 2 * i][t] = v.p2[i].lo;
-        sEv[18 + 2 * i][t] = v.d[i].hi; sEv[19 + 2 * i][t] = v.d[i].lo;
-      }
-      sEv[24][t] = v.sep.hi; sEv[25][t] = v.sep.lo; sEv[26][t] = v.ill ? 1.f : 0.f;
-      if (own >= 0) ev32++;
-    }
-    __syncwarp();
-    if (active) {
-      L.rounds++;
-      for (int j = 0; j < spc; j++) {
-        const int si = wbase + base + j;
-        if (!(slotOwner[si] == lane && sameFF(slotQ[si], L.q0, L.q1))) continue;
-        FFEval w;
-        for (int i = 0; i < 3; i++) {
-          w.c[i] = mkff(sEv[2 * i][si], sEv[2 * i + 1][si]);
-          w.p1[i] = mkff(sEv[6 + 2 * i][si], sEv[7 + 2 * i][si]);
-          w.p2[i] = mkff(sEv[12 + 2 * i][si], sEv[13 + 2 * i][si]);
-          w.d[i] = mkff(sEv[18 + 2 * i][si], sEv[19 + 2 * i][si]);
-        }
-        w.sep = mkff(sEv[24][si], sEv[25][si]);
-        w.ill = sEv[26][si] != 0.f;
-        int r = lmfConsume(L, w);
-        if (r == LMF_END) r = lmfCallEnd(d, L, sId[0][t], sId[1][t],
-                                         d3(ffToD(mkff(sPB[0][t], sPB[1][t])), ffToD(mkff(sPB[2][t], sPB[3][t])),
-                                            ffToD(mkff(sPB[4][t], sPB[5][t]))));
-        if (r == LMF_END) {
-          // the search's geometry to the finish list (merge buffer), completed in FP64 by
-          // k_contacts_lm_ff_finish
-          const int i = atomicAdd(&d.S->nmFin, 1);
-          d.B.owner[i] = L.e;
-          d.B.angle[i] = make_double2(ffToD(L.p0), ffToD(L.p1));
-          d.B.p1[i] = make_double4(ffToD(L.P1[0]), ffToD(L.P1[1]), ffToD(L.P1[2]), 0);
-          d.B.p2[i] = make_double4(ffToD(L.P2[0]), ffToD(L.P2[1]), ffToD(L.P2[2]), 0);
-          d.B.normal[i] = make_double4(ffToD(L.c[0]), ffToD(L.c[1]), ffToD(L.c[2]), 0);
-          d.B.cd[i] = make_int4((int)L.calls, (int)L.iters, (int)L.maxit, L.touching ? 1 : 0);
-        } else if (r == LMF_DEFER) {
-          d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = L.e;
-          deferred++;
-        }
-        if (r != LMF_MORE) {
-          active = false;
-          roundsMax = max(roundsMax, L.rounds);
-          break;   // the rest of this round's slots were planned for the call that ended
-        }
-      }
-    }
-    __syncwarp();
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ev32 += __shfl_down_sync(0xffffffffu, ev32, o);
-    deferred += __shfl_down_sync(0xffffffffu, deferred, o);
-    roundsMax = max(roundsMax, __shfl_down_sync(0xffffffffu, roundsMax, o));
-  }
-  if (lane == 0) {
-    atomicAdd(&d.S->err[E_EVAL32], ev32);
-    atomicAdd(&d.S->err[E_FALLBACK], deferred);
-    atomicMax(&d.S->err[E_ROUNDS_MAX_FF], (unsigned long long)roundsMax);
-  }
-}
+#include "sq_ff_search.cuh"
 
 // The end of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go (Superquadrics_Ig2.cpp:
-// 2054-2095) in FP64 for the searches k_contacts_lm_ff finished, one thread per search: the
+// 2054-2095) in FP64 for the searches the double-float kernels finished, one thread per search: the
 // contact points in the global frame, the depth (deferred to the FP64 kernel when inside the
 // band of the law's contact gate), normal, precompute, then Ip2 and the law.
-__global__ void __launch_bounds__(128) k_contacts_lm_ff_finish(Dev d) {
+__global__ void __launch_bounds__(128) k_ff_finish(Dev d) {
   const SceneState& S = *d.S;
   if (S.skip) return;
-  const int n = S.nmFin;
+  const int n = d.Q->nF;
   const double dt = d.prm->dt;
   Counters cnt = {0, 0, 0, 0, 0};
   unsigned long long deferred = 0;
   for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    if (i >= n) continue;
+    if (i0 + threadIdx.x >= n) continue;
+    const int i = d.waveF[i0 + threadIdx.x];
     const int e = d.B.owner[i];
     const int4 info = d.B.cd[i];
     const unsigned fl = d.A.flags[e];
@@ -2151,14 +2005,15 @@ __global__ void __launch_bounds__(128) k_contacts_lm_ff_finish(Dev d) {
     g.lmCalls = info.x; g.lmIters = info.y; g.lmStop = 0; g.nanNormal = false;
     g.isShearNew = isNew ? true : (d.A.depth[e] <= 0);
     g.cp = isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]);
+    auto unpack = [](double4 v) { return d3(ffToD(ffUnpack(v.x)), ffToD(ffUnpack(v.y)), ffToD(ffUnpack(v.z))); };
     const double2 an = d.B.angle[i];
-    g.ang0 = an.x; g.ang1 = an.y; g.angSet = true;
+    g.ang0 = ffToD(ffUnpack(an.x)); g.ang1 = ffToD(ffUnpack(an.y)); g.angSet = true;
     bool ok = true;
     if (!info.w) {
       g.precomputed = false; g.depth = 0; g.isShearNew = true;
     } else {
-      const D3 P1 = b1.pos + xyz(d.B.p1[i]), P2 = b1.pos + xyz(d.B.p2[i]);
-      const D3 contact = xyz(d.B.normal[i]);
+      const D3 P1 = b1.pos + unpack(d.B.p1[i]), P2 = b1.pos + unpack(d.B.p2[i]);
+      const D3 contact = unpack(d.B.phys[i]);
       const double pDepth = dot(P1 - P2, contact);
       const double E = 4e-13 * (b1.shpA.w + b2.shpA.w);
       if (!(fabs(pDepth - 1e-18) >= E)) ok = false;   // the law's contact gate inside its band
@@ -2824,6 +2679,15 @@ static int waveRounds(const sqdem_ctx* c, const Dev& d) {
   return std::max(4, std::min(WAVE_MAX_ROUNDS, (int)std::lround(3.0 * std::log2(std::max(c->load, d.NP) / 1e4))));
 }
 
+// Mixed form: double-float rounds before the searches left get a warp each.  None up to 8,000 particles
+// (2,197: 25.4 ms for ten steps, 26.5 with four rounds), then one more for each doubling (12,800:
+// 19.1 ms for five steps with four, 21.2 with none; 200,000: 38.3 for three with eight, 39.8 with four).
+static const int FF_WARP_MAX = 8000;
+static int ffRounds(const sqdem_ctx* c, const Dev& d) {
+  const int n = std::max(c->load, d.NP);
+  return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
+}
+
 // The contact stage on c->stream: pass 1, then the searches of the selected contact model
 // (and, for Hertz-Mindlin, the finish pass of the contacts found touching).
 static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
@@ -2847,13 +2711,26 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
       k_search_warp<<<ws, LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
       cudaEventRecord(c->join, c->stream2);
       k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
-      k_contacts_lm_ff<<<grid, LM_BS, 0, s>>>(d);
+      const int blocks = c->numSMs * searchBlocksPerSM(c);
+      const int ffw = std::min(blocks, nblk(d.Pcap, LM_BS / 32));
+      const int rounds = ffRounds(c, d);
+      if (rounds == 0) k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 0, 0);
+      else {
+        const int ff = std::min(blocks, nblk(d.Pcap, LM_BS / 2));
+        k_ff_trial<true><<<ff, LM_BS, 0, s>>>(d, 0);
+        k_ff_probe<<<ff, LM_BS, 0, s>>>(d, 0);
+        for (int r = 1; r < rounds; r++) {
+          k_ff_trial<false><<<ff, LM_BS, 0, s>>>(d, r);
+          k_ff_probe<<<ff, LM_BS, 0, s>>>(d, r);
+        }
+        k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 1, rounds);
+      }
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
-      k_contacts_lm_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
+      k_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
       k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_DEFERRED, 0);
       cudaStreamWaitEvent(s, c->join, 0);
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
-      c->launches += 6;
+      c->launches += 6 + 2 * rounds;
     } else if (std::max(c->load, d.NP) <= WARP_SEARCH_MAX) {
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
       k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_ALL, 0);
@@ -3047,7 +2924,7 @@ sqdem_status sqdem_create(sqdem_ctx** out, const sqdem_config* cfg) {
     int nb = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_wave_trial<false>, LM_BS, 0));
     c->lmBlocksPerSM = nb > 0 ? nb : 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_contacts_lm_ff, LM_BS, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ff_trial<false>, LM_BS, 0));
     c->lmBlocksPerSMmixed = nb > 0 ? nb : 1;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_contacts_nm, LM_BS, 0));
     c->nmBlocksPerSM = nb > 0 ? nb : 1;

@@ -96,19 +96,20 @@ def test_batch_time_e2e_round_trips_kinematics(gpu):
     b.close()
 
 
-@pytest.mark.parametrize("sizes", [(1, 17, 33, 250, 15800), (2, 16400)])
-def test_searches_in_rounds_equal_searches_by_warps(gpu, sizes):
-    """The FP64 form searches scenes of up to 16,000 particles one contact per warp, larger ones (and
-    the scenes of a larger batch) in rounds over compact lists: the same operations per contact, so
-    the same bits, whatever share of the lists' last warps is filled."""
+@pytest.mark.parametrize("precision,sizes", [("fp64", (1, 17, 33, 250, 15800)), ("fp64", (2, 16400)),
+                                             ("mixed", (1, 17, 33, 250, 7800)), ("mixed", (2, 8100))])
+def test_searches_in_rounds_equal_searches_by_warps(gpu, precision, sizes):
+    """Scenes of up to 16,000 particles (8,000 in the mixed form) are searched one contact per warp,
+    larger ones, and the scenes of a larger batch, in rounds over compact lists: the same operations
+    per contact, so the same bits, whatever share of the lists' last warps is filled."""
     ss = [assemblies.cubic_specimen(n, seed=31 + i, eps_range=(0.3, 1.7), spacing=2.1e-3, wall_gap=0.0)
           for i, n in enumerate(sizes)]
-    b = Batch(len(ss))
+    b = Batch(len(ss), precision=precision)
     b.load(ss)
     b.step(6)
     b.sync()
     for i, spec in enumerate(ss):
-        e = Engine()
+        e = Engine(precision=precision)
         e.load(spec)
         e.step(6)
         e.sync()
