@@ -410,12 +410,13 @@ long sqdem_adj_num_pairs(sqdem_adj* adj);
  * shearForce3, then the force on id1 in the last step (3) and whether it was applied. */
 sqdem_status sqdem_adj_get_pairs(sqdem_adj* adj, double* out16);
 /* Forward kernel of the pairs: cooperative = 1 (default) shares each Disfunction evaluation
- * among six lanes (the independent pow calls of each level on separate lanes), 0 runs the
- * pair on one thread.  Both give bitwise the same results. */
+ * among five lanes of a warp (the independent pow calls of each level on separate lanes), which
+ * evaluates six points at a time, 0 runs the pair on one thread.  Both give bitwise the same results. */
 sqdem_status sqdem_adj_set_forward(sqdem_adj* adj, int cooperative);
 /* Shape of the pairs' reverse-step kernel, which replays each pair's narrowphase and law in
  * dual numbers: 0 one thread per pair with all seventeen tangent components, 1 three lanes with
- * six each, 2 two lanes with nine, 3 (default) six lanes with three.  Every shape gives bitwise
+ * six each, 2 two lanes with nine, 3 (default) six slices with three, five lanes of a warp each
+ * that share an evaluation's pow calls.  Every shape gives bitwise
  * the same gradients. */
 sqdem_status sqdem_adj_set_replay(sqdem_adj* adj, int shape);
 /* Resident blocks per SM of the grouped reverse-step kernels (grid-stride over the pairs;

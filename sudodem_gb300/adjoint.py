@@ -163,8 +163,8 @@ class AdjointWindow:
                         out.astype(np.int64).tolist()))
 
     def set_forward(self, cooperative=True):
-        """Forward kernel of the pairs: six lanes share each evaluation (default) or one thread
-        per pair; the results are bitwise the same."""
+        """Forward kernel of the pairs: a warp per pair (default) or one thread; the results are
+        bitwise the same."""
         self._check(self.lib.sqdem_adj_set_forward(self.h, 1 if cooperative else 0))
 
     def num_pairs(self):

@@ -153,8 +153,12 @@ __host__ __device__ __noinline__ void disfunction(const Shape<T>& A, const Shape
   if (val(dot(contact, d)) > 0) stop_flag = true;
 }
 // The Disfunction evaluation lmder2 calls: in sequence on one thread (every instantiation),
-// or by a group of six lanes of a warp (CoopEval, forward kernel only).
+// or by groups of five lanes of a warp (WarpEval in the forward kernel, TangentEval in the reverse
+// kernel).  AHEAD: lmder2 names the points it may ask for next (plan), which the evaluation takes
+// along.
 struct SeqEval {
+  static constexpr bool AHEAD = false;
+  SQA_HD void plan(int, double, double) const {}
   template <class T>
   SQA_HD void operator()(const Shape<T>& A, const Shape<T>& B, const T& pa0, const T& pa1, V3<T>& center, V3<T>& p1,
                          V3<T>& p2, bool& stop_flag) const {
@@ -162,66 +166,122 @@ struct SeqEval {
   }
 };
 
-// Disfunction by six lanes: lanes g0..g0+2 compute body A's support point, g0+3..g0+5 body
-// B's, each triple running the independent pow calls of one level of Normal2Phi + getSurface
-// on separate lanes (Y X W | t u v | Z | pc1 w), so that the dependency chain of one evaluation
-// is 4 pow + 2 atan2 + 4 sincos instead of 18 pow + 4 atan2 + 6 sincos.  Every value is the
-// result of the same operation on the same operands as in disfunction: bitwise the same.
-struct CoopEval {
-  unsigned mask;   // the group's six lanes
-  int g0, sub;     // first lane of the group, this lane's place in it
-#ifdef __CUDA_ARCH__
-  __device__ double pick(double v, int src) const { return __shfl_sync(mask, v, src); }
-  __device__ V3<double> support(const Shape<double>& s, const V3<double>& n, int part, int l0) const {
-    double b, e;
-    if (part == 0) { b = fabs(s.ry * n.y); e = s.i1; }
-    else if (part == 1) { b = fabs(s.rx * n.x); e = s.i1; }
-    else { b = fabs(s.rx * n.x); e = s.i2; }
-    const double r1 = pow(b, e);
-    const double Y = pick(r1, l0), X = pick(r1, l0 + 1), W = pick(r1, l0 + 2);
-    const double ph0 = atan2(tsgn(n.y) * Y, tsgn(n.x) * X);
-    double s0, c0;
-    sincos(ph0, &s0, &c0);
-    if (part == 0) { b = fabs(c0); e = s.a1; }
-    else if (part == 1) { b = fabs(c0); e = s.e1; }
-    else { b = fabs(s0); e = s.e1; }
-    const double r2 = pow(b, e);
-    const double t = pick(r2, l0), u = pick(r2, l0 + 1), v = pick(r2, l0 + 2);
-    const double Z = pow(fabs(s.rz * n.z * t), s.i2);
-    const double ph1 = atan2(tsgn(n.z) * Z, W);
-    double s1, c1;
-    sincos(ph1, &s1, &c1);
-    if (part == 1) { b = fabs(s1); e = s.e2; } else { b = fabs(c1); e = s.e2; }
-    const double r3 = pow(b, e);
-    const double pc1 = pick(r3, l0), w = pick(r3, l0 + 1);
-    V3<double> r;
-    r.x = tsgn(c0) * s.rx * u * pc1;
-    r.y = tsgn(s0) * s.ry * v * pc1;
-    r.z = tsgn(s1) * s.rz * w;
-    return r;
+// Disfunction by five lanes g0..g0+4 (place r): two per body (0, 1: A; 2, 3: B), which run the
+// independent pow calls of a level of Normal2Phi + getSurface side by side, and a fifth that takes
+// the ninth pow of both: the dependency chain of one evaluation is 4 pow + 2 atan2 + 3 sincos instead
+// of 18 pow + 4 atan2 + 6 sincos.  Every value (and tangent, for T a dual number) is the result of
+// the same operation on the same operands as in disfunction: bitwise the same.
+static const int CO_LANES = 5;
+#ifdef __CUDACC__
+__device__ __forceinline__ double pick(unsigned mask, double v, int src) { return __shfl_sync(mask, v, src); }
+template <int N> __device__ __forceinline__ Dual<N> pick(unsigned mask, const Dual<N>& v, int src) {
+  Dual<N> r;
+  r.v = __shfl_sync(mask, v.v, src);
+#pragma unroll
+  for (int k = 0; k < N; k++) r.d[k] = __shfl_sync(mask, v.d[k], src);
+  return r;
+}
+template <class T>
+__device__ __forceinline__ void coopPoint(unsigned mask, int g0, int r, const Shape<T>& A, const Shape<T>& B, const T& pa0,
+                                          const T& pa1, V3<T>& p1, V3<T>& p2, bool& apart) {
+  const bool isB = r == 2 || r == 3, k = r == 1 || r == 3, extra = r == 4;
+  const int mate = extra ? g0 + 1 : g0 + (r ^ 1);
+  const Shape<T>& s = isB ? B : A;
+  T sv, cv;
+  tsincos(k ? pa1 : pa0, &sv, &cv);
+  const T sa0 = pick(mask, sv, g0), ca0 = pick(mask, cv, g0), sa1 = pick(mask, sv, g0 + 1), ca1 = pick(mask, cv, g0 + 1);
+  const V3<T> c = mk<T>(ca0 * ca1, sa0 * ca1, sa1);
+  // local normal +-R^T c: x on k = 1, y on k = 0, z on both
+  T na = (k ? s.R.m[0] : s.R.m[1]) * c.x + ((k ? s.R.m[3] : s.R.m[4]) * c.y + (k ? s.R.m[6] : s.R.m[7]) * c.z);
+  T nz = s.R.m[2] * c.x + (s.R.m[5] * c.y + s.R.m[8] * c.z);
+  if (isB) { na = (-1.0) * na; nz = (-1.0) * nz; }
+  const double no = __shfl_sync(mask, val(na), mate);
+  const double nx = k ? val(na) : no, ny = k ? no : val(na);
+  const T b1 = tfabs((k ? s.rx : s.ry) * na);
+  const T v1 = tpow(b1, s.i1);   // Y | X
+  const T w1 = pick(mask, v1, mate);
+  const T ph0 = tatan2(tsgn(ny) * (k ? w1 : v1), tsgn(nx) * (k ? v1 : w1));
+  T s0, c0;
+  tsincos(ph0, &s0, &c0);
+  const T v2 = tpow(extra ? tfabs(s0) : k ? b1 : tfabs(c0), extra ? s.e1 : k ? s.i2 : s.a1);   // t | W | v of A
+  const T s0B = pick(mask, s0, g0 + 2);
+  const T v3 = tpow(extra ? tfabs(s0B) : k ? tfabs(c0) : tfabs(s.rz * nz * v2), extra ? B.e1 : k ? s.e1 : s.i2);   // Z | u | v of B
+  const T w2 = pick(mask, v2, mate), w3 = pick(mask, v3, mate);
+  const T vA = pick(mask, v2, g0 + 4), vB = pick(mask, v3, g0 + 4);
+  const T ph1 = tatan2(tsgn(nz) * (k ? w3 : v3), k ? v2 : w2);
+  T s1, c1;
+  tsincos(ph1, &s1, &c1);
+  const T v4 = tpow(tfabs(k ? s1 : c1), s.e2);   // |cos phi1|^eps2 | |sin phi1|^eps2
+  const T w4 = pick(mask, v4, mate);
+  const T pc1 = k ? w4 : v4, ps1 = k ? v4 : w4;
+  const T rxy = (k ? tsgn(s0) * s.ry : tsgn(c0) * s.rx) * (k ? (isB ? vB : vA) : w3) * pc1;
+  const T rz = tsgn(s1) * s.rz * ps1;
+  const T rot = pick(mask, rxy, mate);
+  const T rX = k ? rot : rxy, rY = k ? rxy : rot;
+  const T pxy = ((k ? s.R.m[3] : s.R.m[0]) * rX + ((k ? s.R.m[4] : s.R.m[1]) * rY + (k ? s.R.m[5] : s.R.m[2]) * rz)) +
+                (k ? s.pos.y : s.pos.x);
+  const T pz = (s.R.m[6] * rX + (s.R.m[7] * rY + s.R.m[8] * rz)) + s.pos.z;
+  p1 = mk<T>(pick(mask, pxy, g0), pick(mask, pxy, g0 + 1), pick(mask, pz, g0));
+  p2 = mk<T>(pick(mask, pxy, g0 + 2), pick(mask, pxy, g0 + 3), pick(mask, pz, g0 + 2));
+  apart = dot(vval(c), vval(p2) - vval(p1)) > 0;
+}
+
+// The forward kernel's evaluation: one pair per warp, six groups of five lanes, each at a point of
+// its own: the one asked for and up to five that lmder2 planned.  A point it then asks for (same
+// bits) is answered from its group's lanes.
+struct WarpEval {
+  static constexpr bool AHEAD = true;
+  int grp, g0, r;
+  mutable double q0, q1, n0, n1;   // this group's point; the planned one
+  mutable bool have, planned, apart;
+  mutable V3<double> e1, e2;
+  __device__ explicit WarpEval(int lane) {
+    grp = lane < 30 ? lane / CO_LANES : 0; g0 = grp * CO_LANES; r = lane < 30 ? lane - g0 : lane - 30;
+    have = planned = apart = false;
+    q0 = q1 = n0 = n1 = 0;
+    e1 = e2 = zero3<double>();
   }
-#endif
-  SQA_HD void operator()(const Shape<double>& A, const Shape<double>& B, const double& pa0, const double& pa1,
-                         V3<double>& center, V3<double>& p1, V3<double>& p2, bool& stop_flag) const {
-#ifdef __CUDA_ARCH__
-    double sa0, ca0, sa1, ca1;
-    sincos(pa0, &sa0, &ca0);
-    sincos(pa1, &sa1, &ca1);
-    const V3<double> contact = mk<double>(ca0 * ca1, sa0 * ca1, sa1);
-    const int body = sub / 3, part = sub - 3 * body;
-    const Shape<double>& Sh = body ? B : A;
-    const V3<double> n = body ? (-1.0) * mulL(B.R, contact) : mulL(A.R, contact);
-    const V3<double> pt = mulG(Sh.R, support(Sh, n, part, g0 + 3 * body)) + Sh.pos;
-    p1 = mk<double>(pick(pt.x, g0), pick(pt.y, g0), pick(pt.z, g0));
-    p2 = mk<double>(pick(pt.x, g0 + 3), pick(pt.y, g0 + 3), pick(pt.z, g0 + 3));
-    const V3<double> d = p2 - p1;
+  __device__ void plan(int i, double a, double b) const { if (grp == i) { n0 = a; n1 = b; planned = true; } }
+  __device__ unsigned match(double a, double b) const {
+    return __ballot_sync(0xffffffffu, have && __double_as_longlong(q0) == __double_as_longlong(a) &&
+                                          __double_as_longlong(q1) == __double_as_longlong(b));
+  }
+  __device__ void operator()(const Shape<double>& A, const Shape<double>& B, double pa0, double pa1, V3<double>& center,
+                             V3<double>& p1, V3<double>& p2, bool& stop_flag) const {
+    const unsigned FULL = 0xffffffffu;
+    unsigned m = match(pa0, pa1);
+    if (!m) {
+      const bool own = planned && grp > 0;
+      q0 = own ? n0 : pa0; q1 = own ? n1 : pa1;
+      coopPoint(FULL, g0, r, A, B, q0, q1, e1, e2, apart);
+      have = true;
+      m = 1u;   // group 0 holds the point asked for
+    }
+    planned = false;
+    const int l = __ffs(m) - 1;
+    p1 = mk<double>(pick(FULL, e1.x, l), pick(FULL, e1.y, l), pick(FULL, e1.z, l));
+    p2 = mk<double>(pick(FULL, e2.x, l), pick(FULL, e2.y, l), pick(FULL, e2.z, l));
     center = 0.5 * (p1 + p2);
-    if (dot(contact, d) > 0) stop_flag = true;
-#else
-    disfunction(A, B, pa0, pa1, center, p1, p2, stop_flag);
-#endif
+    if ((__ballot_sync(FULL, apart) >> l) & 1u) stop_flag = true;
   }
 };
+
+// The reverse kernel's evaluation: five lanes per evaluation, for a slice of the tangents.
+struct TangentEval {
+  static constexpr bool AHEAD = false;
+  unsigned mask;
+  int g0, r;
+  __device__ void plan(int, double, double) const {}
+  template <class T>
+  __device__ void operator()(const Shape<T>& A, const Shape<T>& B, const T& pa0, const T& pa1, V3<T>& center, V3<T>& p1,
+                             V3<T>& p2, bool& stop_flag) const {
+    bool apart;
+    coopPoint(mask, g0, r, A, B, pa0, pa1, p1, p2, apart);
+    center = 0.5 * (p1 + p2);
+    if (apart) stop_flag = true;
+  }
+};
+#endif
 
 template <class T> SQA_HD void centerLine(const V3<T>& pos1, const V3<T>& pos2, T para[2]) {
   const V3<T> d0 = pos2 - pos1;
@@ -321,6 +381,10 @@ __host__ __device__ __noinline__ void lmder2(const Shape<T>& A, const Shape<T>& 
   int nu = 2, stop = 0, k;
   V3<T> P1, P2, C;
   o.contact = zero3<T>();
+  if constexpr (E::AHEAD) {
+    ev.plan(1, p[0] + Dp0, p[1]);
+    ev.plan(2, p[0], p[1] + Dp1);
+  }
   ev(A, B, p[0], p[1], C, P1, P2, stop_flag);
   br.surf(A, B, p[0], p[1]);
   V3<T> pf = P2 - P1;
@@ -364,6 +428,18 @@ __host__ __device__ __noinline__ void lmder2(const Shape<T>& A, const Shape<T>& 
       if (br(DpL2 < 1e-5)) { stop = 2; break; }
       const T q0 = p[0] + Dp0, q1 = p[1] + Dp1;
       if (br(DpL2 >= (val(pL2) + 1e-3) / (1e-12 * 1e-12))) { stop = 4; break; }
+      if constexpr (E::AHEAD) {
+        // the probes at the trial, should it be accepted; the next trial, with its probes, should it
+        // be rejected (by the operations below)
+        ev.plan(1, q0 + Dp0, q1);
+        ev.plan(2, q0, q1 + Dp1);
+        const double m = mu * (double)nu, i00 = diag0 + m, i11 = diag1 + m, i_a = i00 * i11 - j01 * j01;
+        const double E0 = (jt0 * i11 - jt1 * j01) / i_a, E1 = (jt1 * i00 - jt0 * j01) / i_a;
+        const double r0 = p[0] + E0, r1 = p[1] + E1;
+        ev.plan(3, r0, r1);
+        ev.plan(4, r0 + E0, r1);
+        ev.plan(5, r0, r1 + E1);
+      }
       ev(A, B, q0, q1, C, P1, P2, stop_flag);
       br.surf(A, B, q0, q1);
       o.evals++;
@@ -750,19 +826,18 @@ __global__ void __launch_bounds__(128) k_fwd_contacts(Consts C, State S, StepOut
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < C.P) fwdContact(C, S, O, step, c);
 }
-// The same with six lanes per pair (five pairs per warp, lanes 30 and 31 idle): each
-// Disfunction evaluation is shared by the group (CoopEval); the group's first lane writes.
+// The same with a warp per pair (WarpEval).  A step ends with its longest search, so what counts is
+// the chain of dependent evaluations: with the evaluation's pow calls side by side and the points
+// that follow either outcome of a trial evaluated with it, an iteration takes 1.4 rounds of some 700
+// FP64 instructions (64-76 cycles each) instead of 3.9.  1,500 particles, 16,309 pairs: 2.2 ms a
+// step (4.2 with six lanes a pair and no points ahead).
 static const int COOP_WARPS = 4;
 __global__ void __launch_bounds__(32 * COOP_WARPS) k_fwd_contacts_coop(Consts C, State S, StepOut O, int step) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gw = lane / 6, sub = lane - 6 * gw;
-  const int c = (blockIdx.x * COOP_WARPS + warp) * 5 + gw;
-  if (gw >= 5 || c >= C.P) return;
-  CoopEval ev;
-  ev.mask = 0x3Fu << (6 * gw);
-  ev.g0 = 6 * gw;
-  ev.sub = sub;
-  fwdContact(C, S, O, step, c, ev, sub == 0);
+  const int lane = threadIdx.x & 31;
+  const int c = blockIdx.x * COOP_WARPS + (threadIdx.x >> 5);
+  if (c >= C.P) return;
+  const WarpEval ev(lane);
+  fwdContact(C, S, O, step, c, ev, lane == 0);
 }
 
 // ForceContainer sum of one body over its pairs, in list order (NewtonIntegrator's view)
@@ -1131,6 +1206,68 @@ __global__ void __launch_bounds__(32 * GRP_WARPS) k_bwd_contacts_grp(Consts C, S
   }
 }
 
+// The same reverse step with a warp per pair: six slices of TG tangent components, each on five lanes
+// that share every evaluation (TangentEval).  A step is bound by its longest replay, a chain of
+// dependent dual-number evaluations of which only some hundreds of pairs have any: with 4 powers in
+// a row per evaluation instead of 18, 7.9 ms a step instead of 25 (1,500 particles, 16,309 pairs,
+// 467 replayed).  The same operations per tangent component as in the other shapes: bitwise the
+// same results.
+template <int TG>
+__global__ void __launch_bounds__(32 * GRP_WARPS) k_bwd_contacts_coop(Consts C, State S, StepOut O, Adj A) {
+  constexpr int GL = 6;
+  __shared__ double shLin[GRP_WARPS][2 * NT];
+  __shared__ double shGs[GRP_WARPS][NT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool on = lane < GL * CO_LANES;   // lanes 30 and 31 idle
+  const unsigned mask = 0x3fffffffu;
+  TangentEval ev;
+  const int l = on ? lane / CO_LANES : 0;
+  ev.mask = mask; ev.g0 = l * CO_LANES; ev.r = lane - ev.g0;
+  const bool lead = on && ev.r == 0;
+  const int base = TG * l;
+  for (int i = blockIdx.x * GRP_WARPS + warp; i < C.P; i += gridDim.x * GRP_WARPS) {
+    const int c = A.order ? A.order[i] : i;
+    PairAdjIn q;
+    Geom<Dual<TG>> gd;
+    if (on) {
+      pairAdjIn(C, S, O, A, c, q);
+      if (lead)
+        for (int j = 0; j < TG; j++) {
+          const int k = base + j;
+          if (k < NT) { shLin[warp][k] = 0; shLin[warp][NT + k] = 0; }
+        }
+      __syncwarp(mask);
+      if (q.needed) {
+        if (lane == 0) SQA_CNT(&C.cnt[A_REPLAYED], 1);
+        NoBranch nb;
+        pairGeom<Dual<TG>>(q.p, gd, base, ev, nb);
+        if (lane == 0) checkReplay(C, O, c, q, gd);
+        if (q.pre && q.force) {
+          const V3<double> nv = mk<double>(gd.normal.x.v, gd.normal.y.v, gd.normal.z.v);
+          const V3<double> cpv = mk<double>(gd.cp.x.v, gd.cp.y.v, gd.cp.z.v);
+          for (int chunk = 0; chunk < 2; chunk++) {
+            LawIn<Dual<TG>> in;
+            lawInputs<Dual<TG>>(q.p, gd.depth.v, nv, cpv, chunk, in, base);
+            LawOut<Dual<TG>> out;
+            const bool ran = law(in, gd.isShearNew, C.dt, out);
+            if (lane == 0 && (chunk == 0 || !ran)) checkLaw(C, O, c, ran, out);
+            if (ran && lead)
+              for (int j = 0; j < TG; j++)
+                if (base + j < NT) shLin[warp][chunk * NT + base + j] = lawContract(q, out, j);
+          }
+        }
+      }
+    }
+    __syncwarp();
+    if (lead)
+      for (int j = 0; j < TG; j++)
+        if (base + j < NT) shGs[warp][base + j] = q.needed ? geomContract(q, gd, shLin[warp], j) : 0.0;
+    __syncwarp();
+    if (lane == 0) assemblePair(A, c, q, shLin[warp], shGs[warp]);
+    __syncwarp();
+  }
+}
+
 // Reverse step, (3) each body adds its pairs' contributions, in list order.
 SQA_HD void bwdGather(const Consts& C, const Adj& A, int b) {
   if (C.binfo[b].x == 1) return;
@@ -1383,14 +1520,14 @@ static void launchReplay(sqdem_adj* a, const Consts& C, const State& S, const St
     case 0: k_bwd_contacts<<<nblk(P, 64), 64, 0, a->st>>>(C, S, O, A); break;
     case 2: k_bwd_contacts_grp<9, 2><<<grid(GRP_WARPS * 16), bs, 0, a->st>>>(C, S, O, A); break;
     case 1: k_bwd_contacts_grp<6, 3><<<grid(GRP_WARPS * 10), bs, 0, a->st>>>(C, S, O, A); break;
-    default: k_bwd_contacts_grp<3, 6><<<grid(GRP_WARPS * 5), bs, 0, a->st>>>(C, S, O, A); break;
+    default: k_bwd_contacts_coop<3><<<grid(GRP_WARPS), bs, 0, a->st>>>(C, S, O, A); break;
   }
 }
 
 static void launchStep(sqdem_adj* a, const State& S, const StepOut& O, int step, bool branches = false) {
   const Consts C = consts(a, branches);
   if (a->coopForward)
-    k_fwd_contacts_coop<<<nblk(a->P, COOP_WARPS * 5), 32 * COOP_WARPS, 0, a->st>>>(C, S, O, step);
+    k_fwd_contacts_coop<<<nblk(a->P, COOP_WARPS), 32 * COOP_WARPS, 0, a->st>>>(C, S, O, step);
   else
     k_fwd_contacts<<<nblk(a->P, 128), 128, 0, a->st>>>(C, S, O, step);
   k_fwd_integrate<<<nblk(a->nb, 128), 128, 0, a->st>>>(C, S, O, step);
