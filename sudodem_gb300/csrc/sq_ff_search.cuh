@@ -247,6 +247,7 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_warp(Dev d, int tail, int round
   const int trial = grp < 15 ? grp / 3 : 0, role = grp < 15 ? grp % 3 : 0;   // group 15 mirrors group 0
   const int total = tail ? d.Q->nT[rounds] : d.S->lmCount + d.S->nmShort;
   int* head = tail ? &d.Q->tailHead : &d.S->lmHead;
+  if ((int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x >= total) return;
   unsigned long long ev = 0, deferred = 0;
   unsigned roundsMax = 0;
   for (;;) {

@@ -101,6 +101,8 @@ __device__ __forceinline__ void warpEval(const WShape& s, double e1B, int g0, in
 //   WS_TAIL      the searches left after `rounds` rounds of k_wave_trial / k_wave_probe, from there on
 enum { WS_LONG = 0, WS_DEFERRED = 1, WS_ALL = 2, WS_TAIL = 3 };
 
+// Blocks go to the SMs in turn, so that in blocks of one warp fewer searches than warps have an SM's
+// FP64 pipes to themselves (64 cycles an instruction, 76 with four busy schedulers).
 __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int waveRounds) {
   const unsigned FULL = 0xffffffffu;
   const SceneState& S = *d.S;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
                     : mode == WS_TAIL     ? d.Q->nT[waveRounds]
                                           : nLong + S.lmCount + S.nmShort;
   int* head = mode == WS_DEFERRED ? &d.S->fbHead : mode == WS_TAIL ? &d.Q->tailHead : &d.S->vlHead;
+  if ((int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) >= total) return;
   Counters cnt = {0, 0, 0, 0, 0};
   unsigned long long ev64 = 0;
   unsigned roundsMax = 0;

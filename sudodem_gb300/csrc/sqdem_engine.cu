@@ -135,6 +135,7 @@ struct QueueState {
   int vl2Count;   // long-search queue, from the back of fbQueue: fewer iterations than those at its front
   // FP64 rounds: entries of each round's lists, of the finish list, and the last list's head
   int nT[WAVE_MAX_ROUNDS + 1], nP[WAVE_MAX_ROUNDS + 1], nF, tailHead;
+  int integrated;   // blocks of k_integrate that are through
 };
 
 // Contact table, structure of arrays (one set per buffer).
@@ -157,6 +158,7 @@ struct Dev {
   // bodies
   double4 *pos, *ori, *vel, *angVel, *angMom, *inertia, *shpA, *shpB;   // shpA (rx,ry,rz,rmax) shpB (e1,e2,-,-)
   double* mass; int4* info;  // info: kind, mat, isSphere, wall axis | (sense+1)<<4
+  double* kin;               // staging of the kinematic state, 16 doubles per body
   unsigned* blocked; int* damped; int* aspherical;
   double4 *bmin, *bmax, *ref, *pmin, *pmax;    // bmin.w sweepLength, bmax.w lastUpdateIter, ref.w hasBound
   double4 *force, *torque;
@@ -2051,13 +2053,38 @@ __device__ __forceinline__ void addContribution(const Dev& d, int e, bool asId1,
   else { f = f + (-F); t = t + cross(pos - cp, F); }
 }
 
+// Start of NewtonIntegrator::action (NewtonIntegrator.cpp:107-117): pending velGrad, the
+// cell-size-change velocity that seeds maxVelocitySq, and the gradients the body update uses.
+__device__ void newtonBegin(const Dev& d) {
+  SceneState& S = *d.S;
+  if (!S.periodic) { S.cellTerm = 0; return; }
+  bool nz = false;
+  for (int k = 0; k < 9; k++) nz |= (S.nextVelGrad[k] != 0);
+  if (S.velGradChanged || nz) {
+    for (int k = 0; k < 9; k++) { S.velGrad[k] = S.nextVelGrad[k]; S.nextVelGrad[k] = 0; }
+    S.velGradChanged = 0;
+  }
+  const double dt = d.prm->dt;
+  for (int k = 0; k < 9; k++) { S.dVelGrad[k] = S.velGrad[k] - S.prevVelGrad[k]; S.dtPrevVelGrad[k] = dt * S.prevVelGrad[k]; }
+  const bool differs = S.prevCellSize[0] != S.cellSize[0] || S.prevCellSize[1] != S.cellSize[1] || S.prevCellSize[2] != S.cellSize[2];
+  if (differs && !isnan(S.prevCellSize[0])) {
+    const D3 dd = d3(S.prevCellSize[0] - S.cellSize[0], S.prevCellSize[1] - S.cellSize[1], S.prevCellSize[2] - S.cellSize[2]);
+    S.cellTerm = sqn(dd) / (dt * dt);
+  } else S.cellTerm = 0;
+}
+
 // ForceContainer sum for walls: one block per wall, fixed-order reduction; also the sum of
-// kn over the wall's real contacts (CompressionEngine::get_gain, Compression.cpp:1125-1220).
+// kn over the wall's real contacts (CompressionEngine::get_gain, Compression.cpp:1125-1220).  One
+// more block starts NewtonIntegrator's action (its state is read by nothing before k_integrate).
 __global__ void k_wall_forces(Dev d) {
   const SceneState& S = *d.S;
   if (S.skip) return;
   __shared__ double sh[7][128];
   const int w = blockIdx.x;
+  if (w == d.W) {
+    if (threadIdx.x == 0) newtonBegin(d);
+    return;
+  }
   const int wid = d.walls[w];
   const D3 pos = xyz(d.pos[wid]);
   const int s = d.wCount[d.W + w], n = d.wCount[w];
@@ -2096,6 +2123,31 @@ __device__ __forceinline__ void gatherBody(const Dev& d, int b, D3 pos, D3& f, D
     int e = d.pList[k];
     unsigned fl = d.A.flags[e];
     if (fl & F_FORCE) addContribution(d, e, (fl & F_OWNER_ID1) == 0, pos, f, m);
+  }
+}
+// The same sum, in the same order, for k_integrate: called by all lanes of a warp, b < 0 where there is
+// no body.  A body of a jammed cell has 28 entries, of which 4 carry a force: each lane first steps
+// to its next such entry, then all lanes add theirs together.  With one turn per entry some lane had a force in nearly every turn, and all paid for
+// its 35 FP64 instructions (the FP64 pipe was 83% busy; k_integrate at 200,000 bodies: 0.87 -> 0.40 ms).
+__device__ __forceinline__ void gatherWarp(const Dev& d, int b, D3 pos, D3& f, D3& m) {
+  f = d3(0, 0, 0); m = d3(0, 0, 0);
+  int e = 0, eEnd = 0, k = 0, kEnd = 0;
+  if (b >= 0) { e = d.rowStart[b]; eEnd = d.rowStart[b + 1]; k = d.pStart[b]; kEnd = d.pStart[b + 1]; }
+  for (;;) {
+    int hit = -1;
+    bool asId1 = false;
+    while (hit < 0 && e < eEnd) {
+      const unsigned fl = d.A.flags[e];
+      if (fl & F_FORCE) { hit = e; asId1 = (fl & F_OWNER_ID1) != 0; }
+      e++;
+    }
+    while (hit < 0 && k < kEnd) {
+      const int x = d.pList[k++];
+      const unsigned fl = d.A.flags[x];
+      if (fl & F_FORCE) { hit = x; asId1 = (fl & F_OWNER_ID1) == 0; }
+    }
+    if (!__any_sync(0xffffffffu, hit >= 0)) break;
+    if (hit >= 0) addContribution(d, hit, asId1, pos, f, m);
   }
 }
 
@@ -2398,33 +2450,38 @@ __device__ __forceinline__ void sphericalRotate(Q4& o, D3 w, double dt) {
   qnormalize(o);
 }
 
+// Scene::moveToNextTimeStep's epilogue (Scene.cpp:114-115), by the last block of k_integrate.
+__device__ void stepEnd(const Dev& d) {
+  SceneState& S = *d.S;
+  S.quiet = 0;       // NewtonIntegrator resets quiet_system_flag (:299)
+  if (S.periodic) {  // end of NewtonIntegrator::action (:300-302)
+    for (int k = 0; k < 3; k++) S.prevCellSize[k] = S.cellSize[k];
+    for (int k = 0; k < 9; k++) S.prevVelGrad[k] = S.velGrad[k];
+  }
+  S.iter++;
+  S.time += d.prm->dt;
+  S.err[E_STEPS]++;
+}
+
 __global__ void __launch_bounds__(256) k_integrate(Dev d) {
   const SceneState& S = *d.S;
   if (S.skip) return;
   const Params& P = *d.prm;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   int code = 0;
+  D3 pos = d3(0, 0, 0), f, m;
+  int4 inf = make_int4(KIND_WALL, 0, 0, 0);
+  if (b < d.N) { inf = d.info[b]; pos = xyz(d.pos[b]); }
+  gatherWarp(d, inf.x == KIND_SQ ? b : -1, pos, f, m);
   if (b < d.N) {
-    const int4 inf = d.info[b];
     const double dt = P.dt;
-    D3 pos = xyz(d.pos[b]);
     double4 o4 = d.ori[b];
     Q4 ori; ori.w = o4.x; ori.x = o4.y; ori.y = o4.z; ori.z = o4.w;
     D3 vel = xyz(d.vel[b]), angVel = xyz(d.angVel[b]), angMom = xyz(d.angMom[b]);
     const unsigned blocked = d.blocked[b];
     const bool damped = d.damped[b] != 0;
     const bool aspherical = d.aspherical[b] != 0;
-    D3 f = d3(0, 0, 0), m = d3(0, 0, 0);
     if (inf.x == KIND_SQ) {
-      for (int e = d.rowStart[b]; e < d.rowStart[b + 1]; e++) {
-        unsigned fl = d.A.flags[e];
-        if (fl & F_FORCE) addContribution(d, e, (fl & F_OWNER_ID1) != 0, pos, f, m);
-      }
-      for (int k = d.pStart[b]; k < d.pStart[b + 1]; k++) {
-        int e = d.pList[k];
-        unsigned fl = d.A.flags[e];
-        if (fl & F_FORCE) addContribution(d, e, (fl & F_OWNER_ID1) == 0, pos, f, m);
-      }
       d.force[b] = dd4(f, 0); d.torque[b] = dd4(m, 0);
     } else {
       f = xyz(d.force[b]); m = xyz(d.torque[b]);
@@ -2520,46 +2577,41 @@ __global__ void __launch_bounds__(256) k_integrate(Dev d) {
   for (int o = 16; o > 0; o >>= 1) code = max(code, __shfl_down_sync(0xffffffffu, code, o));
   if ((threadIdx.x & 31) == 0 && code) atomicMax(&d.S->maxDispCode, code);
   if (b == 0) d.S->newtonRan = 1;
-  (void)S;
+  // the block that is through last ends the step: every block has read the scene's state by then
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&d.Q->integrated, 1) == (int)gridDim.x - 1) {
+      d.Q->integrated = 0;
+      stepEnd(d);
+    }
+  }
+}
+
+// The kinematic state as the host exchanges it, 16 doubles per body (pos3 ori4 vel3 angVel3
+// angMom3), packed into or unpacked from d.kin: one contiguous copy instead of five strided ones
+// (200,000 bodies, to pinned memory: 0.48 -> 0.16 ms).
+__global__ void __launch_bounds__(256) k_kinematics(Dev d, int pack) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= d.N) return;
+  double4* k = (double4*)(d.kin + (size_t)b * 16);
+  if (pack) {
+    const double4 p = d.pos[b], o = d.ori[b], v = d.vel[b], w = d.angVel[b], m = d.angMom[b];
+    k[0] = make_double4(p.x, p.y, p.z, o.x); k[1] = make_double4(o.y, o.z, o.w, v.x);
+    k[2] = make_double4(v.y, v.z, w.x, w.y); k[3] = make_double4(w.z, m.x, m.y, m.z);
+  } else {
+    const double4 a = k[0], e = k[1], f = k[2], g = k[3];
+    d.pos[b] = make_double4(a.x, a.y, a.z, d.pos[b].w);
+    d.ori[b] = make_double4(a.w, e.x, e.y, e.z);
+    d.vel[b] = make_double4(e.w, f.x, f.y, d.vel[b].w);
+    d.angVel[b] = make_double4(f.z, f.w, g.x, d.angVel[b].w);
+    d.angMom[b] = make_double4(g.y, g.z, g.w, d.angMom[b].w);
+  }
 }
 
 __global__ void k_reset_queue(Dev d) {
   d.S->lmCount = 0; d.S->lmHead = 0; d.S->fbCount = 0; d.S->fbHead = 0; d.S->vlCount = 0; d.S->vlHead = 0;
   d.S->nmFin = 0; d.S->nmShort = 0; *d.Q = QueueState();
-}
-
-// Start of NewtonIntegrator::action (NewtonIntegrator.cpp:107-117): pending velGrad, the
-// cell-size-change velocity that seeds maxVelocitySq, and the gradients the body update uses.
-__global__ void k_newton_begin(Dev d) {
-  SceneState& S = *d.S;
-  if (S.skip) return;
-  if (!S.periodic) { S.cellTerm = 0; return; }
-  bool nz = false;
-  for (int k = 0; k < 9; k++) nz |= (S.nextVelGrad[k] != 0);
-  if (S.velGradChanged || nz) {
-    for (int k = 0; k < 9; k++) { S.velGrad[k] = S.nextVelGrad[k]; S.nextVelGrad[k] = 0; }
-    S.velGradChanged = 0;
-  }
-  const double dt = d.prm->dt;
-  for (int k = 0; k < 9; k++) { S.dVelGrad[k] = S.velGrad[k] - S.prevVelGrad[k]; S.dtPrevVelGrad[k] = dt * S.prevVelGrad[k]; }
-  const bool differs = S.prevCellSize[0] != S.cellSize[0] || S.prevCellSize[1] != S.cellSize[1] || S.prevCellSize[2] != S.cellSize[2];
-  if (differs && !isnan(S.prevCellSize[0])) {
-    const D3 dd = d3(S.prevCellSize[0] - S.cellSize[0], S.prevCellSize[1] - S.cellSize[1], S.prevCellSize[2] - S.cellSize[2]);
-    S.cellTerm = sqn(dd) / (dt * dt);
-  } else S.cellTerm = 0;
-}
-
-__global__ void k_end(Dev d) {
-  SceneState& S = *d.S;
-  if (S.skip) return;
-  S.quiet = 0;       // NewtonIntegrator resets quiet_system_flag (:299)
-  if (S.periodic) {  // end of NewtonIntegrator::action (:300-302)
-    for (int k = 0; k < 3; k++) S.prevCellSize[k] = S.cellSize[k];
-    for (int k = 0; k < 9; k++) S.prevVelGrad[k] = S.velGrad[k];
-  }
-  S.iter++;
-  S.time += d.prm->dt;
-  S.err[E_STEPS]++;
 }
 
 }  // namespace sqdem
@@ -2683,6 +2735,11 @@ static int waveRounds(const sqdem_ctx* c, const Dev& d) {
 // (2,197: 25.4 ms for ten steps, 26.5 with four rounds), then one more for each doubling (12,800:
 // 19.1 ms for five steps with four, 21.2 with none; 200,000: 38.3 for three with eight, 39.8 with four).
 static const int FF_WARP_MAX = 8000;
+// Particles up to which the mixed form's long FP64 searches are spread over the SMs, a warp per block:
+// there they bound the stage (12,800 particles: 18.3 ms for five steps, 19.0 in blocks of four warps).
+// Above it the double-float searches do, which want SMs of their own (70,000: 13.5 ms for two steps in
+// blocks of four warps, 15.1 spread; 200,000: the same).
+static const int LONG_SPREAD_MAX = 30000;
 static int ffRounds(const sqdem_ctx* c, const Dev& d) {
   const int n = std::max(c->load, d.NP);
   return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
@@ -2699,16 +2756,17 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
     k_contacts_nm_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
     c->launches += 3;
   } else {
-    // one block per SM for the warp searches: one warp per scheduler, whose FP64 pipe serves its
-    // chain alone
-    const int ws = std::min(c->numSMs, nblk(d.Pcap, LM_BS / 32));
+    // four warps per SM for the warp searches: one per scheduler, whose FP64 pipe serves its chain
+    // alone
+    const int ws = std::min(4 * c->numSMs, d.Pcap);
     if (c->precision == SQDEM_MIXED) {
       // the long searches in FP64 beside the double-float searches, then the searches the
       // double-float kernels deferred
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
       cudaEventRecord(c->fork, s);
       cudaStreamWaitEvent(c->stream2, c->fork, 0);
-      k_search_warp<<<ws, LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
+      const int lb = std::max(c->load, d.NP) > LONG_SPREAD_MAX ? LM_BS : 32;
+      k_search_warp<<<nblk(ws, lb / 32), lb, 0, c->stream2>>>(d, WS_LONG, 0);
       cudaEventRecord(c->join, c->stream2);
       k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
       const int blocks = c->numSMs * searchBlocksPerSM(c);
@@ -2727,20 +2785,20 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
       }
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
       k_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_DEFERRED, 0);
+      k_search_warp<<<ws, 32, 0, s>>>(d, WS_DEFERRED, 0);
       cudaStreamWaitEvent(s, c->join, 0);
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
       c->launches += 6 + 2 * rounds;
     } else if (std::max(c->load, d.NP) <= WARP_SEARCH_MAX) {
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
-      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_ALL, 0);
+      k_search_warp<<<ws, 32, 0, s>>>(d, WS_ALL, 0);
       if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
       c->launches += 2;
     } else {
       if (c->timingSearch) cudaEventRecord(c->ev[4], s);
       cudaEventRecord(c->fork, s);
       cudaStreamWaitEvent(c->stream2, c->fork, 0);
-      k_search_warp<<<ws, LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
+      k_search_warp<<<ws, 32, 0, c->stream2>>>(d, WS_LONG, 0);
       cudaEventRecord(c->join, c->stream2);
       const int wave = c->numSMs * searchBlocksPerSM(c);
       k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
@@ -2750,7 +2808,7 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
         k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
         k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
       }
-      k_search_warp<<<ws, LM_BS, 0, s>>>(d, WS_TAIL, rounds);
+      k_search_warp<<<ws, 32, 0, s>>>(d, WS_TAIL, rounds);
       k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
       cudaStreamWaitEvent(s, c->join, 0);
       if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
@@ -2759,19 +2817,17 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
   }
 }
 
-// One timestep of kernels on c->stream.
-static void enqueueStep(sqdem_ctx* c, bool timed) {
+// The collider pass on c->stream (every kernel tests runCollider).
+static void enqueueCollider(sqdem_ctx* c) {
   Dev& d = c->d;
   cudaStream_t s = c->stream;
   const int* gate = gateRun(c);
   const int N = d.N;
-  if (timed) cudaEventRecord(c->ev[0], s);
-  k_gate<<<1, 1, 0, s>>>(d);
   k_bounds<<<nblk(N, 256), 256, 0, s>>>(d);
   k_grid_setup<<<1, 1, 0, s>>>(d);
   k_zero_cells<<<std::min(nblk(d.Gmax + 1, 256), 4096), 256, 0, s>>>(d);
   k_cell_count<<<nblk(N, 256), 256, 0, s>>>(d);
-  c->launches += 5;
+  c->launches += 4;
   launchScan(c, d.cellCount, d.Gmax, d.cellStart, gate);
   k_cell_scatter<<<nblk(N, 256), 256, 0, s>>>(d);
   k_candidates<<<nblk(N, 128), 128, 0, s>>>(d);
@@ -2793,22 +2849,34 @@ static void enqueueStep(sqdem_ctx* c, bool timed) {
     k_wall_lists<<<d.wallChunks, 256, 0, s>>>(d);
     c->launches += 2;
   }
+}
+
+// One timestep of kernels on c->stream.
+static void enqueueStep(sqdem_ctx* c, bool timed) {
+  Dev& d = c->d;
+  cudaStream_t s = c->stream;
+  const int N = d.N;
+  if (timed) cudaEventRecord(c->ev[0], s);
+  k_gate<<<1, 1, 0, s>>>(d);
+  c->launches++;
+  // the collider pass; its kernels return at once when k_gate decided it does not run (a conditional
+  // graph node around them was measured to cost as much as they do: 0.083 against 0.085 ms a step)
+  enqueueCollider(c);
   if (timed) cudaEventRecord(c->ev[1], s);
   // LM grid: all resident blocks, fewer for a small table (at most one lane per 4 entries)
   const int lmFull = c->numSMs * searchBlocksPerSM(c);
   launchContactStage(c, d, std::max(1, std::min(lmFull, nblk(d.Pcap, LM_BS * 4))));
   if (timed) cudaEventRecord(c->ev[2], s);
-  if (d.W > 0) { k_wall_forces<<<d.W, 128, 0, s>>>(d); c->launches++; }
+  k_wall_forces<<<d.W + 1, 128, 0, s>>>(d);
+  c->launches++;
   if (c->servoOn) {   // CompressionEngine between InteractionLoop and NewtonIntegrator
     k_servo_gate<<<1, 1, 0, s>>>(d);
     k_servo_sums<<<d.svBlocks, 128, 0, s>>>(d, -1, 1);
     k_servo<<<1, 1, 0, s>>>(d);
     c->launches += 3;
   }
-  k_newton_begin<<<1, 1, 0, s>>>(d);
   k_integrate<<<nblk(N, 256), 256, 0, s>>>(d);
-  k_end<<<1, 1, 0, s>>>(d);
-  c->launches += 3;
+  c->launches++;
   if (timed) cudaEventRecord(c->ev[3], s);
 }
 
@@ -3053,7 +3121,7 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* c, int n, const int* kind, const double
   CK(dalloc(c, &d.prm, 1)); CK(dalloc(c, &d.S, 1)); CK(dalloc(c, &d.Q, 1));
   CK(dalloc(c, &d.pos, n)); CK(dalloc(c, &d.ori, n)); CK(dalloc(c, &d.vel, n)); CK(dalloc(c, &d.angVel, n));
   CK(dalloc(c, &d.angMom, n)); CK(dalloc(c, &d.inertia, n)); CK(dalloc(c, &d.shpA, n)); CK(dalloc(c, &d.shpB, n));
-  CK(dalloc(c, &d.mass, n)); CK(dalloc(c, &d.info, n)); CK(dalloc(c, &d.blocked, n)); CK(dalloc(c, &d.damped, n));
+  CK(dalloc(c, &d.kin, 16 * (size_t)n)); CK(dalloc(c, &d.mass, n)); CK(dalloc(c, &d.info, n)); CK(dalloc(c, &d.blocked, n)); CK(dalloc(c, &d.damped, n));
   CK(dalloc(c, &d.aspherical, n));
   CK(dalloc(c, &d.bmin, n)); CK(dalloc(c, &d.bmax, n)); CK(dalloc(c, &d.ref, n)); CK(dalloc(c, &d.pmin, n));
   CK(dalloc(c, &d.pmax, n)); CK(dalloc(c, &d.force, n)); CK(dalloc(c, &d.torque, n));
@@ -3250,17 +3318,22 @@ sqdem_status sqdem_put_body_state(sqdem_ctx* c, const double* in) {
   return SQDEM_OK;
 }
 
+// the kinematic state to and from 16 doubles per body of host memory, on the context's stream
+static cudaError_t kinToHost(sqdem_ctx* c, double* out16) {
+  k_kinematics<<<nblk(c->d.N, 256), 256, 0, c->stream>>>(c->d, 1);
+  return cudaMemcpyAsync(out16, c->d.kin, sizeof(double) * 16 * (size_t)c->d.N, cudaMemcpyDeviceToHost, c->stream);
+}
+static cudaError_t kinToDevice(sqdem_ctx* c, const double* in16) {
+  const cudaError_t e = cudaMemcpyAsync(c->d.kin, in16, sizeof(double) * 16 * (size_t)c->d.N, cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) k_kinematics<<<nblk(c->d.N, 256), 256, 0, c->stream>>>(c->d, 0);
+  return e;
+}
+
 sqdem_status sqdem_get_kinematics(sqdem_ctx* c, double* out16) {
   if (!c || !out16) return SQDEM_ERR_ARG;
   if (!c->haveBodies) return fail(c, SQDEM_ERR_STATE, "no bodies");
   CK(cudaSetDevice(c->device));
-  const int n = c->d.N;
-  // five double4 planes -> 16 doubles per body, copied straight from device memory
-  CK(cudaMemcpy2DAsync(out16 + 0, 16 * 8, c->d.pos, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpy2DAsync(out16 + 3, 16 * 8, c->d.ori, 32, 32, n, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpy2DAsync(out16 + 7, 16 * 8, c->d.vel, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpy2DAsync(out16 + 10, 16 * 8, c->d.angVel, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpy2DAsync(out16 + 13, 16 * 8, c->d.angMom, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
+  CK(kinToHost(c, out16));
   CK(cudaStreamSynchronize(c->stream));
   return SQDEM_OK;
 }
@@ -3269,12 +3342,7 @@ sqdem_status sqdem_put_kinematics(sqdem_ctx* c, const double* in16) {
   if (!c->haveBodies) return fail(c, SQDEM_ERR_STATE, "no bodies");
   if (!finiteRows(in16, c->d.N, 16, 16)) return fail(c, SQDEM_ERR_ARG, "non-finite kinematic state");
   CK(cudaSetDevice(c->device));
-  const int n = c->d.N;
-  CK(cudaMemcpy2DAsync(c->d.pos, 32, in16 + 0, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpy2DAsync(c->d.ori, 32, in16 + 3, 16 * 8, 32, n, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpy2DAsync(c->d.vel, 32, in16 + 7, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpy2DAsync(c->d.angVel, 32, in16 + 10, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpy2DAsync(c->d.angMom, 32, in16 + 13, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
+  CK(kinToDevice(c, in16));
   return SQDEM_OK;
 }
 
@@ -3517,24 +3585,15 @@ sqdem_status sqdem_time_e2e(sqdem_ctx* c, int nsteps, const double* in16, double
   if (!c->haveBodies) return fail(c, SQDEM_ERR_STATE, "no bodies");
   CK(cudaSetDevice(c->device));
   if (c->useGraph) { sqdem_status s = ensureGraph(c); if (s) return s; }
-  const int n = c->d.N;
   CK(cudaEventRecord(c->ev[0], c->stream));
   double* bufs[2] = {const_cast<double*>(in16), out16};
   for (int i = 0; i < nsteps; i++) {
     const double* src = bufs[i & 1];
     double* dst = bufs[(i + 1) & 1];
-    CK(cudaMemcpy2DAsync(c->d.pos, 32, src + 0, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpy2DAsync(c->d.ori, 32, src + 3, 16 * 8, 32, n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpy2DAsync(c->d.vel, 32, src + 7, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpy2DAsync(c->d.angVel, 32, src + 10, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpy2DAsync(c->d.angMom, 32, src + 13, 16 * 8, 24, n, cudaMemcpyHostToDevice, c->stream));
+    CK(kinToDevice(c, src));
     if (c->useGraph) { CK(cudaGraphLaunch(c->exec, c->stream)); c->launches += c->launchesPerStep; }
     else enqueueStep(c, false);
-    CK(cudaMemcpy2DAsync(dst + 0, 16 * 8, c->d.pos, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpy2DAsync(dst + 3, 16 * 8, c->d.ori, 32, 32, n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpy2DAsync(dst + 7, 16 * 8, c->d.vel, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpy2DAsync(dst + 10, 16 * 8, c->d.angVel, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpy2DAsync(dst + 13, 16 * 8, c->d.angMom, 32, 24, n, cudaMemcpyDeviceToHost, c->stream));
+    CK(kinToHost(c, dst));
   }
   CK(cudaEventRecord(c->ev[3], c->stream));
   CK(cudaEventSynchronize(c->ev[3]));
