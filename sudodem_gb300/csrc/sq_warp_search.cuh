@@ -94,38 +94,60 @@ __device__ __forceinline__ void warpEval(const WShape& s, double e1B, int g0, in
   o.nrm = sqrt((k ? n1o : n1) + ((k ? n1 : n1o) + n2));
 }
 
-// Work lists: which entries a launch takes, in this order.
-//   WS_LONG      the long-search queue (fbQueue): 64+ iterations at the last step, then 32-63
-//   WS_DEFERRED  the searches the mixed form's double-float kernels deferred (deferQueue)
-//   WS_ALL       the long-search queue, then the main queue (lmQueue), longest first
-//   WS_TAIL      the searches left after `rounds` rounds of k_wave_trial / k_wave_probe, from there on
-enum { WS_LONG = 0, WS_DEFERRED = 1, WS_ALL = 2, WS_TAIL = 3 };
+// A point of a round, as all lanes of a search read it: its evaluation, and for a trial point the
+// step it came from and what follows if it is accepted.
+struct WSlot {
+  double f[3], nrm, sep, c[3], a[3], b[3];   // p2 - p1, |f|, c . f, direction, support points
+  double D0, D1, t0, t1, mu;
+  unsigned bits;
+};
+enum { WB_APART = 1, WB_FINITE = 2, WB_GAIN = 4, WB_SMALL = 8, WB_HUGE = 16 };
 
-// Blocks go to the SMs in turn, so that in blocks of one warp fewer searches than warps have an SM's
-// FP64 pipes to themselves (64 cycles an instruction, 76 with four busy schedulers).
-__global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int waveRounds) {
+// Work lists: which entries a launch takes, in this order.
+//   WS_LONG      the long-search queue (fbQueue), its front first
+//   WS_DEFERRED  the searches the mixed form's double-float kernels deferred (deferQueue)
+//   WS_MAIN      the main queue (lmQueue), longest first
+//   WS_TAIL      the searches left after `rounds` rounds of k_wave_trial / k_wave_probe, from there on
+enum { WS_LONG = 0, WS_DEFERRED = 1, WS_MAIN = 2, WS_TAIL = 3 };
+
+// W warps per search.  W = 1: blocks go to the SMs in turn, so that in blocks of one warp fewer
+// searches than warps have an SM's FP64 pipes to themselves (64 cycles an instruction, 76 with four
+// busy schedulers).  W = 2: a block of two warps, twelve points a round, four trials with their
+// probes each: 1.07 rounds an iteration instead of 1.33 for twice the FP64 work, where few searches
+// bound the stage and the pipes are otherwise idle (12,800 particles, mixed form: 18.3 -> 15.1 ms for
+// five steps; 1,583 in FP64: 3.46 -> 2.82 ms a step; 20,000 polydisperse: 11.1 -> 9.6 for three).
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_warp(Dev d, int mode, int waveRounds) {
   const unsigned FULL = 0xffffffffu;
   const SceneState& S = *d.S;
-  const int lane = threadIdx.x & 31;
-  const int grp = lane < WS_LANES * WS_POINTS ? lane / WS_LANES : 0;
-  const int g0 = grp * WS_LANES;
-  const int r = lane < WS_LANES * WS_POINTS ? lane - g0 : lane - WS_LANES * WS_POINTS;   // lanes 30, 31 mirror 0, 1
+  __shared__ WSlot slots[W == 1 ? LM_BS / 32 : 1][2][WS_POINTS * W];
+  __shared__ int taken[W == 1 ? LM_BS / 32 : 1];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int own = W == 1 ? wib : 0;                 // the search's place in the block
+  const bool real = lane < WS_LANES * WS_POINTS;    // lanes 30, 31: the step of trial 0, no point of their own
+  const int g0 = real ? lane / WS_LANES * WS_LANES : 0;
+  const int r = real ? lane - g0 : lane - WS_LANES * WS_POINTS;
+  const int grp = (W == 1 ? 0 : wib * WS_POINTS) + g0 / WS_LANES;
+  const int gs = real ? g0 : 30;                    // where the lane's step is computed
   const bool odd = r == 1 || r == 3;
-  const int nLong1 = S.vlCount, nLong = mode == WS_DEFERRED ? 0 : S.vlCount + d.Q->vl2Count;
+  const int nLong1 = S.vlCount, nLong = S.vlCount + d.Q->vl2Count;
   const int nFront = S.lmCount;
   const int total = mode == WS_LONG       ? nLong
                     : mode == WS_DEFERRED ? S.fbCount
                     : mode == WS_TAIL     ? d.Q->nT[waveRounds]
-                                          : nLong + S.lmCount + S.nmShort;
-  int* head = mode == WS_DEFERRED ? &d.S->fbHead : mode == WS_TAIL ? &d.Q->tailHead : &d.S->vlHead;
-  if ((int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) >= total) return;
+                                          : S.lmCount + S.nmShort;
+  int* head = mode == WS_LONG ? &d.S->vlHead : mode == WS_DEFERRED ? &d.S->fbHead : mode == WS_TAIL ? &d.Q->tailHead : &d.S->lmHead;
+  if ((int)(W == 1 ? blockIdx.x * (blockDim.x >> 5) + wib : blockIdx.x) >= total) return;
   Counters cnt = {0, 0, 0, 0, 0};
   unsigned long long ev64 = 0;
   unsigned roundsMax = 0;
+  int flip = 0;
+  auto join = [&]() { if (W == 1) __syncwarp(); else __syncthreads(); };
   for (;;) {
-    int idx = 0;
-    if (lane == 0) idx = atomicAdd(head, 1);
-    idx = __shfl_sync(FULL, idx, 0);
+    if (lane == 0 && (W == 1 || wib == 0)) taken[own] = atomicAdd(head, 1);
+    join();
+    const int idx = taken[own];
+    join();
     if (idx >= total) break;
     int e;
     WaveState w;
@@ -135,8 +157,8 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
       e = w.e;
       resume = !w.init;
     } else if (mode == WS_DEFERRED) e = d.deferQueue[idx];
-    else if (idx < nLong) e = idx < nLong1 ? d.fbQueue[idx] : d.fbQueue[d.Pcap - 1 - (idx - nLong1)];
-    else { const int j = idx - nLong; e = j < nFront ? d.lmQueue[j] : d.lmQueue[d.qCap - 1 - (j - nFront)]; }
+    else if (mode == WS_LONG) e = idx < nLong1 ? d.fbQueue[idx] : d.fbQueue[d.Pcap - 1 - (idx - nLong1)];
+    else e = idx < nFront ? d.lmQueue[idx] : d.lmQueue[d.qCap - 1 - (idx - nFront)];
     // start of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom::go up to lmder2
     const unsigned fl = d.A.flags[e];
     int id1, id2;
@@ -171,34 +193,64 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
     unsigned calls = 0, iters = 0, maxit = 0, rounds = 0;
     bool touching = true;
     if (mode == WS_TAIL) { contact = w.contact; phase = (int)w.phase; calls = w.calls; iters = w.iters; maxit = w.maxit; }
+    WSlot* q = slots[own][flip];   // the last round's points
+    // evaluates the lane's group's point into the round's slots; the other trial fields are the caller's
+    auto round = [&](double q0, double q1, bool trial, double D0, double D1, double t0, double t1, double myMu, double pfL2,
+                     double jt0, double jt1, unsigned bits) {
+      WEval v;
+      warpEval(s, e1B, g0, r, q0, q1, v);
+      double muNext = 0;
+      if (v.sep > 0) bits |= WB_APART;
+      if (isfinite(v.nrm)) bits |= WB_FINITE;
+      if (trial) {   // gain ratio and damping update
+        const double dm = (odd ? D1 : D0) * (myMu * (odd ? D1 : D0) + (odd ? jt1 : jt0));
+        const double dmo = __shfl_sync(FULL, dm, r == 4 ? g0 + 1 : gs + (r ^ 1));
+        const double dL = dm + dmo, dF = pfL2 - v.nrm;
+        double tmp = dF / dL;
+        if (tmp > 0.0) bits |= WB_GAIN;
+        tmp = 1.0 - cube(2 * tmp - 1.);
+        muNext = myMu * ((tmp >= 0.3333333333333334) ? tmp : 0.3333333333333334);
+      }
+      flip ^= 1;
+      q = slots[own][flip];
+      if (real) {
+        WSlot& o = q[grp];
+        const int k = odd ? 1 : 0;
+        if (r < 2) { o.f[k] = v.fxy; o.a[k] = v.pxy; }
+        else if (r < 4) o.b[k] = v.pxy;
+        if (r == 0) { o.f[2] = v.fz; o.a[2] = v.pz; o.nrm = v.nrm; o.sep = v.sep; }
+        if (r == 1) { o.c[0] = v.c.x; o.c[1] = v.c.y; o.c[2] = v.c.z; }
+        if (r == 2) o.b[2] = v.pz;
+        if (r == 3) { o.D0 = D0; o.D1 = D1; o.t0 = t0; o.t1 = t1; }
+        if (r == 4) { o.mu = muNext; o.bits = bits; }
+      }
+      join();
+      rounds++;
+    };
     for (;;) {   // one lmder2 call
       touching = true;
       bool stopFlag = false;
       int stop, k = 0, nu = 2;
       double mu = 0, Dp0 = 1e-7, Dp1 = 1e-7, pfL2;
       D3 pf;
-      WEval v = {};
       double diag0 = 0, diag1 = 0, j01 = 0, jt0 = 0, jt1 = 0;
-      unsigned sepPos = 0;   // bit of a group's first lane: its stop predicate
       int last = 0, base = 0;       // the group whose evaluation was consumed last; the accepted point's group
       int probe0 = 1, probe1 = 2;   // the groups of the accepted point's probes
       double muRej = 0;             // damping below which trials were last rejected
       bool more;
       // the accepted point of group `base`, then the top of lmder2's loop (lmOuter)
       auto outer = [&]() {
+        const WSlot& o = q[base];
+        pf = d3(o.f[0], o.f[1], o.f[2]);
+        pfL2 = o.nrm;
         if (!(k < 50 && !stop)) { if (k >= 50) stop = 3; return false; }
         if (pfL2 <= 1e-20) { stop = 6; return false; }
         if (stopFlag) { stop = 9; touching = false; return false; }
-        const int l = base * WS_LANES;
-        contact = d3(__shfl_sync(FULL, v.c.x, l), __shfl_sync(FULL, v.c.y, l), __shfl_sync(FULL, v.c.z, l));
-        if (angleTest(__shfl_sync(FULL, v.sep, l), pfL2, contact)) { stop = 8; return false; }
+        contact = d3(o.c[0], o.c[1], o.c[2]);
+        if (angleTest(o.sep, pfL2, contact)) { stop = 8; return false; }
         return true;
       };
-      auto accept = [&]() {
-        const int l = base * WS_LANES;
-        pf = d3(__shfl_sync(FULL, v.fxy, l), __shfl_sync(FULL, v.fxy, l + 1), __shfl_sync(FULL, v.fz, l));
-        pfL2 = __shfl_sync(FULL, v.nrm, l);
-      };
+      auto end = [&](int code) { stop = code; k++; if (k >= 50) stop = 3; };
       if (resume) {
         stopFlag = w.stopFlag; stop = 0; k = w.k; nu = w.nu; mu = w.mu;
         pf = w.pf; pfL2 = w.pfL2;
@@ -206,25 +258,20 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
         more = true;
       } else {
         // the start point and its two probes
-        warpEval(s, e1B, g0, r, grp == 1 ? p0 + Dp0 : p0, grp == 2 ? p1 + Dp1 : p1, v);
-        rounds++;
+        round(grp == 1 ? p0 + Dp0 : p0, grp == 2 ? p1 + Dp1 : p1, false, 0, 0, 0, 0, 0, 0, 0, 0, 0u);
         ev64 += 3;
-        sepPos = __ballot_sync(FULL, v.sep > 0);
-        accept();
-        if (sepPos & 1u) stopFlag = true;
-        stop = isfinite(pfL2) ? 0 : 7;
+        if (q[0].bits & WB_APART) stopFlag = true;
+        stop = isfinite(q[0].nrm) ? 0 : 7;
         more = outer();
       }
       while (more) {
         if (!resume) {
           // the two probes at the accepted point: Jacobian and normal equations
           last = probe1;
-          if (((sepPos >> (probe0 * WS_LANES)) | (sepPos >> (probe1 * WS_LANES))) & 1u) stopFlag = true;
+          if ((q[probe0].bits | q[probe1].bits) & WB_APART) stopFlag = true;
           const int pc = lane % 3, pj = (lane / 3) & 1;   // lanes 0-5: component pc of column pj
-          const int src = (pj ? probe1 : probe0) * WS_LANES;
-          const double fx = __shfl_sync(FULL, v.fxy, pc == 1 ? src + 1 : src), fz = __shfl_sync(FULL, v.fz, src);
           const double f0c = pc == 0 ? pf.x : pc == 1 ? pf.y : pf.z;
-          const double J = ((pc == 2 ? fz : fx) - f0c) / (pj ? Dp1 : Dp0);
+          const double J = (q[pj ? probe1 : probe0].f[pc] - f0c) / (pj ? Dp1 : Dp0);
           // lane 3 m + pc: product m of component pc: J0 J0, J0 J1, J1 J1, J0 (-f0), J1 (-f0)
           const int pm = lane / 3;
           const double Ja = __shfl_sync(FULL, J, ((pm == 2 || pm == 4) ? 3 : 0) + pc);
@@ -237,102 +284,85 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
           diag0 = __shfl_sync(FULL, sum, 0); j01 = __shfl_sync(FULL, sum, 1); diag1 = __shfl_sync(FULL, sum, 2);
           jt0 = __shfl_sync(FULL, sum, 3); jt1 = __shfl_sync(FULL, sum, 4);
           const double jinf = (fabs(jt0) > fabs(jt1) ? fabs(jt0) : fabs(jt1));
-          more = false;
           if (jinf <= 1e-15) { stop = 1; break; }
           if (k == 0) mu = 1.0 * (diag0 > diag1 ? diag0 : diag1);
         }
         more = false;
         resume = false;
         for (;;) {   // damping loop: the step for mu, and those that follow its rejections
-          // A slow search divides mu by three at every accepted trial, until trials are rejected
-          // (two to five in a row, mu times 2, 4, 8 ...) and mu is above the level again below which
-          // it was rejected last, muRej, which moves little: so the trials up to the first above
-          // that level take a group each, and that one's probes two more.  plan: the trial whose
-          // probes are evaluated with it (0: those of trials 0 and 1; 4: none).
-          // group's trial and role (0: the trial point, 1 and 2: its probes)
+          // Twelve points: four trials with their probes.  Six: a slow search divides mu by three at
+          // every accepted trial, until trials are rejected (two to five in a row, mu times 2, 4, 8
+          // ...) and mu is above the level again below which it was rejected last, muRej, which moves
+          // little: so the trials up to the first above that level take a group each, and that
+          // one's probes two more.  plan: the trial whose probes are evaluated with it (0: those of
+          // every trial; 4: none).
           int rej = 0;
-          for (double m = mu; rej < 4 && m <= muRej; rej++) m *= (double)(2 << rej) * 0.5 * nu;
+          if (W == 1) for (double m = mu; rej < 4 && m <= muRej; rej++) m *= (double)(2 << rej) * 0.5 * nu;
           const int plan = rej < 2 ? 0 : rej;
-          const int trial = plan == 0 ? grp / 3 : plan == 2 ? (grp < 2 ? grp : grp < 5 ? 2 : 3) : plan == 3 ? min(grp, 3) : grp;
+          const int trial = !real ? 0 : plan == 0 ? grp / 3 : plan == 2 ? (grp < 2 ? grp : grp < 5 ? 2 : 3) : plan == 3 ? min(grp, 3) : grp;
           const int role = plan == 0 ? grp % 3 : plan == 4 ? 0 : max(0, min(2, grp - plan)) * (grp < plan + 3 ? 1 : 0);
-          const int trials = plan == 0 ? 2 : plan == 4 ? WS_POINTS : 4;
+          const int trials = plan == 0 ? 2 * W : plan == 4 ? WS_POINTS : 4;
           double myMu = mu;
           for (int j = 0, m = nu; j < trial; j++, m = (int)((unsigned)m << 1)) myMu *= m;
           const double bo = (odd ? diag0 : diag1) + myMu, bx = (odd ? diag1 : diag0) + myMu;   // even lanes: Dp0, odd lanes: Dp1
           const double n_a = bo * bx - j01 * j01;
           const double D = ((odd ? jt1 : jt0) * bo - (odd ? jt0 : jt1) * j01) / n_a;
-          const double D0 = __shfl_sync(FULL, D, g0), D1 = __shfl_sync(FULL, D, g0 + 1);
+          const double D0 = __shfl_sync(FULL, D, gs), D1 = __shfl_sync(FULL, D, gs + 1);
           const double DL2 = sqrt(D0 * D0 + D1 * D1);
           const bool small = DL2 < 1e-5;
           // stop 4 compares with (|p| + 1e-3) / 1e-24, which is above 1e20
           bool huge = false;
           if (!(DL2 < 1e20)) huge = DL2 >= (sqrt(p0 * p0 + p1 * p1) + 1e-3) / (1e-12 * 1e-12);
           const unsigned smallB = __ballot_sync(FULL, small), hugeB = __ballot_sync(FULL, huge);
-          if (smallB & 1u) { stop = 2; k++; if (k >= 50) stop = 3; break; }
-          if (hugeB & 1u) { stop = 4; k++; if (k >= 50) stop = 3; break; }
+          if (smallB >> 30) { end(2); break; }   // lanes 30, 31: trial 0
+          if (hugeB >> 30) { end(4); break; }
           const double t0 = p0 + D0, t1 = p1 + D1;
-          warpEval(s, e1B, g0, r, role == 1 ? t0 + D0 : t0, role == 2 ? t1 + D1 : t1, v);
-          rounds++;
-          ev64 += WS_POINTS;
-          // gain ratio and damping update of each group's trial
-          const double dm = (odd ? D1 : D0) * (myMu * (odd ? D1 : D0) + (odd ? jt1 : jt0));
-          const double dmo = __shfl_sync(FULL, dm, r == 4 ? g0 + 1 : g0 + (r ^ 1));
-          const double dL = dm + dmo;
-          const double dF = pfL2 - v.nrm;
-          double tmp = dF / dL;
-          const unsigned gain = __ballot_sync(FULL, tmp > 0.0);
-          tmp = 1.0 - cube(2 * tmp - 1.);
-          const double muNext = myMu * ((tmp >= 0.3333333333333334) ? tmp : 0.3333333333333334);
-          const unsigned fin = __ballot_sync(FULL, isfinite(v.nrm));
-          sepPos = __ballot_sync(FULL, v.sep > 0);
-          bool ended = false, taken = false;
+          round(role == 1 ? t0 + D0 : t0, role == 2 ? t1 + D1 : t1, true, D0, D1, t0, t1, myMu, pfL2, jt0, jt1,
+                (small ? WB_SMALL : 0u) | (huge ? WB_HUGE : 0u));
+          ev64 += WS_POINTS * W;
+          bool ended = false, accepted = false;
           for (int a = 0; a < trials; a++) {
-            const int g = plan == 0 ? 3 * a : plan == 2 && a == 3 ? 5 : a, l = g * WS_LANES;
-            if (a > 0) {   // the step after the last rejection ends the call
-              const bool sm = (smallB >> l) & 1u, hu = (hugeB >> l) & 1u;
-              if (sm || hu) { stop = sm ? 2 : 4; k++; if (k >= 50) stop = 3; ended = true; break; }
+            const int g = plan == 0 ? 3 * a : plan == 2 && a == 3 ? 5 : a;
+            const WSlot& o = q[g];
+            if (a > 0 && (o.bits & (WB_SMALL | WB_HUGE))) {   // the step after the last rejection ends the call
+              end((o.bits & WB_SMALL) ? 2 : 4);
+              ended = true;
+              break;
             }
             last = g;
-            if ((sepPos >> l) & 1u) stopFlag = true;
-            if (!((fin >> l) & 1u)) { stop = 7; k++; if (k >= 50) stop = 3; ended = true; break; }
-            if ((gain >> l) & 1u) {
+            if (o.bits & WB_APART) stopFlag = true;
+            if (!(o.bits & WB_FINITE)) { end(7); ended = true; break; }
+            if (o.bits & WB_GAIN) {
               base = g;
-              const double myAcc = mu;
-              mu = __shfl_sync(FULL, muNext, l);
+              if (mu <= muRej) muRej = 0.5 * mu;
+              mu = o.mu;
               nu = 2;
-              Dp0 = __shfl_sync(FULL, D0, l); Dp1 = __shfl_sync(FULL, D1, l);
-              p0 = __shfl_sync(FULL, t0, l); p1 = __shfl_sync(FULL, t1, l);
-              accept();
+              Dp0 = o.D0; Dp1 = o.D1;
+              p0 = o.t0; p1 = o.t1;
               k++;
               more = outer();
-              taken = true;
+              accepted = true;
               // the probes at the accepted trial: in this round's groups, or a round of their own
               const bool have = plan == 0 || a == plan;
               probe0 = have ? g + 1 : 0; probe1 = have ? g + 2 : 1;
               if (more && !have) {
-                warpEval(s, e1B, g0, r, grp == 0 ? p0 + Dp0 : p0, grp == 1 ? p1 + Dp1 : p1, v);
-                rounds++;
+                round(grp == 0 ? p0 + Dp0 : p0, grp == 1 ? p1 + Dp1 : p1, false, 0, 0, 0, 0, 0, 0, 0, 0, 0u);
                 ev64 += 2;
-                sepPos = __ballot_sync(FULL, v.sep > 0);
               }
-              if (myAcc <= muRej) muRej = 0.5 * myAcc;
               break;
             }
             muRej = mu;
             mu *= nu;
             const int nn = (int)((unsigned)nu << 1);
-            if (nn <= nu) { stop = 5; k++; if (k >= 50) stop = 3; ended = true; break; }
+            if (nn <= nu) { end(5); ended = true; break; }
             nu = nn;
           }
-          if (ended || taken) break;
+          if (ended || accepted) break;
         }
       }
-      {
-        const int l = last * WS_LANES;
-        P1 = d3(__shfl_sync(FULL, v.pxy, l), __shfl_sync(FULL, v.pxy, l + 1), __shfl_sync(FULL, v.pz, l));
-        P2 = d3(__shfl_sync(FULL, v.pxy, l + 2), __shfl_sync(FULL, v.pxy, l + 3), __shfl_sync(FULL, v.pz, l + 2));
-      }
-      // the restart rules of Superquadrics_Ig2.cpp:2013-2053 (as lmCallEnd)
+      P1 = d3(q[last].a[0], q[last].a[1], q[last].a[2]);
+      P2 = d3(q[last].b[0], q[last].b[1], q[last].b[2]);
+      // the restart rules of Superquadrics_Ig2.cpp:2013-2053
       bool again = false;
       for (;;) {
         calls++; iters += k; maxit += (stop == 3);
@@ -347,12 +377,12 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
             const double rmaxA = __shfl_sync(FULL, s.rmax, 0);
             if (touching && 10.0 * nrm(P2 - P1) > rmaxA) {
               // isInside (Superquadrics.cpp:103-108) of the other body's point, each body on its lanes
-              SqShape q;
-              q.rx = s.rx; q.ry = s.ry; q.rz = s.rz; q.e1 = s.e1; q.e2 = s.e2;
-              for (int i = 0; i < 9; i++) q.R.m[i] = s.R[i];
+              SqShape b;
+              b.rx = s.rx; b.ry = s.ry; b.rz = s.rz; b.e1 = s.e1; b.e2 = s.e2;
+              for (int i = 0; i < 9; i++) b.R.m[i] = s.R[i];
               const D3 rel = (bodyB ? P1 : P2) - s.pos;
-              const int fast = insideFast(q, rel);
-              const bool mine = __any_sync(FULL, fast < 0) ? isInside(q, rel) : fast == 1;
+              const int fast = insideFast(b, rel);
+              const bool mine = __any_sync(FULL, fast < 0) ? isInside(b, rel) : fast == 1;
               const unsigned in = __ballot_sync(FULL, mine);
               if (!(in & 1u) || !(in & 4u)) { phase = 2; restart = true; }
             }
@@ -365,12 +395,12 @@ __global__ void __launch_bounds__(LM_BS, 3) k_search_warp(Dev d, int mode, int w
       }
       if (!again) break;
     }
-    if (lane == 0)
+    if (threadIdx.x == (W == 1 ? threadIdx.x & ~31 : 0))
       finishSearch(d, e, fl, id1, id2, isNew, p0, p1, touching, P1, P2, contact, calls, iters, maxit, cnt);
     roundsMax = max(roundsMax, rounds);
   }
   flushCounters(d, cnt);
-  if (lane == 0 && roundsMax) {
+  if (lane == 0 && (W == 1 || wib == 0) && roundsMax) {
     atomicAdd(&d.S->err[E_EVAL64], ev64);
     atomicMax(&d.S->err[E_ROUNDS_MAX], (unsigned long long)roundsMax);
   }

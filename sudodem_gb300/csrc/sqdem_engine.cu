@@ -2735,11 +2735,10 @@ static int waveRounds(const sqdem_ctx* c, const Dev& d) {
 // (2,197: 25.4 ms for ten steps, 26.5 with four rounds), then one more for each doubling (12,800:
 // 19.1 ms for five steps with four, 21.2 with none; 200,000: 38.3 for three with eight, 39.8 with four).
 static const int FF_WARP_MAX = 8000;
-// Particles up to which the mixed form's long FP64 searches are spread over the SMs, a warp per block:
-// there they bound the stage (12,800 particles: 18.3 ms for five steps, 19.0 in blocks of four warps).
-// Above it the double-float searches do, which want SMs of their own (70,000: 13.5 ms for two steps in
-// blocks of four warps, 15.1 spread; 200,000: the same).
-static const int LONG_SPREAD_MAX = 30000;
+// Particles up to which the mixed form's long FP64 searches take two warps each: there they bound the
+// stage.  Above it the double-float searches beside them do, which want SMs of their own, and the long
+// ones go in blocks of four warps (70,000 particles: 13.5 ms for two steps, 15.1 in blocks of one warp).
+static const int LONG_PAIR_MAX = 30000;
 static int ffRounds(const sqdem_ctx* c, const Dev& d) {
   const int n = std::max(c->load, d.NP);
   return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
@@ -2757,17 +2756,18 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
     c->launches += 3;
   } else {
     // four warps per SM for the warp searches: one per scheduler, whose FP64 pipe serves its chain
-    // alone
-    const int ws = std::min(4 * c->numSMs, d.Pcap);
+    // alone; in blocks of one warp, of four (mixed form of a large scene) or of a search's two
+    const int n = std::max(c->load, d.NP);
+    const int ws = std::min(4 * c->numSMs, d.Pcap), ws2 = std::min(2 * c->numSMs, d.Pcap);
+    auto fork = [&]() { cudaEventRecord(c->fork, s); cudaStreamWaitEvent(c->stream2, c->fork, 0); };
+    auto join = [&]() { cudaEventRecord(c->join, c->stream2); cudaStreamWaitEvent(s, c->join, 0); };
+    if (c->timingSearch) cudaEventRecord(c->ev[4], s);
+    fork();
     if (c->precision == SQDEM_MIXED) {
       // the long searches in FP64 beside the double-float searches, then the searches the
       // double-float kernels deferred
-      if (c->timingSearch) cudaEventRecord(c->ev[4], s);
-      cudaEventRecord(c->fork, s);
-      cudaStreamWaitEvent(c->stream2, c->fork, 0);
-      const int lb = std::max(c->load, d.NP) > LONG_SPREAD_MAX ? LM_BS : 32;
-      k_search_warp<<<nblk(ws, lb / 32), lb, 0, c->stream2>>>(d, WS_LONG, 0);
-      cudaEventRecord(c->join, c->stream2);
+      if (n <= LONG_PAIR_MAX) k_search_warp<2><<<ws2, 64, 0, c->stream2>>>(d, WS_LONG, 0);
+      else k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
       k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
       const int blocks = c->numSMs * searchBlocksPerSM(c);
       const int ffw = std::min(blocks, nblk(d.Pcap, LM_BS / 32));
@@ -2785,34 +2785,31 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
       }
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
       k_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      k_search_warp<<<ws, 32, 0, s>>>(d, WS_DEFERRED, 0);
-      cudaStreamWaitEvent(s, c->join, 0);
+      k_search_warp<2><<<ws2, 64, 0, s>>>(d, WS_DEFERRED, 0);
+      join();
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
       c->launches += 6 + 2 * rounds;
-    } else if (std::max(c->load, d.NP) <= WARP_SEARCH_MAX) {
-      if (c->timingSearch) cudaEventRecord(c->ev[4], s);
-      k_search_warp<<<ws, 32, 0, s>>>(d, WS_ALL, 0);
-      if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
-      c->launches += 2;
     } else {
-      if (c->timingSearch) cudaEventRecord(c->ev[4], s);
-      cudaEventRecord(c->fork, s);
-      cudaStreamWaitEvent(c->stream2, c->fork, 0);
-      k_search_warp<<<ws, 32, 0, c->stream2>>>(d, WS_LONG, 0);
-      cudaEventRecord(c->join, c->stream2);
-      const int wave = c->numSMs * searchBlocksPerSM(c);
-      k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
-      k_wave_probe<<<wave, LM_BS, 0, s>>>(d, 0);
-      const int rounds = waveRounds(c, d);
-      for (int r = 1; r < rounds; r++) {
-        k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
-        k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
+      if (n <= WARP_SEARCH_MAX) {
+        k_search_warp<2><<<ws2, 64, 0, c->stream2>>>(d, WS_LONG, 0);
+        k_search_warp<1><<<ws, 32, 0, s>>>(d, WS_MAIN, 0);
+        c->launches += 3;
+      } else {
+        k_search_warp<1><<<ws, 32, 0, c->stream2>>>(d, WS_LONG, 0);
+        const int wave = c->numSMs * searchBlocksPerSM(c);
+        k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
+        k_wave_probe<<<wave, LM_BS, 0, s>>>(d, 0);
+        const int rounds = waveRounds(c, d);
+        for (int r = 1; r < rounds; r++) {
+          k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
+          k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
+        }
+        k_search_warp<1><<<ws, 32, 0, s>>>(d, WS_TAIL, rounds);
+        k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
+        c->launches += 4 + 2 * rounds;
       }
-      k_search_warp<<<ws, 32, 0, s>>>(d, WS_TAIL, rounds);
-      k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      cudaStreamWaitEvent(s, c->join, 0);
+      join();
       if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
-      c->launches += 4 + 2 * rounds;
     }
   }
 }
