@@ -120,12 +120,12 @@ __device__ __forceinline__ void disfunction(const SqShape& A, const SqShape& B, 
   if (dot(contact, d) > 0) stop_flag = true;
 }
 
-__device__ __forceinline__ void centerLine(D3 pos1, D3 pos2, double para[2]) {
-  D3 d0 = pos2 - pos1;
+__device__ __forceinline__ void centerLineOf(D3 d0, double para[2]) {
   para[0] = atan2(d0.y, d0.x);
   para[1] = atan(d0.z / sqrt(d0.x * d0.x + d0.y * d0.y));
   para[0] += 1e-5; para[1] += 1e-5;
 }
+__device__ __forceinline__ void centerLine(D3 pos1, D3 pos2, double para[2]) { centerLineOf(pos2 - pos1, para); }
 
 }  // namespace sqdem
 

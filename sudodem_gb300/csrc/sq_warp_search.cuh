@@ -120,7 +120,8 @@ template <int W>
 __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_warp(Dev d, int mode, int waveRounds) {
   const unsigned FULL = 0xffffffffu;
   const SceneState& S = *d.S;
-  __shared__ WSlot slots[W == 1 ? LM_BS / 32 : 1][2][WS_POINTS * W];
+  extern __shared__ WSlot wsSlots[];   // per search of the block: two rounds of WS_POINTS * W (wsShared)
+  WSlot (*slots)[2][WS_POINTS * W] = reinterpret_cast<WSlot(*)[2][WS_POINTS * W]>(wsSlots);
   __shared__ int taken[W == 1 ? LM_BS / 32 : 1];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int own = W == 1 ? wib : 0;                 // the search's place in the block

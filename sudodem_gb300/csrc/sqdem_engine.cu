@@ -1204,6 +1204,23 @@ __device__ void finishHM(const Dev& d, int e, unsigned fl, int id1, const BodyVi
   d.A.flags[e] = fl | F_FORCE;
 }
 
+// Ip2_SuperquadricsMat_SuperquadricsMat_SuperquadricsPhys::go (Superquadrics.cpp:1086-1116): kn, ks,
+// tan(phi) of a pair with materials m1, m2 (a called function: once per pair's life)
+__device__ __noinline__ double4 linearPhys(const Dev& d, int id1, int mat1, int mat2) {
+  const double4 m1 = d.mats[mat1], m2 = d.mats[mat2];
+  double4 ph;
+  if (id1 > 5) {
+    double fa = fmin_ref(m1.z, m2.z);
+    ph.z = tan(fa);
+    ph.x = 2.0 * m1.x * m2.x / (m1.x + m2.x);
+    ph.y = 2.0 * m1.y * m2.y / (m1.y + m2.y);
+  } else {
+    ph.z = tan(m1.z); ph.x = m1.x; ph.y = m1.y;
+  }
+  ph.w = 0;
+  return ph;
+}
+
 // Geometry history writes, Ip2_SuperquadricsMat_SuperquadricsMat_SuperquadricsPhys::go
 // (Superquadrics.cpp:1086-1116) and SuperquadricsLaw::go (Superquadrics.cpp:1209-1361) for
 // one entry whose geometry g was just computed.
@@ -1239,16 +1256,7 @@ __device__ void finishEntry(const Dev& d, int e, unsigned fl, bool isNew, int id
   const double2 mb1 = d.matsB[b1.info.y], mb2 = d.matsB[b2.info.y];
   beta.x = fmax_ref(mb1.x, mb2.x); beta.y = fmax_ref(mb1.y, mb2.y);
   if (!(fl & F_PHYS)) {
-    const double4 m1 = d.mats[b1.info.y], m2 = d.mats[b2.info.y];
-    if (id1 > 5) {
-      double fa = fmin_ref(m1.z, m2.z);
-      ph.z = tan(fa);
-      ph.x = 2.0 * m1.x * m2.x / (m1.x + m2.x);
-      ph.y = 2.0 * m1.y * m2.y / (m1.y + m2.y);
-    } else {
-      ph.z = tan(m1.z); ph.x = m1.x; ph.y = m1.y;
-    }
-    ph.w = 0;
+    ph = linearPhys(d, id1, b1.info.y, b2.info.y);
     d.A.phys[e] = ph;
     fl |= F_PHYS;
   } else ph = d.A.phys[e];
@@ -1295,6 +1303,27 @@ __device__ void finishEntry(const Dev& d, int e, unsigned fl, bool isNew, int id
   d.A.flags[e] = fl;
 }
 
+// finishEntry for particles that do not touch, without a search: no FP64 arithmetic but a new pair's
+// Ip2.  ang: the contact angles are set to (ang0, ang1), else a new pair's are (0, 0).
+__device__ __forceinline__ void finishApart(const Dev& d, int e, unsigned fl, bool isNew, int id1, int m1, int m2, bool ang,
+                                            double ang0, double ang1) {
+  const double4 z = make_double4(0, 0, 0, 0);
+  if (ang) d.A.angle[e] = make_double2(ang0, ang1);
+  else if (isNew) d.A.angle[e] = make_double2(0, 0);
+  d.A.depth[e] = 0;
+  if (isNew) {
+    d.A.normal[e] = z; d.A.cp[e] = z;
+    if (d.prm->recordFull != 0) {
+      d.A.p1[e] = z; d.A.p2[e] = z; d.A.shearInc[e] = z; d.A.twist[e] = z; d.A.ortho[e] = z; d.A.relVn[e] = z; d.A.relVs[e] = z;
+      d.A.hmCurv[e] = z; d.A.hmEll[e] = z; d.A.hmSum[e] = make_double2(0, 0);
+    }
+  }
+  if (!(fl & F_PHYS)) d.A.phys[e] = linearPhys(d, id1, m1, m2);
+  d.A.nforce[e] = z;
+  d.A.shear[e] = z;
+  d.A.flags[e] = (fl | F_GEOM | F_PHYS | F_SHEARNEW) & ~(F_FORCE | F_ITERS_MASK);
+}
+
 __device__ __forceinline__ void entryIds(const Dev& d, int e, unsigned fl, int& id1, int& id2) {
   const int owner = d.A.owner[e], partner = d.A.partner[e];
   id1 = (fl & F_OWNER_ID1) ? owner : partner;
@@ -1322,16 +1351,16 @@ __device__ __forceinline__ void shapeInitF32(SqShapeF& s, const BodyView& b, F3 
 // point has a positive gap too, so lmder2 stops at its first check with stop_flag set
 // (Superquadrics_Ig2.cpp:1138-1143): not touching, contactAngle unchanged, depth 0.
 static const float SCREEN_MARGIN = 1e-4f;
-__device__ bool screenSeparated(const BodyView& b1, const BodyView& b2, double pa0, double pa1, D3 shift2) {
+// rel: centre of B relative to A's, rsum: the summed bounding radii.
+__device__ __forceinline__ bool screenSeparated(const BodyView& b1, const BodyView& b2, F3 rel, float rsum, double pa0, double pa1) {
   if (!isfinite(pa0) || !isfinite(pa1)) return false;
   SqShapeF A, B;
-  const D3 rel = (b2.pos + shift2) - b1.pos;
   shapeInitF32(A, b1, f3(0, 0, 0));
-  shapeInitF32(B, b2, f3((float)rel.x, (float)rel.y, (float)rel.z));
+  shapeInitF32(B, b2, rel);
   F3 p1, p2;
   float sep;
   disfunctionF(A, B, (float)pa0, (float)pa1, p1, p2, sep);
-  return sep > SCREEN_MARGIN * (float)(b1.shpA.w + b2.shpA.w);
+  return sep > SCREEN_MARGIN * rsum;
 }
 
 // The same screen for the Nelder-Mead search of the Hertz-Mindlin geometry over the three
@@ -1382,93 +1411,146 @@ __device__ int screenSeparatedNM(const BodyView& b1, const BodyView& b2, double 
   return 0;
 }
 
-// Pass 1 over the table: every entry that needs no Levenberg-Marquardt iteration is finished
-// here (bound-separated pairs, wall contacts, sphere pairs, bounding-sphere rejections, pairs the
-// FP32 screen proves separated at the LM start point); the rest is queued for pass 2.
-__global__ void __launch_bounds__(128, 3) k_contacts_pre(Dev d) {
+// SuperquadricsLaw's bound-separation erase (Superquadrics.cpp:1194-1207) discards what the geometry
+// functor computed, so it is tested first (B's bounds shifted by shift2).  True when entry e is done.
+__device__ __forceinline__ bool boundsApart(const Dev& d, const SceneState& S, int e, unsigned fl, int id1, int id2, D3 shift2) {
+  const double4 amn = d.bmin[id1], amx = d.bmax[id1];
+  double4 bmn = d.bmin[id2], bmx = d.bmax[id2];
+  if (S.periodic) {
+    bmn.x += shift2.x; bmn.y += shift2.y; bmn.z += shift2.z;
+    bmx.x += shift2.x; bmx.y += shift2.y; bmx.z += shift2.z;
+  }
+  if (!(amn.x >= bmx.x || bmn.x >= amx.x || amn.y >= bmx.y || bmn.y >= amx.y || amn.z >= bmx.z || bmn.z >= amx.z)) return false;
+  d.A.flags[e] = (fl & ~(F_GEOM | F_PHYS | F_FORCE)) | F_SHEARNEW;
+  d.A.nforce[e] = make_double4(0, 0, 0, 0);
+  d.A.shear[e] = make_double4(0, 0, 0, 0);
+  return true;
+}
+
+// Pairs of particles both flagged as spheres (a called function: its registers are not the kernel's).
+__device__ __noinline__ void finishSpheres(const Dev& d, int e, unsigned fl, int id1, int id2, D3 shift2, Counters& cnt) {
+  const SceneState& S = *d.S;
+  const BodyView b1 = loadBody(d, id1), b2 = loadBody(d, id2);
+  const bool isNew = !(fl & F_GEOM);
+  const double prevDepth = isNew ? 0.0 : d.A.depth[e];
+  const D3 oldNormal = isNew ? d3(0, 0, 0) : xyz(d.A.normal[e]);
+  const D3 oldCp = isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]);
+  const D3 shiftVel = shiftVelOf(S, *d.prm, shift2);
+  GeomOut g;
+  if (d.prm->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) geomSqSq2Simple(g, isNew, prevDepth, oldNormal, oldCp, b1, b2, d.prm->dt, shift2, shiftVel);
+  else geomSqSqSimple(g, isNew, prevDepth, oldNormal, oldCp, b1, b2, d.prm->dt, shift2, shiftVel);
+  finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
+}
+
+// The wall contacts, one thread per entry of the walls' lists.  They run beside pass 1 and the
+// searches: a support point is 9 pow in a row, 35 us, which pass 1 of every walled scene waited for.
+__global__ void __launch_bounds__(64) k_contacts_walls(Dev d) {
+  const SceneState& S = *d.S;
+  if (S.skip) return;
+  const int n = d.wCount[d.W - 1] + d.wCount[2 * d.W - 1];
+  const double dt = d.prm->dt;
+  Counters cnt = {0, 0, 0, 0, 0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int e = d.wList[i];
+    const unsigned fl = d.A.flags[e];
+    int id1, id2;
+    entryIds(d, e, fl, id1, id2);
+    if (d.info[id1].x != KIND_WALL) continue;   // an imported pair with the wall second: pass 1's
+    const D3 shift2 = cellShift(S, d.A.cd[e]);
+    if (boundsApart(d, S, e, fl, id1, id2, shift2)) continue;
+    const BodyView b1 = loadBody(d, id1), b2 = loadBody(d, id2);
+    const bool isNew = !(fl & F_GEOM);
+    GeomOut g;
+    geomWallSq(g, isNew, isNew ? 0.0 : d.A.depth[e], isNew ? d3(0, 0, 0) : xyz(d.A.normal[e]),
+               isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]), b1, b2, dt);
+    finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
+  }
+  flushCounters(d, cnt);
+}
+
+// Pass 1 over the table, pairs of particles: every entry that needs no Levenberg-Marquardt (HM:
+// Nelder-Mead) iteration is finished here (bound-separated pairs, sphere pairs, bounding-sphere
+// rejections, pairs the FP32 screen proves separated at the search's start point); the rest is queued
+// for pass 2.  What bounds it: FP64 instructions (positions, bounds, periodic shifts, the
+// conversions of the screen's operands: 87 an entry, the pipe 58% busy) and their latency: 168
+// registers held it to 12 warps per SM.  So the wall contacts have a kernel of their own, sphere
+// pairs a called function, what is apart is finished without the general finish, and the distance
+// test is taken in FP32 where it is clear.  A step of 200,000 in the mixed form 10.3 -> 9.96 ms, of a
+// servo specimen of 2,197 1.375 -> 1.29, of a deposition of 1,000 0.090 -> 0.083.
+template <bool HM>
+__global__ void __launch_bounds__(128, HM ? 3 : 4) k_contacts_pre(Dev d) {
   const SceneState& S = *d.S;
   if (S.skip) return;
   const int Pn = S.P;
-  const double dt = d.prm->dt;
   Counters cnt = {0, 0, 0, 0, 0};
   const int stride = gridDim.x * blockDim.x;
   for (int e0 = blockIdx.x * blockDim.x; e0 < Pn; e0 += stride) {
     const int e = e0 + threadIdx.x;
     bool queue = false, shortq = false;
     if (e < Pn) {
-      unsigned fl = d.A.flags[e];
+      const unsigned fl = d.A.flags[e];
       int id1, id2;
       entryIds(d, e, fl, id1, id2);
+      const int4 i1 = d.info[id1], i2 = d.info[id2];
       const D3 shift2 = cellShift(S, d.A.cd[e]);
-      // SuperquadricsLaw's bound-separation erase (Superquadrics.cpp:1194-1207) discards what
-      // the geometry functor computed, so it is tested first (B's bounds shifted by shift2).
-      const double4 amn = d.bmin[id1], amx = d.bmax[id1];
-      double4 bmn = d.bmin[id2], bmx = d.bmax[id2];
-      if (S.periodic) {
-        bmn.x += shift2.x; bmn.y += shift2.y; bmn.z += shift2.z;
-        bmx.x += shift2.x; bmx.y += shift2.y; bmx.z += shift2.z;
-      }
-      if (amn.x >= bmx.x || bmn.x >= amx.x || amn.y >= bmx.y || bmn.y >= amx.y || amn.z >= bmx.z || bmn.z >= amx.z) {
-        d.A.flags[e] = (fl & ~(F_GEOM | F_PHYS | F_FORCE)) | F_SHEARNEW;
-        d.A.nforce[e] = make_double4(0, 0, 0, 0);
-        d.A.shear[e] = make_double4(0, 0, 0, 0);
-      } else {
-        const BodyView b1 = loadBody(d, id1), b2 = loadBody(d, id2);
+      if (i1.x != KIND_WALL && !boundsApart(d, S, e, fl, id1, id2, shift2)) {
+        BodyView b1, b2;
+        b1.pos = xyz(d.pos[id1]); b1.ori = d.ori[id1]; b1.shpA = d.shpA[id1]; b1.shpB = d.shpB[id1]; b1.info = i1;
+        b2.pos = xyz(d.pos[id2]); b2.ori = d.ori[id2]; b2.shpA = d.shpA[id2]; b2.shpB = d.shpB[id2]; b2.info = i2;
         const bool isNew = !(fl & F_GEOM);
-        const double prevDepth = isNew ? 0.0 : d.A.depth[e];
-        const D3 oldNormal = isNew ? d3(0, 0, 0) : xyz(d.A.normal[e]);
-        const D3 oldCp = isNew ? d3(0, 0, 0) : xyz(d.A.cp[e]);
-        GeomOut g;
-        bool done = true;
-        if (b1.info.x == KIND_WALL) geomWallSq(g, isNew, prevDepth, oldNormal, oldCp, b1, b2, dt);
-        else if (d.prm->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) {
-          const bool sph = (b1.info.z != 0) && (b2.info.z != 0);
-          if (sph || nrm(b1.pos - b2.pos) > b1.shpA.w + b2.shpA.w) {
-            geomSqSq2Simple(g, isNew, prevDepth, oldNormal, oldCp, b1, b2, dt, shift2, shiftVelOf(S, *d.prm, shift2));
-          } else {
+        const bool sph = i1.z != 0 && i2.z != 0;
+        if (HM) {
+          if (sph || nrm(b1.pos - b2.pos) > b1.shpA.w + b2.shpA.w) finishSpheres(d, e, fl, id1, id2, shift2, cnt);
+          else {
             const double2 an = isNew ? make_double2(0, 0) : d.A.angle[e];
             const int nev = screenSeparatedNM(b1, b2, an.x, an.y, isNew ? 0.1 : 0.001);
             if (nev) {
+              GeomOut g;
               g.precomputed = false; g.nanNormal = false; g.lmIters = nev; g.lmStop = 0; g.lmCalls = 1; g.hm = 0;
-              g.cp = oldCp; g.depth = 0; g.isShearNew = true;
+              g.cp = d3(0, 0, 0); g.depth = 0; g.isShearNew = true;
               g.ang0 = an.x; g.ang1 = an.y; g.angSet = true;
               cnt.lmCalls++; cnt.lmIters += nev;
-            } else done = false;
+              finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
+            } else {
+              queue = true;
+              // searches expected short go to the back of the queue, so that the long ones start
+              // first: those of a contact touching at the previous step (the warm start usually
+              // converges on its first simplex)
+              shortq = !isNew && d.A.depth[e] > 0;
+            }
           }
-        } else {
-          const bool sph = (b1.info.z != 0) && (b2.info.z != 0);
-          if (!sph && !(nrm(b1.pos - (b2.pos + shift2)) > b1.shpA.w + b2.shpA.w)) {
-            double para[2];
-            if (isNew) centerLine(b1.pos, b2.pos + shift2, para);
-            else { const double2 an = d.A.angle[e]; para[0] = an.x; para[1] = an.y; }
-            if (screenSeparated(b1, b2, para[0], para[1], shift2)) {
-              g.precomputed = false; g.nanNormal = false; g.lmIters = 0; g.lmStop = 0; g.lmCalls = 1;
-              g.cp = oldCp; g.depth = 0; g.isShearNew = true;
-              g.ang0 = para[0]; g.ang1 = para[1]; g.angSet = true;
-              cnt.lmCalls++;
-            } else done = false;
-          } else geomSqSqSimple(g, isNew, prevDepth, oldNormal, oldCp, b1, b2, dt, shift2, shiftVelOf(S, *d.prm, shift2));
-        }
-        if (done) finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
+        } else if (sph) finishSpheres(d, e, fl, id1, id2, shift2, cnt);
         else {
-          queue = true;
-          // searches expected short go to the back of the queue, so that the long ones start
-          // first: Nelder-Mead searches of a contact touching at the previous step (the warm start
-          // usually converges on its first simplex), Levenberg-Marquardt searches of an existing
-          // contact that took fewer than 4 iterations at the last step
-          shortq = d.prm->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN
-                       ? (!isNew && prevDepth > 0)
-                       : (!isNew && ((fl & F_ITERS_MASK) >> F_ITERS_SHIFT) < LONG_ITERS_BUCKET);
-          // Levenberg-Marquardt searches that ran long at the last step go to the long-search queue
-          // (fbQueue, the longest from its front): a warp each (k_search_warp), in FP64 in both forms
-          // (a double-float search that long would be deferred)
-          const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
-          if (d.prm->contactModel != SQDEM_CONTACT_HERTZ_MINDLIN && !isNew && bucket >= d.prm->vlongBucket) {
-            queue = false;
-            shortq = false;
-            if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
-            else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
-            atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
+          const D3 rel = (b2.pos + shift2) - b1.pos;
+          const double rsum = b1.shpA.w + b2.shpA.w;
+          // |rel| > rsum, in FP32 outside a band of 1e-5 around it (and above FP32's subnormals)
+          const F3 relF = f3((float)rel.x, (float)rel.y, (float)rel.z);
+          const float d2 = dotf(relF, relF), rF = (float)rsum, r2 = rF * rF;
+          const bool clear = r2 > 1e-30f && (d2 > r2 * 1.00001f || d2 < r2 * 0.99999f);
+          const bool far = clear ? d2 > r2 : nrm(rel) > rsum;
+          if (far) finishApart(d, e, fl, isNew, id1, i1.y, i2.y, false, 0, 0);
+          else {
+            double para[2];
+            if (isNew) centerLineOf(rel, para);
+            else { const double2 an = d.A.angle[e]; para[0] = an.x; para[1] = an.y; }
+            if (screenSeparated(b1, b2, relF, rF, para[0], para[1])) {
+              finishApart(d, e, fl, isNew, id1, i1.y, i2.y, true, para[0], para[1]);
+              cnt.lmCalls++;
+            } else {
+              // searches expected short (fewer than 4 iterations at the last step) go to the back of
+              // the queue, so that the long ones start first; those that ran long at the last step
+              // go to the long-search queue (fbQueue, the longest from its front), in FP64 in both
+              // forms (a double-float search that long would be deferred)
+              const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
+              if (!isNew && bucket >= d.prm->vlongBucket) {
+                if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
+                else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
+                atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
+              } else {
+                queue = true;
+                shortq = !isNew && bucket < (int)LONG_ITERS_BUCKET;
+              }
+            }
           }
         }
       }
@@ -2627,7 +2709,8 @@ struct sqdem_ctx {
   int shapeSearch = 0, shapePass1 = 0;   // launch shapes set by the caller or the autotuner (0: defaults)
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;   // the long searches, beside the rest of the contact stage
-  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t stream3 = nullptr;   // the wall contacts, beside pass 1 and the searches
+  cudaEvent_t fork = nullptr, join = nullptr, join3 = nullptr;
   Dev d;
   bool haveBodies = false, haveMats = false, haveParams = false;
   cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr; bool graphValid = false;
@@ -2744,17 +2827,29 @@ static int ffRounds(const sqdem_ctx* c, const Dev& d) {
   return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
 }
 
+// shared memory of a k_search_warp<W> block: the trial points of its searches, two rounds of them
+static size_t wsShared(int W, int threads) { return sizeof(WSlot) * 2 * WS_POINTS * W * (threads / (32 * W)); }
+
 // The contact stage on c->stream: pass 1, then the searches of the selected contact model
 // (and, for Hertz-Mindlin, the finish pass of the contacts found touching).
 static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
   cudaStream_t s = c->stream;
   const int p1 = c->shapePass1 > 0 ? c->shapePass1 : PASS1_BLOCKS_PER_SM;
-  k_contacts_pre<<<std::min(nblk(d.Pcap, 128), c->numSMs * p1), 128, 0, s>>>(d);
+  const int pre = std::min(nblk(d.Pcap, 128), c->numSMs * p1);
+  if (d.W > 0) {   // the wall contacts, beside the rest of the stage
+    cudaEventRecord(c->fork, s);
+    cudaStreamWaitEvent(c->stream3, c->fork, 0);
+    k_contacts_walls<<<std::min(nblk(d.Pcap, 64), c->numSMs * 4), 64, 0, c->stream3>>>(d);
+    cudaEventRecord(c->join3, c->stream3);
+    c->launches++;
+  }
   if (c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) {
+    k_contacts_pre<true><<<pre, 128, 0, s>>>(d);
     k_contacts_nm<<<grid, LM_BS, 0, s>>>(d);
     k_contacts_nm_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
     c->launches += 3;
   } else {
+    k_contacts_pre<false><<<pre, 128, 0, s>>>(d);
     // four warps per SM for the warp searches: one per scheduler, whose FP64 pipe serves its chain
     // alone; in blocks of one warp, of four (mixed form of a large scene) or of a search's two
     const int n = std::max(c->load, d.NP);
@@ -2766,8 +2861,8 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
     if (c->precision == SQDEM_MIXED) {
       // the long searches in FP64 beside the double-float searches, then the searches the
       // double-float kernels deferred
-      if (n <= LONG_PAIR_MAX) k_search_warp<2><<<ws2, 64, 0, c->stream2>>>(d, WS_LONG, 0);
-      else k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, 0, c->stream2>>>(d, WS_LONG, 0);
+      if (n <= LONG_PAIR_MAX) k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0);
+      else k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0);
       k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
       const int blocks = c->numSMs * searchBlocksPerSM(c);
       const int ffw = std::min(blocks, nblk(d.Pcap, LM_BS / 32));
@@ -2785,17 +2880,17 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
       }
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
       k_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      k_search_warp<2><<<ws2, 64, 0, s>>>(d, WS_DEFERRED, 0);
+      k_search_warp<2><<<ws2, 64, wsShared(2, 64), s>>>(d, WS_DEFERRED, 0);
       join();
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
       c->launches += 6 + 2 * rounds;
     } else {
       if (n <= WARP_SEARCH_MAX) {
-        k_search_warp<2><<<ws2, 64, 0, c->stream2>>>(d, WS_LONG, 0);
-        k_search_warp<1><<<ws, 32, 0, s>>>(d, WS_MAIN, 0);
+        k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0);
+        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_MAIN, 0);
         c->launches += 3;
       } else {
-        k_search_warp<1><<<ws, 32, 0, c->stream2>>>(d, WS_LONG, 0);
+        k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0);
         const int wave = c->numSMs * searchBlocksPerSM(c);
         k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
         k_wave_probe<<<wave, LM_BS, 0, s>>>(d, 0);
@@ -2804,7 +2899,7 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
           k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
           k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
         }
-        k_search_warp<1><<<ws, 32, 0, s>>>(d, WS_TAIL, rounds);
+        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_TAIL, rounds);
         k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
         c->launches += 4 + 2 * rounds;
       }
@@ -2812,6 +2907,7 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
       if (c->timingSearch) { cudaEventRecord(c->ev[5], s); cudaEventRecord(c->ev[6], s); }
     }
   }
+  if (d.W > 0) cudaStreamWaitEvent(s, c->join3, 0);
 }
 
 // The collider pass on c->stream (every kernel tests runCollider).
@@ -2984,6 +3080,8 @@ sqdem_status sqdem_create(sqdem_ctx** out, const sqdem_config* cfg) {
   CK(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->join, cudaEventDisableTiming));
+  CK(cudaStreamCreateWithFlags(&c->stream3, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&c->join3, cudaEventDisableTiming));
   CK(cudaDeviceGetAttribute(&c->numSMs, cudaDevAttrMultiProcessorCount, c->device));
   {
     int nb = 0;
@@ -3011,6 +3109,8 @@ void sqdem_destroy(sqdem_ctx* c) {
   for (int i = 0; i < 7; i++) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->fork) cudaEventDestroy(c->fork);
   if (c->join) cudaEventDestroy(c->join);
+  if (c->join3) cudaEventDestroy(c->join3);
+  if (c->stream3) cudaStreamDestroy(c->stream3);
   if (c->stream2) cudaStreamDestroy(c->stream2);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

@@ -6,6 +6,7 @@ import pytest
 
 from oracle import OracleScene
 from sudodem_gb300 import Engine, SqdemError, assemblies
+from sudodem_gb300._native import shape_props
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +87,21 @@ def test_host_limits(gpu):
     e2 = Engine(device=0)
     with pytest.raises(SqdemError):
         e2.step(1)                # bodies and materials first
+
+
+@pytest.mark.parametrize("size", [1e-3, 1.0, 1e-17])
+@pytest.mark.parametrize("off", [-2e-5, -3e-6, -1e-15, 0.0, 1e-15, 3e-6, 2e-5])
+def test_bounding_sphere_rejection_near_its_threshold(gpu, size, off):
+    """Pairs whose centres are at the summed bounding radii times (1 + off).  A pair beyond them is
+    rejected without a start point (contactAngle (0, 0)), any other gets the centre line's.  The FP32
+    test decides outside a band around the threshold only, so the answer is FP64's at every size."""
+    s1, s2 = [size, 0.9 * size, 0.8 * size, 0.7, 1.3], [0.9 * size, 0.8 * size, size, 1.1, 0.9]
+    rsum = shape_props(*s1)[4] + shape_props(*s2)[4]
+    gap = rsum * (1 + off)
+    spec = assemblies.pair_scene(s1, s2, [0, 0, 0], [gap, 0, 0], [1, 0, 0, 0], [1, 0, 0, 0], walls=False)
+    spec.params["verletDist"] = size
+    eng = _engine(spec)
+    eng.step(1); eng.sync()
+    recs = eng.interactions(True)
+    assert len(recs) == 1
+    assert np.all(recs[0, 5:7] == 0) == (gap > rsum)
