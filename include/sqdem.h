@@ -209,12 +209,10 @@ sqdem_status sqdem_put_scalars(sqdem_ctx* ctx, const double* in9);
  * the step then writes only the history the next step needs. */
 sqdem_status sqdem_set_record_full(sqdem_ctx* ctx, int on);
 
-/* Schedule of the search evaluations of the double-float and Nelder-Mead kernels (no counterpart
- * in the reference, which runs one search per thread).  on = 1 (default): once the contact queue is
- * drained, lanes without a contact evaluate the points the searches still running in their warp
- * will ask for next; on = 0: every lane evaluates only its own search's point.  Results are
- * identical bit for bit; only the time of the longest searches changes.  (The FP64
- * Levenberg-Marquardt searches have one schedule.) */
+/* Schedule of the evaluations of the Nelder-Mead searches (no counterpart in the reference, which
+ * runs one search per thread).  on = 1 (default): the lanes a search does not need evaluate the
+ * points it may ask for next; on = 0: one point per search and round.  Results are identical bit
+ * for bit; only the time changes.  (The Levenberg-Marquardt searches have one schedule.) */
 sqdem_status sqdem_set_lm_spread(sqdem_ctx* ctx, int on);
 
 /* Periodic-boundary correction, off by default (the reference's behaviour).  For a contact

@@ -243,54 +243,83 @@ __device__ __forceinline__ bool nmConsume(NMState& M, double f, bool apart) {
   }
 }
 
-// amotry's trial point for the factor fac from the vertex sum ps and the high vertex ph
-__device__ __forceinline__ double2 nmTryPoint(const double ps[2], const double ph[2], double fac) {
-  const double fac1 = (1.0 - fac) / 2.0;
-  const double fac2 = fac1 - fac;
-  return make_double2(ps[0] * fac1 - ph[0] * fac2, ps[1] * fac1 - ph[1] * fac2);
-}
+// Points the search may ask for after the one it asks for now, in the order of their use: point k of
+// the plan (k = 0: the one asked for); false if there is none.  After the first simplex (whose
+// ranking is not known in advance) a point follows from the vertex sum ps, the high vertex H, the
+// second highest N and the point T asked for in one or two steps of the machine, each of the form
+// amotry(vertex sum, vertex, factor); which ones, the bits of nmPlans say (all values distinct: what an
+// evaluation's class leads to is known before its value).  Every point is computed with the operations the
+// machine uses, so one that it later asks for matches bit for bit; one it does not ask for is
+// dropped.  With twelve points a round the longest searches of a packed lattice (63-85 evaluations) take
+// 27-41 rounds; with the five points of one step of the machine alone they took 45-56.
+enum {
+  NP_REP = 1,                                   // T has replaced H in the vertex sum
+  NP_H = 0, NP_T = 2, NP_N = 4,                 // vertex of the first step
+  NP_R = 0, NP_C = 8, NP_E = 16,                // its factor: reflection -1, contraction 0.5, expansion 2
+  NP_2 = 32, NP_2I = 64,                        // a second step, which its point (I) precedes: through N, or through I
+  NP_2C = 128, NP_2E = 256,                     // its factor (else -1)
+  NP_S1 = 512, NP_S2 = 1024,                    // the first, the second vertex of the shrink
+  NP_NONE = 2048
+};
+static const int NM_POINTS = 12;
+static __constant__ unsigned short nmPlans[3][NM_POINTS] = {
+    // reflection: contraction from the old or the new simplex, expansion, the next reflection if it is
+    // neither best nor worst; the reflections after these; the shrink; what follows the next reflection
+    {0, NP_H | NP_C, NP_REP | NP_T | NP_C, NP_REP | NP_T | NP_E, NP_REP | NP_N, NP_H | NP_C | NP_2, NP_REP | NP_T | NP_C | NP_2,
+     NP_REP | NP_T | NP_E | NP_2, NP_S1, NP_S2, NP_REP | NP_N | NP_C, NP_REP | NP_N | NP_2 | NP_2I | NP_2C},
+    // expansion: the next reflection with or without it, and what follows
+    {0, NP_REP | NP_N, NP_N, NP_REP | NP_N | NP_C, NP_N | NP_C, NP_REP | NP_N | NP_2 | NP_2I | NP_2E,
+     NP_REP | NP_N | NP_2 | NP_2I | NP_2C, NP_N | NP_2 | NP_2I | NP_2E, NP_N | NP_2 | NP_2I | NP_2C, NP_NONE, NP_NONE, NP_NONE},
+    // contraction: the next reflection through N or through the contracted vertex, the shrink, and
+    // what follows the reflections
+    {0, NP_REP | NP_N, NP_S1, NP_S2, NP_REP | NP_T, NP_REP | NP_N | NP_C, NP_REP | NP_N | NP_2 | NP_2I | NP_2C,
+     NP_REP | NP_N | NP_2 | NP_2I | NP_2E, NP_REP | NP_T | NP_C, NP_REP | NP_T | NP_2 | NP_2I | NP_2C,
+     NP_REP | NP_T | NP_2 | NP_2I | NP_2E, NP_NONE}};
 
-// Points the search asks for after the one it asks for now, under the outcomes of that
-// evaluation (written to q[1..], at most S - 1 of them; returns how many points, q[0] being
-// the current one).  Every point is computed with the operations the state machine uses, so
-// one that the search later asks for matches bit for bit.  The vertex order after an
-// evaluation follows from the comparison that selects the branch (all values distinct).
-__device__ __forceinline__ int nmPlan(const NMState& M, double2* q, int S) {
-  int n = 0;
-  q[n++] = make_double2(M.q0, M.q1);
-  if (M.st == NM_V0 || M.st == NM_V1 || M.st == NM_V2) {
-    // vertices of the first simplex still to be evaluated; after the third the next point
-    // depends on the ranking, which is not known yet
-    for (int v = M.st + 1; v < 3 && n < S; v++) q[n++] = make_double2(M.p[v][0], M.p[v][1]);
-    return n;
+// amotry's (1 - fac) / 2 and (1 - fac) / 2 - fac for the factors -1, 0.5, 2, all exact
+__device__ __forceinline__ double2 nmTryPoint(const double2 ps, const double2 ph, bool c, bool e) {
+  const double fac1 = e ? -0.5 : c ? 0.25 : 1.0, fac2 = e ? -2.5 : c ? -0.25 : 2.0;
+  return make_double2(ps.x * fac1 - ph.x * fac2, ps.y * fac1 - ph.y * fac2);
+}
+__device__ __forceinline__ double2 nmShrunk(const NMState& M, int i) {
+  return make_double2(0.5 * (M.p[i][0] + M.p[M.ilo][0]), 0.5 * (M.p[i][1] + M.p[M.ilo][1]));
+}
+__device__ __forceinline__ bool nmPlanned(const NMState& M, int k, double2& q) {
+  q = make_double2(M.q0, M.q1);
+  if (k == 0) return true;
+  if (M.st <= NM_V2) {   // the vertices left
+    const int v = M.st + k;
+    if (v > 2) return false;
+    q = make_double2(M.p[v][0], M.p[v][1]);
+    return true;
   }
-  const double* ph = M.p[M.ihi];
-  double psA[2];   // vertex sum once the trial point replaces the high vertex
-  psA[0] = M.psum[0] + (M.ptry[0] - ph[0]);
-  psA[1] = M.psum[1] + (M.ptry[1] - ph[1]);
-  if (M.st == NM_REFLECT) {
-    // better than the best: expansion; worse than the second highest: contraction (from the
-    // simplex with or without the trial point); in between: the next reflection, through the
-    // old second-highest vertex, now the highest
-    if (n < S) q[n++] = nmTryPoint(psA, M.ptry, 2.0);
-    if (n < S) q[n++] = nmTryPoint(psA, M.ptry, 0.5);
-    if (n < S) q[n++] = nmTryPoint(M.psum, ph, 0.5);
-    if (n < S) q[n++] = nmTryPoint(psA, M.p[M.inhi], -1.0);
-  } else if (M.st == NM_EXPAND) {
-    // the expanded vertex stays the lowest; the next reflection goes through the old
-    // second-highest vertex, with or without the expansion point in the sum
-    if (n < S) q[n++] = nmTryPoint(psA, M.p[M.inhi], -1.0);
-    if (n < S) q[n++] = nmTryPoint(M.psum, M.p[M.inhi], -1.0);
-  } else {
-    // a rejected contraction (or a shrink step) continues with the shrink towards the low vertex
-    const int from = M.st == NM_SHRINK ? M.si + 1 : 0;
-    for (int i = from; i < 3 && n < S; i++)
-      if (i != M.ilo) {
-        q[n++] = make_double2(0.5 * (M.p[i][0] + M.p[M.ilo][0]), 0.5 * (M.p[i][1] + M.p[M.ilo][1]));
-        break;
-      }
+  const int a = M.ilo == 0 ? 1 : 0, b = M.ilo == 2 ? 1 : 2;   // the vertices that shrink, in order
+  if (M.st == NM_SHRINK) {   // the second vertex, then the reflections of the shrunk simplex
+    const double2 A = M.si == a ? make_double2(M.p[a][0], M.p[a][1]) : nmShrunk(M, a);
+    const double2 B = M.si == b ? make_double2(M.p[b][0], M.p[b][1]) : nmShrunk(M, b);
+    if (k == 1 && M.si == a) { q = B; return true; }
+    const int v = k - (M.si == a ? 1 : 0);   // 1: through the second vertex, 2: the first
+    if (v > 2) return false;
+    const double2 v0 = a == 0 ? A : make_double2(M.p[0][0], M.p[0][1]);
+    const double2 v1 = a == 1 ? A : b == 1 ? B : make_double2(M.p[1][0], M.p[1][1]);
+    const double2 v2 = b == 2 ? B : make_double2(M.p[2][0], M.p[2][1]);
+    q = nmTryPoint(make_double2((v0.x + v1.x) + v2.x, (v0.y + v1.y) + v2.y), v == 1 ? B : A, false, false);
+    return true;
   }
-  return n;
+  const unsigned c = nmPlans[M.st - NM_REFLECT][k];
+  if (c & NP_NONE) return false;
+  if (c & (NP_S1 | NP_S2)) { q = nmShrunk(M, (c & NP_S1) ? a : b); return true; }
+  const double2 T = make_double2(M.ptry[0], M.ptry[1]), H = make_double2(M.p[M.ihi][0], M.p[M.ihi][1]);
+  const double2 N = make_double2(M.p[M.inhi][0], M.p[M.inhi][1]);
+  double2 ps = make_double2(M.psum[0], M.psum[1]);
+  if (c & NP_REP) ps = make_double2(ps.x + (T.x - H.x), ps.y + (T.y - H.y));
+  const double2 ph = (c & NP_T) ? T : (c & NP_N) ? N : H;
+  q = nmTryPoint(ps, ph, c & NP_C, c & NP_E);
+  if (c & NP_2) {
+    ps = make_double2(ps.x + (q.x - ph.x), ps.y + (q.y - ph.y));
+    q = nmTryPoint(ps, (c & NP_2I) ? q : N, c & NP_2C, c & NP_2E);
+  }
+  return true;
 }
 
 }  // namespace sqdem

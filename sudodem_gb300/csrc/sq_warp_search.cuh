@@ -37,6 +37,15 @@ struct WShape {
   D3 pos;
 };
 
+__device__ __forceinline__ void warpShape(const Dev& d, int b, WShape& s) {
+  const double4 a = d.shpA[b], x = d.shpB[b], q = d.ori[b];
+  s.rx = a.x; s.ry = a.y; s.rz = a.z; s.rmax = a.w; s.e1 = x.x; s.e2 = x.y;
+  s.a1 = 2. - x.x; s.i1 = 1 / (2. - x.x); s.i2 = 1 / (2. - x.y);
+  const Rot R = quatToRot(q.x, q.y, q.z, q.w);
+  for (int i = 0; i < 9; i++) s.R[i] = R.m[i];
+  s.pos = xyz(d.pos[b]);
+}
+
 // What a round leaves in the lanes of each point's group.
 struct WEval {
   double pxy, pz;    // support point of the lane's body: x (k = 0) or y (k = 1), and z
@@ -45,8 +54,10 @@ struct WEval {
   D3 c;              // contact direction at the point
 };
 
-// g0: first lane of the group, r: the lane's place in it (0, 1: body A; 2, 3: body B; 4: v of both)
-__device__ __forceinline__ void warpEval(const WShape& s, double e1B, int g0, int r, double q0, double q1, WEval& o) {
+// g0: first lane of the group, r: the lane's place in it (0, 1: body A; 2, 3: body B; 4: v of both);
+// G: frame of the angles, if any (the Hertz-Mindlin model's Disfun)
+__device__ __forceinline__ void warpEval(const WShape& s, double e1B, int g0, int r, double q0, double q1, WEval& o,
+                                         const Rot* G = nullptr) {
   const unsigned FULL = 0xffffffffu;
   const bool isB = r == 2 || r == 3, k = r == 1 || r == 3, extra = r == 4;
   const int mate = extra ? g0 + 1 : g0 + (r ^ 1);
@@ -55,6 +66,7 @@ __device__ __forceinline__ void warpEval(const WShape& s, double e1B, int g0, in
   const double sa0 = __shfl_sync(FULL, sv, g0), ca0 = __shfl_sync(FULL, cv, g0);
   const double sa1 = __shfl_sync(FULL, sv, g0 + 1), ca1 = __shfl_sync(FULL, cv, g0 + 1);
   o.c = d3(ca0 * ca1, sa0 * ca1, sa1);
+  if (G) o.c = mulG(*G, o.c);
   // local normal +-R^T c: x on k = 1, y on k = 0, z on both
   double na = (k ? s.R[0] : s.R[1]) * o.c.x + ((k ? s.R[3] : s.R[4]) * o.c.y + (k ? s.R[6] : s.R[7]) * o.c.z);
   double nz = s.R[2] * o.c.x + (s.R[5] * o.c.y + s.R[8] * o.c.z);
@@ -167,13 +179,7 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
     const bool bodyB = r == 2 || r == 3;
     WShape s;
     {
-      const int b = bodyB ? id2 : id1;
-      const double4 a = d.shpA[b], x = d.shpB[b], q = d.ori[b];
-      s.rx = a.x; s.ry = a.y; s.rz = a.z; s.rmax = a.w; s.e1 = x.x; s.e2 = x.y;
-      s.a1 = 2. - x.x; s.i1 = 1 / (2. - x.x); s.i2 = 1 / (2. - x.y);
-      const Rot R = quatToRot(q.x, q.y, q.z, q.w);
-      for (int i = 0; i < 9; i++) s.R[i] = R.m[i];
-      s.pos = xyz(d.pos[b]);
+      warpShape(d, bodyB ? id2 : id1, s);
       if (bodyB) s.pos = s.pos + cellShift(S, d.A.cd[e]);
     }
     const double e1B = d.shpB[id2].x;

@@ -73,7 +73,8 @@ struct PairLane {
   SqShape s;
   bool isB;
 };
-__device__ __forceinline__ void pairLoad(const Dev& d, int e, bool isB, PairLane& l) {
+// shift: body B's nearest image (the Hertz-Mindlin search takes the positions as they are)
+__device__ __forceinline__ void pairLoad(const Dev& d, int e, bool isB, PairLane& l, bool shift = true) {
   const unsigned fl = d.A.flags[e];
   int id1, id2;
   entryIds(d, e, fl, id1, id2);
@@ -82,21 +83,24 @@ __device__ __forceinline__ void pairLoad(const Dev& d, int e, bool isB, PairLane
   shapeInit(l.s, a.x, a.y, a.z, x.x, x.y, a.w);
   l.s.R = quatToRot(q.x, q.y, q.z, q.w);
   l.s.pos = xyz(d.pos[b]);
-  if (isB) l.s.pos = l.s.pos + cellShift(*d.S, d.A.cd[e]);
+  if (isB && shift) l.s.pos = l.s.pos + cellShift(*d.S, d.A.cd[e]);
   l.isB = isB;
 }
 __device__ __forceinline__ D3 swapD3(D3 a) {
   const unsigned FULL = 0xffffffffu;
   return d3(__shfl_xor_sync(FULL, a.x, 1), __shfl_xor_sync(FULL, a.y, 1), __shfl_xor_sync(FULL, a.z, 1));
 }
-// Disfunction at (q0, q1): support points, their difference and c . (p2 - p1)
-__device__ __forceinline__ void pairEval(const PairLane& l, double q0, double q1, D3& c, D3& P1, D3& P2, D3& f, double& sep) {
+// Disfunction at (q0, q1), in the frame G if given (Disfun): support points, their difference and
+// c . (p2 - p1)
+__device__ __forceinline__ void pairEval(const PairLane& l, double q0, double q1, D3& c, D3& P1, D3& P2, D3& f, double& sep,
+                                         const Rot* G = nullptr) {
   const unsigned FULL = 0xffffffffu;
   double sv, cv;
   sincos(l.isB ? q1 : q0, &sv, &cv);
   const double so = __shfl_xor_sync(FULL, sv, 1), co = __shfl_xor_sync(FULL, cv, 1);
   const double sa0 = l.isB ? so : sv, ca0 = l.isB ? co : cv, sa1 = l.isB ? sv : so, ca1 = l.isB ? cv : co;
   c = d3(ca0 * ca1, sa0 * ca1, sa1);
+  if (G) c = mulG(*G, c);
   D3 n = mulL(l.s.R, c);
   if (l.isB) n = -n;
   const D3 own = mulG(l.s.R, supportLocal(l.s, n)) + l.s.pos;

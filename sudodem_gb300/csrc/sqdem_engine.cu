@@ -72,6 +72,9 @@ static const unsigned LONG_ITERS_BUCKET = 3;   // iterations >= 4
 // (32 specimens of 300-4,000 particles: 13.6 ms for two steps from 16, 14.8 from 8).
 static const int LONG_BUCKET_MIXED = 6, LONG_BUCKET_FP64 = 4, LONG_BUCKET_BATCH = 5;
 static const int LONG_FRONT_MIXED = 7, LONG_FRONT_FP64 = 6;
+// Hertz-Mindlin model: 32 and 64 Nelder-Mead evaluations (a packed lattice of 20,000: 2.1 ms a step, 2.27
+// from 16; 19 in 20 of those searches take 32 again at the next step).
+static const int LONG_BUCKET_NM = 6, LONG_FRONT_NM = 7;
 __device__ __forceinline__ unsigned itersBucket(int iters) { return iters > 0 ? min(15u, 32u - __clz((unsigned)iters)) : 0u; }
 enum { KIND_SQ = 0, KIND_WALL = 1 };
 static const unsigned DOF_ALL = 63u;
@@ -117,7 +120,7 @@ struct SceneState {
   int lmCount, lmHead;
   int vlCount, vlHead;   // long-search queue, from the front of fbQueue: the longest at the last step
   int fbCount, fbHead;   // searches the mixed form deferred to FP64 (deferQueue)
-  int nmFin;   // Hertz-Mindlin searches that ended touching, for the finish pass
+  int unused;  // keeps the layout of saved states
   int nmShort; // searches queued from the back of the queue (expected short)
   int numReinit; long long colliderRuns;
   unsigned long long bbLo[3], bbHi[3];   // order-preserving encodings of the bbox of particle bound centres
@@ -315,7 +318,7 @@ __global__ void k_scan_apply(const int* __restrict__ in, int n, const int* __res
 __global__ void k_gate(Dev d) {
   SceneState& S = *d.S;
   S.skip = (S.haltAt >= 0 && S.iter >= S.haltAt) ? 1 : 0;
-  if (S.skip) { S.runCollider = 0; S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0; *d.Q = QueueState(); return; }
+  if (S.skip) { S.runCollider = 0; S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmShort = 0; *d.Q = QueueState(); return; }
   if (S.newtonRan) {
     const double code = S.maxDispCode == 2 ? 2.0 : (S.maxDispCode == 1 ? 0.5 : 0.0);
     S.maxVelocitySq = fmax_ref(S.cellTerm, code);
@@ -344,7 +347,7 @@ __global__ void k_gate(Dev d) {
     else run = 0;
   }
   S.runCollider = run;
-  S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmFin = 0; S.nmShort = 0; *d.Q = QueueState();
+  S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmShort = 0; *d.Q = QueueState();
   if (run) {
     int init = 0;
     if (S.doSort) { init = 1; S.doSort = 0; }
@@ -1139,6 +1142,7 @@ __device__ void finishHM(const Dev& d, int e, unsigned fl, int id1, const BodyVi
     ph.w = 0;
     fl |= F_PHYS;
   } else ph = d.A.phys[e];
+  fl = (fl & ~F_ITERS_MASK) | (itersBucket(g.lmCalls > 0 ? g.lmIters : 0) << F_ITERS_SHIFT);
   const double2 beta = make_double2(fmax_ref(mb1.x, mb2.x), fmax_ref(mb1.y, mb2.y));
   if (!(g.depth > 1E-18)) {
     d.A.phys[e] = ph;
@@ -1427,6 +1431,16 @@ __device__ __forceinline__ bool boundsApart(const Dev& d, const SceneState& S, i
   return true;
 }
 
+// Queues a search that ran long at the last step for a warp of its own; false: it did not.
+__device__ __forceinline__ bool longSearch(const Dev& d, int e, unsigned fl) {
+  const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
+  if (bucket < d.prm->vlongBucket) return false;
+  if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
+  else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
+  atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
+  return true;
+}
+
 // Pairs of particles both flagged as spheres (a called function: its registers are not the kernel's).
 __device__ __noinline__ void finishSpheres(const Dev& d, int e, unsigned fl, int id1, int id2, D3 shift2, Counters& cnt) {
   const SceneState& S = *d.S;
@@ -1512,11 +1526,11 @@ __global__ void __launch_bounds__(128, HM ? 3 : 4) k_contacts_pre(Dev d) {
               cnt.lmCalls++; cnt.lmIters += nev;
               finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
             } else {
-              queue = true;
-              // searches expected short go to the back of the queue, so that the long ones start
-              // first: those of a contact touching at the previous step (the warm start usually
-              // converges on its first simplex)
-              shortq = !isNew && d.A.depth[e] > 0;
+              // searches that ran long at the last step go to the long-search queue; of the others
+              // those of a contact touching then (whose warm start usually converges on its first
+              // simplex) to the back of the queue, so that a warp's searches are alike
+              queue = isNew || !longSearch(d, e, fl);
+              shortq = queue && !isNew && d.A.depth[e] > 0;
             }
           }
         } else if (sph) finishSpheres(d, e, fl, id1, id2, shift2, cnt);
@@ -1541,15 +1555,8 @@ __global__ void __launch_bounds__(128, HM ? 3 : 4) k_contacts_pre(Dev d) {
               // the queue, so that the long ones start first; those that ran long at the last step
               // go to the long-search queue (fbQueue, the longest from its front), in FP64 in both
               // forms (a double-float search that long would be deferred)
-              const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
-              if (!isNew && bucket >= d.prm->vlongBucket) {
-                if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
-                else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
-                atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
-              } else {
-                queue = true;
-                shortq = !isNew && bucket < (int)LONG_ITERS_BUCKET;
-              }
+              queue = isNew || !longSearch(d, e, fl);
+              shortq = queue && !isNew && (fl & F_ITERS_MASK) >> F_ITERS_SHIFT < LONG_ITERS_BUCKET;
             }
           }
         }
@@ -1630,83 +1637,6 @@ __device__ __forceinline__ void finishSearch(const Dev& d, int e, unsigned fl, i
   finishEntry(d, e, fl, isNew, id1, b1, b2, g, cnt);
 }
 
-// One Disfunction evaluation (Superquadrics_Ig2.cpp:622-687) by a group of six lanes:
-// lanes 0-2 of the group compute body A's support point, lanes 3-5 body B's, and the
-// independent pow calls of each level of supportLocal run on separate lanes (Y,X,W |
-// t,u,v | Z | pc1,w), so that the dependency chain is 4 pow + 2 atan2 + 3 sincos instead of
-// 18 pow + 4 atan2 + 6 sincos.  Every value is computed with the operations of
-// disfunction/supportLocal (bitwise the same results).  Lane 0 of the group ends with p1,
-// p2 and the stop predicate.  All 32 lanes call it (full-warp shuffles); g0 is the group's
-// first lane, sub the lane's place in it.  (Four-lane groups, eight points per round, were
-// measured slower: one more pow on the chain.)
-static const int COOP_LANES = 6, COOP_POINTS = 5;
-__device__ __forceinline__ void coopEval(const SqShape& A, const SqShape& B, double q0, double q1, int g0, int sub,
-                                         D3& p1, D3& p2, bool& flag, const Rot* G = nullptr, double* dist = nullptr) {
-  const unsigned FULL = 0xffffffffu;
-  const int body = sub >= 3 ? 1 : 0;
-  const int k = sub - 3 * body;
-  const int gb = g0 + 3 * body;
-  const SqShape& s = body ? B : A;
-  double sv, cv;
-  sincos(sub == 1 ? q1 : q0, &sv, &cv);
-  const double sa0 = __shfl_sync(FULL, sv, g0), ca0 = __shfl_sync(FULL, cv, g0);
-  const double sa1 = __shfl_sync(FULL, sv, g0 + 1), ca1 = __shfl_sync(FULL, cv, g0 + 1);
-  const D3 contact = G ? mulG(*G, d3(ca0 * ca1, sa0 * ca1, sa1)) : d3(ca0 * ca1, sa0 * ca1, sa1);
-  D3 n = mulL(s.R, contact);
-  if (body) n = (-1.0) * n;
-  const double v1 = pow(k == 0 ? fabs(s.ry * n.y) : fabs(s.rx * n.x), k == 2 ? s.i2 : s.i1);
-  const double Y = __shfl_sync(FULL, v1, gb), X = __shfl_sync(FULL, v1, gb + 1), W = __shfl_sync(FULL, v1, gb + 2);
-  const double ph0 = atan2(sgn(n.y) * Y, sgn(n.x) * X);
-  double s0, c0;
-  sincos(ph0, &s0, &c0);
-  const double v2 = pow(k == 2 ? fabs(s0) : fabs(c0), k == 0 ? s.a1 : s.e1);
-  const double t = __shfl_sync(FULL, v2, gb), u = __shfl_sync(FULL, v2, gb + 1), v = __shfl_sync(FULL, v2, gb + 2);
-  const double Z = pow(fabs(s.rz * n.z * t), s.i2);
-  const double ph1 = atan2(sgn(n.z) * Z, W);
-  double s1, c1;
-  sincos(ph1, &s1, &c1);
-  const double v3 = pow(k == 1 ? fabs(s1) : fabs(c1), s.e2);
-  const double pc1 = __shfl_sync(FULL, v3, gb), w = __shfl_sync(FULL, v3, gb + 1);
-  D3 r;
-  r.x = sgn(c0) * s.rx * u * pc1;
-  r.y = sgn(s0) * s.ry * v * pc1;
-  r.z = sgn(s1) * s.rz * w;
-  const D3 p = mulG(s.R, r) + s.pos;
-  const double x2 = __shfl_sync(FULL, p.x, g0 + 3), y2 = __shfl_sync(FULL, p.y, g0 + 3), z2 = __shfl_sync(FULL, p.z, g0 + 3);
-  p1 = p;
-  p2 = d3(x2, y2, z2);
-  const D3 dd = p2 - p1;
-  flag = dot(contact, dd) > 0;
-  if (dist) *dist = nrm(dd);
-}
-
-// Slot allocation of one evaluation round: every searching lane (in) gets one slot, the rest
-// of the budget goes evenly to all, the remainder to the searches of highest priority (prio:
-// the long-search flag above the rounds run so far, the likeliest to bound the kernel), at
-// most maxExtra more each.  Returns the lane's slot count (spc) and first slot (base), and the
-// round's largest slot count (jmax) for the uniform consume pass.
-__device__ __forceinline__ void allocSlots(bool in, unsigned prio, int budget, int maxExtra, int& spc, int& base,
-                                           int& jmax) {
-  const int lane = threadIdx.x & 31;
-  const unsigned act = __ballot_sync(0xffffffffu, in);
-  const int nA = __popc(act);
-  const int share = budget / nA, extra = budget - share * nA;
-  if (!in) prio = 0u;
-  int before = 0;
-  for (int o = 0; o < 32; o++) {
-    const unsigned po = __shfl_sync(0xffffffffu, prio, o);
-    if ((act >> o) & 1u) before += (po > prio || (po == prio && o < lane)) ? 1 : 0;
-  }
-  spc = in ? share + max(0, min(maxExtra, extra - before * maxExtra)) : 0;
-  base = spc;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, base, o);
-    if (lane >= o) base += y;
-  }
-  base -= spc;
-  jmax = share + min(maxExtra, extra);
-}
-
 // c.(p2 - p1) against |p2 - p1| |c|: |cos(f, c)| > 0.95 as lmder2 tests it
 // (Superquadrics_Ig2.cpp:1144-1154).  |c| is 1 to a few ulps, so that outside a band of 1e-9 around
 // the threshold the test needs neither |c| nor the division.
@@ -1735,20 +1665,7 @@ __device__ __forceinline__ int insideFast(const SqShape& s, D3 p) {
 #include "sq_wave_search.cuh"
 #include "sq_warp_search.cuh"
 
-// ---------------------------------------------------------------------------
-// Pass 2 of the Hertz-Mindlin model: the Nelder-Mead searches of
-// Ig2_Superquadrics_Superquadrics_SuperquadricsGeom2::go (Superquadrics_Ig2.cpp:2391-2430),
-// one per lane, each round one Disfun evaluation per lane (NMState asks for one point per
-// step), a lane that finishes a contact taking the next one from the queue.  The search
-// starts at the stored contactAngle with the simplex size 0.1 rad for a new geometry and
-// 0.001 rad for an existing one.
-struct NMLane {
-  int e;
-  bool isNew;
-  NMState M;
-  D3 P1, P2;   // support points of the last evaluation (the reference keeps those)
-  unsigned rounds;
-};
+#include "sq_nm_search.cuh"
 
 // End of Ig2_Superquadrics_Superquadrics_SuperquadricsGeom2::go after a search that found the
 // particles apart (Superquadrics_Ig2.cpp:2392-2397): contactAngle = the returned vertex, no
@@ -1773,19 +1690,22 @@ __device__ void nmFinishApart(const Dev& d, int e, double r0, double r1, int nfu
 // (Superquadrics_Ig2.cpp:2398-2516): normal and depth from the last evaluation's support
 // points, principal curvatures of both surfaces at the returned direction, the contact
 // ellipse; then Ip2 + Law2.  One thread per contact.  The searches leave their results in the
-// merge buffer of the collider (free until the next collider pass): owner = entry,
-// flags = evaluations, angle = returned vertex, depth = distance, p1/p2 = support points.
-__global__ void __launch_bounds__(128) k_contacts_nm_finish(Dev d) {
+// merge buffer of the collider (free until the next collider pass): owner = entry, cd = evaluations
+// and whether it ended touching, angle = returned vertex, depth = distance, p1/p2 = support points.
+// What bounds it: 36 pow and some 9,900 FP64 instructions a contact, in one warp per scheduler (17,000
+// contacts: 0.32 ms).  (Finishing the long searches where they end, beside the rounds, gained nothing:
+// 11.2 ms for five steps instead of 11.0; the pipes are busy.)
+__global__ void __launch_bounds__(128) k_nm_finish(Dev d) {
   const SceneState& S = *d.S;
-  if (S.skip) return;
-  const int n = S.nmFin;
+  const int n = d.Q->nF;
   Counters cnt = {0, 0, 0, 0, 0};
   for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    if (i < n) {
+    if (i0 + (int)threadIdx.x < n) {
+      const int i = d.waveF[i0 + threadIdx.x];
       const int e = d.B.owner[i];
-      const int nfunc = (int)d.B.flags[i];
+      const int nfunc = d.B.cd[i].x;
       const double2 r = d.B.angle[i];
+      if (!d.B.cd[i].y) { nmFinishApart(d, e, r.x, r.y, nfunc, cnt); continue; }
       const double dist = d.B.depth[i];
       const D3 P1 = xyz(d.B.p1[i]), P2 = xyz(d.B.p2[i]);
       const unsigned fl = d.A.flags[e];
@@ -1837,134 +1757,6 @@ __global__ void __launch_bounds__(128) k_contacts_nm_finish(Dev d) {
     }
   }
   flushCounters(d, cnt);
-}
-
-__global__ void __launch_bounds__(LM_BS) k_contacts_nm(Dev d) {
-  __shared__ SqShape shA[LM_BS], shB[LM_BS];
-  __shared__ Rot shG[LM_BS];
-  __shared__ double2 slotQ[LM_BS];
-  __shared__ int slotOwner[LM_BS];
-  const SceneState& S = *d.S;
-  const int nFront = S.lmCount, count = S.lmCount + S.nmShort;
-  const int lane = threadIdx.x & 31;
-  const int wbase = threadIdx.x & ~31;
-  const bool spread = d.prm->lmSpread != 0;
-  Counters cnt = {0, 0, 0, 0, 0};
-  unsigned long long ev64 = 0;
-  unsigned roundsMax = 0;
-  NMLane L;
-  bool active = false, exhausted = false;
-  while (true) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !active && !exhausted);
-    if (idle) {
-      const int leader = __ffs(idle) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(&d.S->lmHead, __popc(idle));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!active && !exhausted) {
-        const int idx = base + __popc(idle & ((1u << lane) - 1));
-        if (idx < count) {
-          SqShape& A = shA[threadIdx.x];
-          SqShape& B = shB[threadIdx.x];
-          L.e = idx < nFront ? d.lmQueue[idx] : d.lmQueue[d.qCap - 1 - (idx - nFront)];
-          const unsigned fl = d.A.flags[L.e];
-          int id1, id2;
-          entryIds(d, L.e, fl, id1, id2);
-          const double4 o1 = d.ori[id1], o2 = d.ori[id2];
-          const double4 a1 = d.shpA[id1], a2 = d.shpA[id2], e1 = d.shpB[id1], e2 = d.shpB[id2];
-          shapeInit(A, a1.x, a1.y, a1.z, e1.x, e1.y, a1.w); A.R = quatToRot(o1.x, o1.y, o1.z, o1.w); A.pos = xyz(d.pos[id1]);
-          shapeInit(B, a2.x, a2.y, a2.z, e2.x, e2.y, a2.w); B.R = quatToRot(o2.x, o2.y, o2.z, o2.w); B.pos = xyz(d.pos[id2]);
-          shG[threadIdx.x] = cRotationMat(A.pos, B.pos);
-          L.isNew = !(fl & F_GEOM);
-          const double2 an = L.isNew ? make_double2(0, 0) : d.A.angle[L.e];
-          nmStart(L.M, an.x, an.y, L.isNew ? 0.1 : 0.001);
-          L.P1 = d3(0, 0, 0); L.P2 = d3(0, 0, 0); L.rounds = 0;
-          active = true;
-        } else exhausted = true;
-      }
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (!act) break;
-    // One point per search while the queue has work.  Once it is drained the warp's slots
-    // (five groups of six lanes, coopEval, while at most COOP_POINTS searches run, else 32
-    // lanes) are shared out, and each search fills its share with the points nmPlan says it
-    // may ask for next.
-    const int nA = __popc(act);
-    const bool drained = spread && __any_sync(0xffffffffu, exhausted);
-    const bool coop = drained && nA <= COOP_POINTS;
-    int spc, base, jmax;
-    allocSlots(active, L.rounds, drained ? (coop ? COOP_POINTS : 32) : nA, 1, spc, base, jmax);
-    slotOwner[threadIdx.x] = -1;
-    __syncwarp();
-    if (active) {
-      const int n = nmPlan(L.M, &slotQ[wbase + base], spc);
-      for (int i = 0; i < n; i++) slotOwner[wbase + base + i] = lane;
-    }
-    __syncwarp();
-    D3 P1 = d3(0, 0, 0), P2 = d3(0, 0, 0);
-    bool flag = false;
-    double f = 0;
-    if (coop) {
-      const int graw = lane / COOP_LANES;
-      const int grp = graw < COOP_POINTS ? graw : 0;
-      const int sub = graw < COOP_POINTS ? lane - grp * COOP_LANES : lane - COOP_POINTS * COOP_LANES;
-      const int o = slotOwner[wbase + grp];
-      const bool has = graw < COOP_POINTS && o >= 0;
-      const int slot = has ? grp : 0;
-      const int src = wbase + slotOwner[wbase + slot];
-      const double2 q = slotQ[wbase + slot];
-      coopEval(shA[src], shB[src], q.x, q.y, grp * COOP_LANES, sub, P1, P2, flag, &shG[src], &f);
-      if (has && sub == 0) ev64++;
-    } else {
-      const int own = slotOwner[threadIdx.x];
-      if (own >= 0) {
-        const double2 q = slotQ[threadIdx.x];
-        f = disfunNM(shA[wbase + own], shB[wbase + own], shG[wbase + own], q.x, q.y, P1, P2, flag);
-        ev64++;
-      }
-    }
-    if (active) L.rounds++;
-    for (int j = 0; j < jmax; j++) {
-      const int si = base + j;
-      const bool mine = j < spc;
-      const int src = mine ? (coop ? si * COOP_LANES : si) : lane;
-      const double x1 = __shfl_sync(0xffffffffu, P1.x, src), y1 = __shfl_sync(0xffffffffu, P1.y, src),
-                   z1 = __shfl_sync(0xffffffffu, P1.z, src);
-      const double x2 = __shfl_sync(0xffffffffu, P2.x, src), y2 = __shfl_sync(0xffffffffu, P2.y, src),
-                   z2 = __shfl_sync(0xffffffffu, P2.z, src);
-      const double fs = __shfl_sync(0xffffffffu, f, src);
-      const bool apart = __shfl_sync(0xffffffffu, (int)flag, src) != 0;
-      bool done = false;
-      if (mine && active && slotOwner[wbase + si] == lane && sameBits(slotQ[wbase + si], L.M.q0, L.M.q1)) {
-        L.P1 = d3(x1, y1, z1); L.P2 = d3(x2, y2, z2);
-        done = !nmConsume(L.M, fs, apart);
-      }
-      // searches that ended touching go to the finish pass (warp-aggregated append)
-      const bool fin = done && L.M.touching;
-      const unsigned m = __ballot_sync(0xffffffffu, fin);
-      if (m) {
-        const int leader = __ffs(m) - 1;
-        int b0 = 0;
-        if (lane == leader) b0 = atomicAdd(&d.S->nmFin, __popc(m));
-        b0 = __shfl_sync(0xffffffffu, b0, leader);
-        if (fin) {
-          const int i = b0 + __popc(m & ((1u << lane) - 1));
-          d.B.owner[i] = L.e; d.B.flags[i] = (unsigned)L.M.nfunc;
-          d.B.angle[i] = make_double2(L.M.r0, L.M.r1); d.B.depth[i] = L.M.dist;
-          d.B.p1[i] = dd4(L.P1, 0); d.B.p2[i] = dd4(L.P2, 0);
-        }
-      }
-      if (done && !L.M.touching) nmFinishApart(d, L.e, L.M.r0, L.M.r1, L.M.nfunc, cnt);
-      if (done) { active = false; roundsMax = max(roundsMax, L.rounds); }
-    }
-    __syncwarp();
-  }
-  flushCounters(d, cnt);
-  for (int o = 16; o > 0; o >>= 1) {
-    ev64 += __shfl_down_sync(0xffffffffu, ev64, o);
-    roundsMax = max(roundsMax, __shfl_down_sync(0xffffffffu, roundsMax, o));
-  }
-  if (lane == 0) { atomicAdd(&d.S->err[E_EVAL64], ev64); atomicMax(&d.S->err[E_ROUNDS_MAX], (unsigned long long)roundsMax); }
 }
 
 // ---------------------------------------------------------------------------
@@ -2693,7 +2485,7 @@ __global__ void __launch_bounds__(256) k_kinematics(Dev d, int pack) {
 
 __global__ void k_reset_queue(Dev d) {
   d.S->lmCount = 0; d.S->lmHead = 0; d.S->fbCount = 0; d.S->fbHead = 0; d.S->vlCount = 0; d.S->vlHead = 0;
-  d.S->nmFin = 0; d.S->nmShort = 0; *d.Q = QueueState();
+  d.S->nmShort = 0; *d.Q = QueueState();
 }
 
 }  // namespace sqdem
@@ -2797,7 +2589,7 @@ static int maxSearchBlocksPerSM(const sqdem_ctx* c) {
 static int searchBlocksPerSM(const sqdem_ctx* c) {
   const int mx = maxSearchBlocksPerSM(c);
   if (c->shapeSearch > 0) return std::min(c->shapeSearch, mx);
-  return c->contactModel != SQDEM_CONTACT_HERTZ_MINDLIN && c->precision == SQDEM_FP64 ? std::min(WAVE_BLOCKS_PER_SM, mx) : mx;
+  return c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN || c->precision == SQDEM_FP64 ? std::min(WAVE_BLOCKS_PER_SM, mx) : mx;
 }
 static const int PASS1_BLOCKS_PER_SM = 16;   // grid-stride blocks of pass 1 per SM (default)
 
@@ -2827,6 +2619,15 @@ static int ffRounds(const sqdem_ctx* c, const Dev& d) {
   return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
 }
 
+// Hertz-Mindlin model: rounds before the searches left get a warp each; none up to NM_WARP_MAX particles
+// (a packed lattice of 977: 0.86 ms a step, 1.06 in rounds; of 7,001: 1.28 and 1.40; of 20,000: 2.74
+// without rounds, 2.35 with four, 2.10 with six, 2.15 with ten).
+static const int NM_WARP_MAX = 10000;
+static int nmRounds(const sqdem_ctx* c, const Dev& d) {
+  const int n = std::max(c->load, d.NP);
+  return n <= NM_WARP_MAX ? 0 : 6;
+}
+
 // shared memory of a k_search_warp<W> block: the trial points of its searches, two rounds of them
 static size_t wsShared(int W, int threads) { return sizeof(WSlot) * 2 * WS_POINTS * W * (threads / (32 * W)); }
 
@@ -2845,9 +2646,22 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
   }
   if (c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) {
     k_contacts_pre<true><<<pre, 128, 0, s>>>(d);
-    k_contacts_nm<<<grid, LM_BS, 0, s>>>(d);
-    k_contacts_nm_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-    c->launches += 3;
+    const int ws = std::min(4 * c->numSMs, d.Pcap);
+    const int rounds = nmRounds(c, d);
+    cudaEventRecord(c->fork, s);
+    cudaStreamWaitEvent(c->stream2, c->fork, 0);
+    k_nm_warp<2><<<std::min(2 * c->numSMs, d.Pcap), 64, 0, c->stream2>>>(d, WS_LONG, 0);
+    cudaEventRecord(c->join, c->stream2);
+    if (rounds == 0) k_nm_warp<1><<<ws, 32, 0, s>>>(d, WS_MAIN, 0);
+    else {
+      const int blocks = std::min(c->numSMs * searchBlocksPerSM(c), nblk(d.Pcap, LM_BS / 8));
+      k_nm_round<true><<<blocks, LM_BS, 0, s>>>(d, 0);
+      for (int r = 1; r < rounds; r++) k_nm_round<false><<<blocks, LM_BS, 0, s>>>(d, r);
+      k_nm_warp<1><<<ws, 32, 0, s>>>(d, WS_TAIL, rounds);
+    }
+    cudaStreamWaitEvent(s, c->join, 0);
+    k_nm_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
+    c->launches += 4 + rounds;
   } else {
     k_contacts_pre<false><<<pre, 128, 0, s>>>(d);
     // four warps per SM for the warp searches: one per scheduler, whose FP64 pipe serves its chain
@@ -3016,8 +2830,9 @@ static sqdem_status uploadParams(sqdem_ctx* c) {
   P.periodicFix = c->periodicFix;
   // (from 64 in the mixed form was measured no faster: the double-float kernel then deferred more
   // searches past 50 iterations, run again in FP64)
-  P.vlongBucket = c->precision == SQDEM_MIXED ? LONG_BUCKET_MIXED : c->inBatch ? LONG_BUCKET_BATCH : LONG_BUCKET_FP64;
-  P.vlongFront = c->precision == SQDEM_MIXED ? LONG_FRONT_MIXED : LONG_FRONT_FP64;
+  const bool nm = c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN;
+  P.vlongBucket = nm ? LONG_BUCKET_NM : c->precision == SQDEM_MIXED ? LONG_BUCKET_MIXED : c->inBatch ? LONG_BUCKET_BATCH : LONG_BUCKET_FP64;
+  P.vlongFront = nm ? LONG_FRONT_NM : c->precision == SQDEM_MIXED ? LONG_FRONT_MIXED : LONG_FRONT_FP64;
   P.h0 = hostH0(c);
   CK(cudaMemcpyAsync(c->d.prm, &P, sizeof(P), cudaMemcpyHostToDevice, c->stream));
   return SQDEM_OK;
@@ -3089,7 +2904,7 @@ sqdem_status sqdem_create(sqdem_ctx** out, const sqdem_config* cfg) {
     c->lmBlocksPerSM = nb > 0 ? nb : 1;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ff_trial<false>, LM_BS, 0));
     c->lmBlocksPerSMmixed = nb > 0 ? nb : 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_contacts_nm, LM_BS, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_nm_round<false>, LM_BS, 0));
     c->nmBlocksPerSM = nb > 0 ? nb : 1;
   }
   for (int i = 0; i < 7; i++) CK(cudaEventCreate(&c->ev[i]));

@@ -16,7 +16,7 @@ import pytest
 
 import oracle as O
 from oracle import OracleScene
-from sudodem_gb300 import Engine, assemblies
+from sudodem_gb300 import Batch, Engine, assemblies
 
 CURV = slice(47, 51)
 ELL = slice(51, 55)
@@ -283,3 +283,29 @@ def test_gpu_precision_flag_does_not_change_the_hm_search(gpu):
     a.sync(); b.sync()
     assert np.array_equal(a.body_state(), b.body_state())
     assert np.array_equal(a.interactions(True), b.interactions(True))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1, 33, 250, 9800), (2, 10200)])
+def test_nelder_mead_schedules_agree(gpu, sizes):
+    """Scenes of up to 10,000 particles search one contact per warp, larger ones and the scenes of a
+    larger batch in rounds, in both forms with a warp pair per search that ran long at the last step;
+    without spare-lane evaluation one point per search and round.  The same operations per contact,
+    so the same bits."""
+    ss = [assemblies.hertz_mindlin(assemblies.cubic_specimen(n, seed=41 + i, eps_range=(0.5, 1.5), spacing=2.0e-3, wall_gap=0.0),
+                                   G=1e6, nu=0.3) for i, n in enumerate(sizes)]
+    b = Batch(len(ss))
+    b.load(ss)
+    b.step(6)
+    b.sync()
+    for i, spec in enumerate(ss):
+        for spread in (True, False):
+            e = engine_for(spec)
+            e.set_lm_spread(spread)
+            e.step(6)
+            rep = e.sync()
+            assert np.array_equal(b.scenes[i].interactions(True), e.interactions(True)), (i, spread)
+            assert np.array_equal(b.scenes[i].body_state(), e.body_state()), (i, spread)
+            e.close()
+    assert rep["lm_calls"] > 0 and rep["long_queue"] > 0
+    b.close()
