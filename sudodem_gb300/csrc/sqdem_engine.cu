@@ -12,16 +12,19 @@
 //     k_candidates    overlap tests against the 27 neighbour cells and the walls, then a
 //                     sorted per-body candidate row merged with the body's previous row
 //                     (conditionalyEraseNonReal + insert, InteractionContainer.cpp:13-39)
-//     k_merge         writes the new contact table (rows ordered by partner id), keeping
+//     k_merge / k_merge_entries   the new contact table (rows ordered by partner id), keeping
 //                     contact history for pairs that survive
 //     k_pcount / k_pscatter / k_psort / k_wall_*   incidence lists for the force gather
-//   k_contacts      InteractionLoop body: Ig2_* + Ip2_* + SuperquadricsLaw
+//     (small scenes: the gate and all of these in k_collider_cluster)
+//   contact stage   InteractionLoop body: Ig2_* + Ip2_* + SuperquadricsLaw
 //                   (InteractionLoop.cpp:56-141; Superquadrics_Ig2.cpp:1880-2317,2522-2611;
 //                   Superquadrics.cpp:1030-1116,1181-1363)
+//     k_contacts_walls, k_contacts_pre   walls; pairs that need no search, the rest queued
+//     k_search_warp, k_wave_*, k_ff_*, k_nm_*   the searches (launchContactStage)
 //   k_wall_forces   ForceContainer sum for walls (ForceContainer.hpp:134-162)
 //   k_integrate     ForceContainer sum for particles + NewtonIntegrator::action
 //                   (NewtonIntegrator.cpp:99-304)
-//   k_end           Scene::moveToNextTimeStep epilogue (Scene.cpp:114-115)
+//                   and, in its last block, Scene::moveToNextTimeStep's epilogue (Scene.cpp:114-115)
 //
 // Collider kernels return at once when k_gate decided the collider does not run this step.
 // Compiled with --fmad=false: FP64 results keep the reference's rounding sequence up to the
@@ -185,6 +188,7 @@ struct Dev {
   int* bodyCell; int* cellCount; int* cellStart; int* cellFill; int* cellBodies;
   float4* cellBox;   // per cell slot: bound centre (xyz) and, in the next entry, half extents (xyz)
   int* scanTmp;
+  int* ccTmp;   // k_collider_cluster: one sum per block
   unsigned long long* bbPart;
   // boundary controller: per-wall kn sums of real contacts, per-block partial sums
   double* wallKn; double* svPart; int svBlocks;
@@ -315,7 +319,7 @@ __global__ void k_scan_apply(const int* __restrict__ in, int n, const int* __res
 // ---------------------------------------------------------------------------
 // Collider gate: InsertionSortCollider::isActivated (InsertionSortCollider.cpp:177-189)
 // plus the start of action() (:205-252) and the NewtonIntegrator maxVelocitySq readout.
-__global__ void k_gate(Dev d) {
+__device__ __forceinline__ void gate(const Dev& d) {
   SceneState& S = *d.S;
   S.skip = (S.haltAt >= 0 && S.iter >= S.haltAt) ? 1 : 0;
   if (S.skip) { S.runCollider = 0; S.lmCount = 0; S.lmHead = 0; S.fbCount = 0; S.fbHead = 0; S.vlCount = 0; S.vlHead = 0; S.nmShort = 0; *d.Q = QueueState(); return; }
@@ -359,16 +363,20 @@ __global__ void k_gate(Dev d) {
     for (int k = 0; k < 3; k++) { S.bbLo[k] = ~0ull; S.bbHi[k] = 0ull; }
   }
 }
+__global__ void k_gate(Dev d) { gate(d); }
+
+// The collider's passes are device functions over threads t0, t0 + nt, ...: a kernel each, or all
+// of them in one (k_collider_cluster).
+#define GRID_T0 (blockIdx.x * blockDim.x + threadIdx.x)
+#define GRID_NT (gridDim.x * blockDim.x)
 
 // BoundDispatcher::processBody (Dispatching.cpp:30-62), Bo1_Superquadrics_Aabb::go
 // (Superquadrics.cpp:639-686), Bo1_Wall_Aabb::go (Wall.cpp:13-21).
-__global__ void k_bounds(Dev d) {
+__device__ __forceinline__ void boundsPass(const Dev& d, int t0, int nt) {
   const SceneState& S = *d.S;
-  if (!S.runCollider) return;
   const Params& P = *d.prm;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
   double cmin[3] = {INFINITY, INFINITY, INFINITY}, cmax[3] = {-INFINITY, -INFINITY, -INFINITY};
-  if (b < d.N) {
+  for (int b = t0; b < d.N; b += nt) {
     const double sweepDist = S.verletDistCur;
     double4 pos = d.pos[b];
     double4 mn = d.bmin[b], mx = d.bmax[b], rf = d.ref[b];
@@ -408,7 +416,8 @@ __global__ void k_bounds(Dev d) {
     d.ref[b] = make_double4(pos.x, pos.y, pos.z, 1.0);
     if (inf.x == KIND_SQ) {
       D3 c = 0.5 * (lo + hi);
-      cmin[0] = cmax[0] = c.x; cmin[1] = cmax[1] = c.y; cmin[2] = cmax[2] = c.z;
+      cmin[0] = fmin(cmin[0], c.x); cmin[1] = fmin(cmin[1], c.y); cmin[2] = fmin(cmin[2], c.z);
+      cmax[0] = fmax(cmax[0], c.x); cmax[1] = fmax(cmax[1], c.y); cmax[2] = fmax(cmax[2], c.z);
     }
   }
   // block bbox of particle bound centres -> global atomics on ordered encodings
@@ -425,10 +434,10 @@ __global__ void k_bounds(Dev d) {
     }
   }
 }
+__global__ void k_bounds(Dev d) { if (d.S->runCollider) boundsPass(d, GRID_T0, GRID_NT); }
 
-__global__ void k_grid_setup(Dev d) {
+__device__ __forceinline__ void gridSetup(const Dev& d) {
   SceneState& S = *d.S;
-  if (!S.runCollider) return;
   const Params& P = *d.prm;
   // post-dispatch stride bookkeeping (InsertionSortCollider.cpp:263-284)
   if (S.verletDistCur > 0) S.newtonFound = 1;
@@ -476,13 +485,12 @@ __global__ void k_grid_setup(Dev d) {
   S.h = h;
   S.nCells = (int)cells;
 }
+__global__ void k_grid_setup(Dev d) { if (d.S->runCollider) gridSetup(d); }
 
-__global__ void k_zero_cells(Dev d) {
-  if (!d.S->runCollider) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= d.Gmax; i += gridDim.x * blockDim.x) {
-    d.cellCount[i] = 0; d.cellFill[i] = 0;
-  }
+__device__ __forceinline__ void zeroCells(const Dev& d, int t0, int nt) {
+  for (int i = t0; i <= d.Gmax; i += nt) { d.cellCount[i] = 0; d.cellFill[i] = 0; }
 }
+__global__ void k_zero_cells(Dev d) { if (d.S->runCollider) zeroCells(d, GRID_T0, GRID_NT); }
 
 // clamped cell coordinate; NaN maps to 0 so that no index leaves [0, dim)
 __device__ __forceinline__ int cellCoord(double c, double org, double h, int dim) {
@@ -513,11 +521,8 @@ __device__ __forceinline__ void bodyCellCoords(const SceneState& S, double4 mn, 
   }
 }
 
-__global__ void k_cell_count(Dev d) {
+__device__ __forceinline__ void cellCountOf(const Dev& d, int b) {
   const SceneState& S = *d.S;
-  if (!S.runCollider) return;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.N) return;
   if (d.info[b].x != KIND_SQ) { d.bodyCell[b] = -1; return; }
   double4 mn = d.bmin[b], mx = d.bmax[b];
   int cx, cy, cz;
@@ -526,10 +531,8 @@ __global__ void k_cell_count(Dev d) {
   d.bodyCell[b] = cell;
   atomicAdd(&d.cellCount[cell], 1);
 }
-__global__ void k_cell_scatter(Dev d) {
-  if (!d.S->runCollider) return;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.N) return;
+__global__ void k_cell_count(Dev d) { if (d.S->runCollider && GRID_T0 < d.N) cellCountOf(d, GRID_T0); }
+__device__ __forceinline__ void cellScatterOf(const Dev& d, int b) {
   int cell = d.bodyCell[b];
   if (cell < 0) return;
   int slot = d.cellStart[cell] + atomicAdd(&d.cellFill[cell], 1);
@@ -538,6 +541,7 @@ __global__ void k_cell_scatter(Dev d) {
   d.cellBox[2 * slot] = make_float4((float)(0.5 * (mn.x + mx.x)), (float)(0.5 * (mn.y + mx.y)), (float)(0.5 * (mn.z + mx.z)), 0.f);
   d.cellBox[2 * slot + 1] = make_float4((float)(0.5 * (mx.x - mn.x)), (float)(0.5 * (mx.y - mn.y)), (float)(0.5 * (mx.z - mn.z)), 0.f);
 }
+__global__ void k_cell_scatter(Dev d) { if (d.S->runCollider && GRID_T0 < d.N) cellScatterOf(d, GRID_T0); }
 
 // FP32 pre-filter of the candidate search: true when the two bounds cannot overlap, in any
 // periodic image (minimum-image distance of the centres above the summed half extents on
@@ -654,11 +658,8 @@ static const int UNDECIDED = 0x40000000;   // candidate tag: overlap left to the
 // Threads take the particles in cell order (cellBodies), so that a warp scans neighbouring
 // cells and its loads of cellBodies/cellBox overlap; bodies outside the grid (walls) get an
 // empty row from the thread of their own index.
-__global__ void k_candidates(Dev d) {
+__device__ __forceinline__ void candidatesOf(const Dev& d, int t) {
   const SceneState& S = *d.S;
-  if (!S.runCollider) return;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.N) return;
   if (d.bodyCell[t] < 0) { d.rowCount[t] = 0; d.candCount[t] = 0; }
   if (t >= d.cellStart[S.nCells]) return;
   const int i = d.cellBodies[t];
@@ -755,14 +756,15 @@ __global__ void k_candidates(Dev d) {
   d.candCount[i] = m;
   d.rowCount[i] = cnt;
 }
+__global__ void k_candidates(Dev d) { if (d.S->runCollider && GRID_T0 < d.N) candidatesOf(d, GRID_T0); }
 
-__global__ void k_check_capacity(Dev d) {
+__device__ __forceinline__ void checkCapacity(const Dev& d) {
   SceneState& S = *d.S;
-  if (!S.runCollider) return;
   int Pn = d.rowStartNew[d.N];
   S.Pnew = Pn;
   if (Pn > d.Pcap) { S.overflowRun = 1; atomicAdd(&S.err[E_OVERFLOW], 1ull); }
 }
+__global__ void k_check_capacity(Dev d) { if (d.S->runCollider) checkCapacity(d); }
 
 __device__ __forceinline__ void copyEntry(const Table& s, int a, const Table& t, int b, bool full) {
   t.owner[b] = s.owner[a]; t.partner[b] = s.partner[a]; t.flags[b] = s.flags[a];
@@ -785,55 +787,69 @@ __device__ __forceinline__ void initEntry(const Table& t, int b, int owner, int 
   }
 }
 
-__global__ void k_merge(Dev d) {
-  const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.N) return;
+__device__ __forceinline__ bool tableChanges(const Dev& d) { return d.S->runCollider && !d.S->overflowRun; }
+// The new rows in two passes: where each entry comes from, one thread per particle (waveT0: the old
+// entry, or -1 for a new pair, whose candidate word is left in B.partner), then the entries
+// themselves, one thread each (a thread per particle that copied its row's 13 fields entry by entry
+// took 75 us at 2,197 particles; these take 8 and 11).
+__device__ __forceinline__ void mergeOf(const Dev& d, int i) {
   if (d.info[i].x != KIND_SQ) return;
-  const bool full = d.prm->recordFull != 0;
   const int* cand = d.cand + (size_t)i * d.MAXC;
   const int n = d.candCount[i];
-  const int os = d.rowStart[i], oe = d.rowStart[i + 1];
+  const int oe = d.rowStart[i + 1];
   int out = d.rowStartNew[i];
-  int o = os, c = 0;
+  int o = d.rowStart[i], c = 0;
   while (o < oe || c < n) {
     int po = o < oe ? d.A.partner[o] : 0x7fffffff;
     int raw = c < n ? cand[c] : 0x7fffffff;
     int pc = raw & 0x7fffffff;
-    if (po == pc) { copyEntry(d.A, o, d.B, out++, full); o++; c++; }
+    if (po == pc) { d.waveT0[out++] = o; o++; c++; }
     else if (po < pc) {
-      if ((d.A.flags[o] & (F_GEOM | F_PHYS)) == (F_GEOM | F_PHYS)) copyEntry(d.A, o, d.B, out++, full);
+      if ((d.A.flags[o] & (F_GEOM | F_PHYS)) == (F_GEOM | F_PHYS)) d.waveT0[out++] = o;
       o++;
     } else {
-      const bool ownerIsId1 = (raw & 0x80000000) != 0;
-      initEntry(d.B, out, i, pc, ownerIsId1, full);
-      if (S.periodic) {
-        const int a = ownerIsId1 ? i : pc, b = ownerIsId1 ? pc : i;
-        int per[3];
-        overlapPeri(S, d.bmin[a], d.bmax[a], d.bmin[b], d.bmax[b], per);
-        d.B.cd[out] = make_int4(per[0], per[1], per[2], 0);
-      }
+      d.waveT0[out] = -1;
+      d.B.owner[out] = i; d.B.partner[out] = raw;
       out++; c++;
     }
   }
 }
-
-__global__ void k_copy_back(Dev d) {
+__global__ void k_merge(Dev d) { if (tableChanges(d) && GRID_T0 < d.N) mergeOf(d, GRID_T0); }
+__device__ __forceinline__ void mergeEntries(const Dev& d, int t0, int nt) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
   const bool full = d.prm->recordFull != 0;
   const int Pn = S.Pnew;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < Pn; e += gridDim.x * blockDim.x) copyEntry(d.B, e, d.A, e, full);
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= d.N; b += gridDim.x * blockDim.x) {
+  for (int e = t0; e < Pn; e += nt) {
+    const int o = d.waveT0[e];
+    if (o >= 0) { copyEntry(d.A, o, d.B, e, full); continue; }
+    const int i = d.B.owner[e], raw = d.B.partner[e];
+    const int pc = raw & 0x7fffffff;
+    const bool ownerIsId1 = (raw & 0x80000000) != 0;
+    initEntry(d.B, e, i, pc, ownerIsId1, full);
+    if (S.periodic) {
+      const int a = ownerIsId1 ? i : pc, b = ownerIsId1 ? pc : i;
+      int per[3];
+      overlapPeri(S, d.bmin[a], d.bmax[a], d.bmin[b], d.bmax[b], per);
+      d.B.cd[e] = make_int4(per[0], per[1], per[2], 0);
+    }
+  }
+}
+__global__ void k_merge_entries(Dev d) { if (tableChanges(d)) mergeEntries(d, GRID_T0, GRID_NT); }
+
+__device__ __forceinline__ void copyBack(const Dev& d, int t0, int nt) {
+  const SceneState& S = *d.S;
+  const bool full = d.prm->recordFull != 0;
+  const int Pn = S.Pnew;
+  for (int e = t0; e < Pn; e += nt) copyEntry(d.B, e, d.A, e, full);
+  for (int b = t0; b <= d.N; b += nt) {
     d.rowStart[b] = d.rowStartNew[b];
     if (b < d.N) { d.pCount[b] = 0; d.pFill[b] = 0; }
   }
 }
+__global__ void k_copy_back(Dev d) { if (tableChanges(d)) copyBack(d, GRID_T0, GRID_NT); }
 
-__global__ void k_commit(Dev d) {
+__device__ __forceinline__ void commit(const Dev& d) {
   SceneState& S = *d.S;
-  if (!S.runCollider) return;
   if (!S.overflowRun) S.P = S.Pnew;
   S.bbInit = 1;
   for (int k = 0; k < 3; k++) S.prevRunCellSize[k] = S.cellSize[k];
@@ -849,42 +865,43 @@ __global__ void k_commit(Dev d) {
     }
   S.nWW = n;
 }
+__global__ void k_commit(Dev d) { if (d.S->runCollider) commit(d); }
 
 // incidence lists: entries in which a particle is the partner (not the row owner)
-__global__ void k_pcount(Dev d) {
+__device__ __forceinline__ void partnerCount(const Dev& d, int t0, int nt) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < S.P; e += gridDim.x * blockDim.x) {
+  for (int e = t0; e < S.P; e += nt) {
     int p = d.A.partner[e];
     if (d.info[p].x == KIND_SQ) atomicAdd(&d.pCount[p], 1);
   }
 }
-__global__ void k_pscatter(Dev d) {
+__global__ void k_pcount(Dev d) { if (tableChanges(d)) partnerCount(d, GRID_T0, GRID_NT); }
+__device__ __forceinline__ void partnerScatter(const Dev& d, int t0, int nt) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < S.P; e += gridDim.x * blockDim.x) {
+  for (int e = t0; e < S.P; e += nt) {
     int p = d.A.partner[e];
-    if (d.info[p].x == KIND_SQ) d.pList[d.pStart[p] + atomicAdd(&d.pFill[p], 1)] = e;
+    if (d.info[p].x == KIND_SQ) d.waveT0[d.pStart[p] + atomicAdd(&d.pFill[p], 1)] = e;
   }
 }
-// make each partner list ascending in entry index (deterministic summation order)
-__global__ void k_psort(Dev d) {
+__global__ void k_pscatter(Dev d) { if (tableChanges(d)) partnerScatter(d, GRID_T0, GRID_NT); }
+// each partner list ascending in entry index (deterministic summation order): an entry's place is the
+// number of smaller ones in its list (6 us at 2,197 particles; a sort per particle took 32)
+__device__ __forceinline__ void partnerSort(const Dev& d, int t0, int nt) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.N) return;
-  int s = d.pStart[b], e = d.pStart[b + 1];
-  for (int a = s + 1; a < e; a++) {
-    int v = d.pList[a]; int c = a - 1;
-    while (c >= s && d.pList[c] > v) { d.pList[c + 1] = d.pList[c]; c--; }
-    d.pList[c + 1] = v;
+  for (int e = t0; e < S.P; e += nt) {
+    const int p = d.A.partner[e];
+    if (d.info[p].x != KIND_SQ) continue;
+    const int s = d.pStart[p], n = d.pStart[p + 1];
+    int at = s;
+    for (int k = s; k < n; k++) at += d.waveT0[k] < e ? 1 : 0;
+    d.pList[at] = e;
   }
 }
+__global__ void k_psort(Dev d) { if (tableChanges(d)) partnerSort(d, GRID_T0, GRID_NT); }
 // Per-wall lists of table entries in table order (the order the wall force sums follow).
 // The table is cut into WALL_CHUNKS contiguous chunks, one block each: k_wall_count counts
 // each wall's entries per chunk; k_wall_lists places chunk b's entries of wall w after
-// those of the walls before w and of the chunks before b, in table order within the chunk
-// (one block scan per wall and tile).
+// those of the walls before w and of the chunks before b, in table order within the chunk.
 static const int WALL_CHUNKS = 256, MAX_WALLS = 64;   // WALL_CHUNKS: most chunks of a table
 __device__ __forceinline__ int wallSlot(const Dev& d, int p) {
   if (d.info[p].x != KIND_WALL) return -1;
@@ -895,32 +912,30 @@ __device__ __forceinline__ void wallChunk(int P, int chunks, int b, int& lo, int
   const int len = (P + chunks - 1) / chunks;
   lo = min(P, b * len); hi = min(P, lo + len);
 }
-__global__ void k_wall_count(Dev d) {
+__device__ __forceinline__ void wallCount(const Dev& d, int chunk, int chunks) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
   __shared__ int cnt[MAX_WALLS];
   for (int w = threadIdx.x; w < d.W; w += blockDim.x) cnt[w] = 0;
   __syncthreads();
   int lo, hi;
-  wallChunk(S.P, d.wallChunks, blockIdx.x, lo, hi);
+  wallChunk(S.P, chunks, chunk, lo, hi);
   for (int e = lo + threadIdx.x; e < hi; e += blockDim.x) {
     const int w = wallSlot(d, d.A.partner[e]);
     if (w >= 0) atomicAdd(&cnt[w], 1);
   }
   __syncthreads();
-  for (int w = threadIdx.x; w < d.W; w += blockDim.x) d.wBlk[blockIdx.x * d.W + w] = cnt[w];
+  for (int w = threadIdx.x; w < d.W; w += blockDim.x) d.wBlk[chunk * d.W + w] = cnt[w];
 }
-__global__ void k_wall_lists(Dev d) {
+__global__ void k_wall_count(Dev d) { if (tableChanges(d)) wallCount(d, blockIdx.x, d.wallChunks); }
+__device__ __forceinline__ void wallLists(const Dev& d, int chunk, int chunks) {
   const SceneState& S = *d.S;
-  if (!S.runCollider || S.overflowRun) return;
-  __shared__ int sh[32];
   __shared__ int tot[MAX_WALLS], off[MAX_WALLS];
   for (int w = threadIdx.x; w < d.W; w += blockDim.x) {
     int before = 0, all = 0;
-    for (int b = 0; b < d.wallChunks; b++) {
+    for (int b = 0; b < chunks; b++) {
       const int c = d.wBlk[b * d.W + w];
       all += c;
-      if (b < blockIdx.x) before += c;
+      if (b < chunk) before += c;
     }
     tot[w] = all; off[w] = before;
   }
@@ -929,26 +944,104 @@ __global__ void k_wall_lists(Dev d) {
     int start = 0;
     for (int w = 0; w < d.W; w++) {
       off[w] += start;
-      if (blockIdx.x == 0) { d.wCount[w] = tot[w]; d.wCount[d.W + w] = start; }
+      if (chunk == 0) { d.wCount[w] = tot[w]; d.wCount[d.W + w] = start; }
       start += tot[w];
     }
   }
   __syncthreads();
   int lo, hi;
-  wallChunk(S.P, d.wallChunks, blockIdx.x, lo, hi);
+  wallChunk(S.P, chunks, chunk, lo, hi);
+  // a tile's entries of a wall follow those of the warps before, in a warp by lane
+  __shared__ int inWarp[32][MAX_WALLS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
   for (int e0 = lo; e0 < hi; e0 += blockDim.x) {
     const int e = e0 + threadIdx.x;
     const int ws = e < hi ? wallSlot(d, d.A.partner[e]) : -1;
-    for (int w = 0; w < d.W; w++) {
-      const int f = ws == w ? 1 : 0;
-      int tt;
-      const int ex = blockExclusiveScan(f, sh, tt);
-      if (f) d.wList[off[w] + ex] = e;
-      __syncthreads();
-      if (threadIdx.x == 0) off[w] += tt;
-      __syncthreads();
+    for (int w = lane; w < d.W; w += 32) inWarp[wid][w] = 0;
+    const unsigned same = __match_any_sync(0xffffffffu, ws);
+    const int before = __popc(same & ((1u << lane) - 1));
+    __syncwarp();
+    if (ws >= 0 && before == 0) inWarp[wid][ws] = __popc(same);
+    __syncthreads();
+    if (ws >= 0) {
+      int at = off[ws] + before;
+      for (int v = 0; v < wid; v++) at += inWarp[v][ws];
+      d.wList[at] = e;
     }
+    __syncthreads();
+    for (int w = threadIdx.x; w < d.W; w += blockDim.x)
+      for (int v = 0; v < warps; v++) off[w] += inWarp[v][w];
+    __syncthreads();
   }
+}
+__global__ void k_wall_lists(Dev d) { if (tableChanges(d)) wallLists(d, blockIdx.x, d.wallChunks); }
+
+// ---------------------------------------------------------------------------
+// The gate and all of the collider's passes in one launch of one thread-block cluster, for small
+// scenes.  What bounds a small scene's step is its launches: the gate and 22 kernels, 1.2 us each
+// in a graph, which most steps leave at once.  Here they are one launch, with cluster barriers
+// between the passes; eight blocks of 512 threads.  A step of 27 particles between walls takes 127 us
+// instead of 149, of a deposition of 1,000 69 instead of 96, of a servo specimen of 700 (whose collider
+// runs at every step) 807 instead of 838.
+static const int CC_BLOCKS = 8, CC_BS = 512;
+__device__ __forceinline__ void clusterSync() {
+  __threadfence();
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// out[i] = sum(in[0..i)) for i in [0, n]; out[n] = total
+__device__ __forceinline__ void clusterScan(const Dev& d, const int* in, int n, int* out, int* tmp, int rank, int* sh) {
+  const int perBlock = (n + CC_BLOCKS) / CC_BLOCKS, per = (perBlock + CC_BS - 1) / CC_BS;
+  const int end = min(n + 1, (rank + 1) * perBlock);
+  const int lo = min(end, rank * perBlock + (int)threadIdx.x * per), hi = min(end, lo + per);
+  int sum = 0;
+  for (int i = lo; i < hi; i++) sum += i < n ? in[i] : 0;
+  int total;
+  int ex = blockExclusiveScan(sum, sh, total);
+  if (threadIdx.x == 0) tmp[rank] = total;
+  clusterSync();
+  for (int r = 0; r < rank; r++) ex += tmp[r];
+  for (int i = lo; i < hi; i++) { out[i] = ex; ex += i < n ? in[i] : 0; }
+  clusterSync();
+}
+__global__ void __cluster_dims__(CC_BLOCKS, 1, 1) __launch_bounds__(CC_BS) k_collider_cluster(Dev d) {
+  __shared__ int sh[32];
+  const int rank = blockIdx.x, t0 = GRID_T0, nt = CC_BLOCKS * CC_BS;
+  if (t0 == 0) gate(d);
+  clusterSync();
+  if (!d.S->runCollider) return;
+  boundsPass(d, t0, nt);
+  zeroCells(d, t0, nt);
+  clusterSync();
+  if (t0 == 0) gridSetup(d);
+  clusterSync();
+  for (int b = t0; b < d.N; b += nt) cellCountOf(d, b);
+  clusterSync();
+  clusterScan(d, d.cellCount, d.S->nCells, d.cellStart, d.ccTmp, rank, sh);
+  for (int b = t0; b < d.N; b += nt) cellScatterOf(d, b);
+  clusterSync();
+  for (int t = t0; t < d.N; t += nt) candidatesOf(d, t);
+  clusterSync();
+  clusterScan(d, d.rowCount, d.N, d.rowStartNew, d.ccTmp, rank, sh);
+  if (t0 == 0) checkCapacity(d);
+  clusterSync();
+  const bool change = !d.S->overflowRun;
+  if (change) for (int i = t0; i < d.N; i += nt) mergeOf(d, i);
+  clusterSync();
+  if (change) mergeEntries(d, t0, nt);
+  clusterSync();
+  if (change) copyBack(d, t0, nt);
+  if (t0 == 0) commit(d);
+  clusterSync();
+  if (!change) return;
+  partnerCount(d, t0, nt);
+  clusterSync();
+  clusterScan(d, d.pCount, d.N, d.pStart, d.ccTmp, rank, sh);
+  partnerScatter(d, t0, nt);
+  const int chunks = min(CC_BLOCKS, d.wallChunks);
+  if (d.W > 0 && rank < chunks) wallCount(d, rank, chunks);
+  clusterSync();
+  partnerSort(d, t0, nt);
+  if (d.W > 0 && rank < chunks) wallLists(d, rank, chunks);
 }
 
 // ---------------------------------------------------------------------------
@@ -1761,8 +1854,8 @@ __global__ void __launch_bounds__(128) k_nm_finish(Dev d) {
 
 // ---------------------------------------------------------------------------
 // Mixed form of pass 2: the searches of lmder2 (Superquadrics_Ig2.cpp:1057-1354) in
-// double-float arithmetic on the FP32 pipes (sq_ff.cuh), Disfunction included, with the same
-// lockstep lanes, work queue and spare-lane evaluation as the FP64 kernel.  GB300 issues FP64 at
+// double-float arithmetic on the FP32 pipes (sq_ff.cuh), Disfunction included, in rounds over
+// compact lists or a warp per search as the FP64 form (sq_ff_search.cuh).  GB300 issues FP64 at
 // 1/64 of its FP32 rate: a double-float evaluation costs ~1/12 of the FP64 one, and the search's
 // own arithmetic (Jacobian, normal equations, damping, step control) in double-float costs a
 // few percent of its evaluations instead of more than they do.
@@ -2724,12 +2817,25 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
   if (d.W > 0) cudaStreamWaitEvent(s, c->join3, 0);
 }
 
-// The collider pass on c->stream (every kernel tests runCollider).
+// Bodies up to which the gate and the collider pass are one launch of one cluster.  Above, where the
+// collider runs at every step, the eight SMs' FP64 pipes are too few for the candidates' exact tests
+// (servo specimen of 2,197: 1.270 ms a step, 1.257 in kernels; 32 specimens of 300-4,000: 13.1 and 12.8 ms
+// for two steps).
+static const int CLUSTER_COLLIDER_MAX = 1600;
+
+// The gate and the collider pass on c->stream (every kernel tests runCollider).
 static void enqueueCollider(sqdem_ctx* c) {
   Dev& d = c->d;
   cudaStream_t s = c->stream;
   const int* gate = gateRun(c);
   const int N = d.N;
+  if (N <= CLUSTER_COLLIDER_MAX) {
+    k_collider_cluster<<<CC_BLOCKS, CC_BS, 0, s>>>(d);
+    c->launches++;
+    return;
+  }
+  k_gate<<<1, 1, 0, s>>>(d);
+  c->launches++;
   k_bounds<<<nblk(N, 256), 256, 0, s>>>(d);
   k_grid_setup<<<1, 1, 0, s>>>(d);
   k_zero_cells<<<std::min(nblk(d.Gmax + 1, 256), 4096), 256, 0, s>>>(d);
@@ -2743,13 +2849,14 @@ static void enqueueCollider(sqdem_ctx* c) {
   const int tblBlocks = std::min(nblk(d.Pcap, 256), c->numSMs * 8);
   k_check_capacity<<<1, 1, 0, s>>>(d);
   k_merge<<<nblk(N, 128), 128, 0, s>>>(d);
+  k_merge_entries<<<tblBlocks, 256, 0, s>>>(d);
   k_copy_back<<<tblBlocks, 256, 0, s>>>(d);
   k_commit<<<1, 1, 0, s>>>(d);
   k_pcount<<<tblBlocks, 256, 0, s>>>(d);
-  c->launches += 5;
+  c->launches += 6;
   launchScan(c, d.pCount, N, d.pStart, gate);
   k_pscatter<<<tblBlocks, 256, 0, s>>>(d);
-  k_psort<<<nblk(N, 256), 256, 0, s>>>(d);
+  k_psort<<<tblBlocks, 256, 0, s>>>(d);
   c->launches += 2;
   if (d.W > 0) {
     k_wall_count<<<d.wallChunks, 256, 0, s>>>(d);
@@ -2764,9 +2871,7 @@ static void enqueueStep(sqdem_ctx* c, bool timed) {
   cudaStream_t s = c->stream;
   const int N = d.N;
   if (timed) cudaEventRecord(c->ev[0], s);
-  k_gate<<<1, 1, 0, s>>>(d);
-  c->launches++;
-  // the collider pass; its kernels return at once when k_gate decided it does not run (a conditional
+  // the gate and the collider pass; its kernels return at once when k_gate decided it does not run (a conditional
   // graph node around them was measured to cost as much as they do: 0.083 against 0.085 ms a step)
   enqueueCollider(c);
   if (timed) cudaEventRecord(c->ev[1], s);
@@ -3046,7 +3151,7 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* c, int n, const int* kind, const double
   CK(dalloc(c, &d.pCount, n + 1)); CK(dalloc(c, &d.pStart, n + 1)); CK(dalloc(c, &d.pFill, n + 1));
   CK(dalloc(c, &d.pList, d.Pcap));
   CK(dalloc(c, &d.wCount, 2 * std::max(d.W, 1))); CK(dalloc(c, &d.wList, d.Pcap));
-  d.wallChunks = std::max(1, std::min(WALL_CHUNKS, nblk(d.Pcap, 4096)));
+  d.wallChunks = std::max(1, std::min(WALL_CHUNKS, nblk(d.Pcap, 1024)));
   CK(dalloc(c, &d.wBlk, (size_t)d.wallChunks * std::max(d.W, 1)));
   d.svBlocks = std::max(1, std::min(nblk(d.Pcap, 128), c->numSMs * 2));
   CK(dalloc(c, &d.wallKn, std::max(d.W, 1))); CK(dalloc(c, &d.svPart, (size_t)d.svBlocks * SV_PART));
@@ -3060,6 +3165,7 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* c, int n, const int* kind, const double
   CK(dalloc(c, &d.bodyCell, n)); CK(dalloc(c, &d.cellCount, d.Gmax + 1)); CK(dalloc(c, &d.cellStart, d.Gmax + 1));
   CK(dalloc(c, &d.cellFill, d.Gmax + 1)); CK(dalloc(c, &d.cellBodies, n)); CK(dalloc(c, &d.cellBox, 2 * (size_t)n));
   CK(dalloc(c, &d.scanTmp, nblk((long)std::max(std::max(d.Gmax, d.Pcap), d.N) + 2, SCAN_TILE) + 2));
+  CK(dalloc(c, &d.ccTmp, CC_BLOCKS));
   // host-side body arrays
   std::vector<double4> v[5];
   for (int k = 0; k < 5; k++) v[k].resize(n);

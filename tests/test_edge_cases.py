@@ -7,6 +7,7 @@ import pytest
 from oracle import OracleScene
 from sudodem_gb300 import Engine, SqdemError, assemblies
 from sudodem_gb300._native import shape_props
+from test_gpu_parity import canon_pairs
 
 pytestmark = pytest.mark.gpu
 
@@ -105,3 +106,21 @@ def test_bounding_sphere_rejection_near_its_threshold(gpu, size, off):
     recs = eng.interactions(True)
     assert len(recs) == 1
     assert np.all(recs[0, 5:7] == 0) == (gap > rsum)
+
+
+@pytest.mark.parametrize("n,periodic", [(1, False), (1594, False), (1595, False), (1600, True), (1601, True)])
+def test_collider_pass_in_one_launch_and_in_kernels(gpu, n, periodic):
+    """Scenes of up to 1,600 bodies run the collider pass as one thread-block cluster, larger ones as
+    one kernel per pass: either way the pairs and their orientation are the oracle's."""
+    if periodic:
+        spec = assemblies.periodic_cell(n, seed=3, solid_fraction=0.5)
+    else:
+        spec = assemblies.cubic_specimen(n, seed=3, eps_range=(0.6, 1.4), spacing=2.1e-3, wall_gap=0.0)
+    eng, orc = _engine(spec), OracleScene.from_spec(spec)
+    for steps in (1,) if periodic else (1, 4):   # the first pass sorts all bounds, later ones insert
+        eng.step(steps); eng.sync(); orc.step(steps)
+        G, R = eng.interactions(True), orc.interactions()
+        assert canon_pairs(G, spec.kind) == canon_pairs(R, spec.kind)
+        assert canon_pairs(G[G[:, 2] == 1], spec.kind) == canon_pairs(R[R[:, 2] == 1], spec.kind)
+        if steps == 1:   # bounds, reference positions, sweep lengths: bit for bit
+            assert np.array_equal(eng.body_state()[:, 22:33], orc.bodies()[:, 22:33])
