@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
   const int grp = (W == 1 ? 0 : wib * WS_POINTS) + g0 / WS_LANES;
   const int gs = real ? g0 : 30;                    // where the lane's step is computed
   const bool odd = r == 1 || r == 3;
-  const int nLong1 = S.vlCount, nLong = S.vlCount + d.Q->vl2Count;
+  const int nLong1 = S.vlCount, nLong = S.vlCount + min(d.Q->vl2Count, d.prm->vlongMax);
   const int nFront = S.lmCount;
   const int total = mode == WS_LONG       ? nLong
                     : mode == WS_DEFERRED ? S.fbCount

@@ -30,6 +30,7 @@
 // Compiled with --fmad=false: FP64 results keep the reference's rounding sequence up to the
 // last-ulp differences between CUDA's and glibc's pow/atan2/sin/cos.
 #include <cuda_runtime.h>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -73,8 +74,13 @@ static const unsigned LONG_ITERS_BUCKET = 3;   // iterations >= 4
 // rounds (43,011 particles: 6.3 ms a step from 8, 6.6 from 16, 7.1 from 32); in a batch 16, since the
 // other specimens fill the FP64 pipe and a warp per search is three times the work of the rounds
 // (32 specimens of 300-4,000 particles: 13.6 ms for two steps from 16, 14.8 from 8).
+// LONG_MAX_FP64: how many searches of 8-31 iterations take a warp in the FP64 form; the others go to the
+// rounds, which need a third of the FP64 work per evaluation asked for: where there are many, their
+// number bounds the stage and not their length.  200,000 particles, second step after loading (109,000
+// such searches): 43.6 -> 29.1 ms, third to ninth (12,000-13,600): 28 -> 26.4; with 3,000 a settled cell's
+// step went from 19.0 to 19.6, with 6,000 19.1.
 static const int LONG_BUCKET_MIXED = 6, LONG_BUCKET_FP64 = 4, LONG_BUCKET_BATCH = 5;
-static const int LONG_FRONT_MIXED = 7, LONG_FRONT_FP64 = 6;
+static const int LONG_FRONT_MIXED = 7, LONG_FRONT_FP64 = 6, LONG_MAX_FP64 = 6000;
 // Hertz-Mindlin model: 32 and 64 Nelder-Mead evaluations (a packed lattice of 20,000: 2.1 ms a step, 2.27
 // from 16; 19 in 20 of those searches take 32 again at the next step).
 static const int LONG_BUCKET_NM = 6, LONG_FRONT_NM = 7;
@@ -90,6 +96,7 @@ struct Params {
   int periodicFix;    // sqdem_set_periodic_fix: torque arm and relative velocity of image contacts
   int vlongBucket;    // iteration bucket from which a search goes to the long-search queue
   int vlongFront;     // and from which to that queue's front
+  int vlongMax;       // searches that queue's back takes
 };
 
 enum { E_NAN_NORMAL = 0, E_NAN_FORCE, E_LM_CALLS, E_LM_ITERS, E_LM_MAX, E_OVERFLOW, E_COLLIDER_RUNS, E_STEPS, E_EVAL32, E_EVAL64, E_ROUNDS_MAX,
@@ -1524,12 +1531,17 @@ __device__ __forceinline__ bool boundsApart(const Dev& d, const SceneState& S, i
   return true;
 }
 
-// Queues a search that ran long at the last step for a warp of its own; false: it did not.
+// Queues a search that ran long at the last step for a warp of its own; false: it did not, or the
+// queue's back is full.
 __device__ __forceinline__ bool longSearch(const Dev& d, int e, unsigned fl) {
   const int bucket = (int)((fl & F_ITERS_MASK) >> F_ITERS_SHIFT);
   if (bucket < d.prm->vlongBucket) return false;
   if (bucket >= d.prm->vlongFront) d.fbQueue[atomicAdd(&d.S->vlCount, 1)] = e;
-  else d.fbQueue[d.Pcap - 1 - atomicAdd(&d.Q->vl2Count, 1)] = e;
+  else {
+    const int i = atomicAdd(&d.Q->vl2Count, 1);
+    if (i >= d.prm->vlongMax) return false;
+    d.fbQueue[d.Pcap - 1 - i] = e;
+  }
   atomicAdd(&d.S->err[E_LONG_QUEUE], 1ull);
   return true;
 }
@@ -2938,6 +2950,8 @@ static sqdem_status uploadParams(sqdem_ctx* c) {
   const bool nm = c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN;
   P.vlongBucket = nm ? LONG_BUCKET_NM : c->precision == SQDEM_MIXED ? LONG_BUCKET_MIXED : c->inBatch ? LONG_BUCKET_BATCH : LONG_BUCKET_FP64;
   P.vlongFront = nm ? LONG_FRONT_NM : c->precision == SQDEM_MIXED ? LONG_FRONT_MIXED : LONG_FRONT_FP64;
+  // (the mixed form's results depend on which searches run in FP64)
+  P.vlongMax = nm || c->precision == SQDEM_MIXED ? INT_MAX : LONG_MAX_FP64;
   P.h0 = hostH0(c);
   CK(cudaMemcpyAsync(c->d.prm, &P, sizeof(P), cudaMemcpyHostToDevice, c->stream));
   return SQDEM_OK;

@@ -1,6 +1,7 @@
 """Batches of specimens: one graph launch steps every scene; each scene's results are those of
 its context stepped alone (bitwise), in both precision forms, with the CompressionEngine."""
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
@@ -115,4 +116,26 @@ def test_searches_in_rounds_equal_searches_by_warps(gpu, precision, sizes):
         e.sync()
         assert np.array_equal(b.scenes[i].interactions(True), e.interactions(True)), i
         assert np.array_equal(b.scenes[i].body_state(), e.body_state()), i
+    b.close()
+
+
+def test_more_long_searches_than_warps_take_at_once(gpu):
+    """The second step of a freshly loaded dense cell has some 23,000 searches that ran 8 iterations or
+    more: the FP64 form gives the longest and 6,000 others a warp, the rest goes to the rounds.  In a
+    batch the line is 16 iterations (some 6,000 searches, all of which take a warp): the same bits."""
+    tile = os.path.join(os.path.dirname(__file__), "golden", "config1_tile.npz")
+    spec = assemblies.config1_dense(tile, tiles=3)
+    e = Engine()
+    e.load(spec)
+    e.step(1)
+    e.sync()
+    e.step(1)
+    assert e.sync()["long_queue"] > 6000
+    e.step(1)
+    b = Batch(1)
+    b.load([spec])
+    b.step(3)
+    b.sync()
+    assert np.array_equal(b.scenes[0].interactions(True), e.interactions(True))
+    assert np.array_equal(b.scenes[0].body_state(), e.body_state())
     b.close()
