@@ -569,8 +569,8 @@ def run_ours(args):
     flops = pipe_flops_per_eval()
     traffic = profiled_search_traffic(args.workload)
     # the roofline of each form's dominant kernel (the search kernel): issue-bound on the pipe
-    # its evaluations run on (FP64 for k_contacts_lm; FP32 for the double-float
-    # k_contacts_lm_ff), against this GPU's measured FMA peak of that pipe
+    # its evaluations run on (FP64: k_search_warp and the k_wave_* rounds; FP32: the double-float
+    # k_ff_* rounds), against this GPU's measured FMA peak of that pipe
     for p, r in res.items():
         ev = r["evals_per_step"]["double_float" if p == "mixed" else "fp64"]
         kms = r["search_kernel_ms"]
@@ -580,7 +580,8 @@ def run_ours(args):
         peak_eval = peaks["disfunction_ff_geval_s" if p == "mixed" else "disfunction_fp64_geval_s"] * 1e9
         rate = ev / (kms / 1e3) if kms > 0 else 0.0
         achieved = rate * fpe / 1e12 if fpe else None
-        r["roofline"] = {"bound": pipe, "kernel": "k_contacts_lm_ff" if p == "mixed" else "k_contacts_lm",
+        r["roofline"] = {"bound": pipe, "kernel": "k_ff_trial, k_ff_probe, k_ff_warp" if p == "mixed" else
+                         "k_search_warp, k_wave_trial, k_wave_probe",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak if achieved is not None else None,
                          "peak_source": "measured on this GPU by sqdem_pipe_peaks (FMA loop of that pipe)",

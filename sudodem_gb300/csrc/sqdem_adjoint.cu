@@ -9,9 +9,9 @@
 // depth gate.  Ip2 is applied afresh to every pair at the start of the window, so the contact
 // stiffness and friction are functions of the current material parameters.
 //
-// Forward: a group of six lanes per pair runs the narrowphase (Levenberg-Marquardt restated one
-// evaluation after another, lmder2 Superquadrics_Ig2.cpp:1057-1354, with its restart rules
-// :2013-2053; each evaluation shared by the group), precompute (Superquadrics.cpp:1030-1050)
+// Forward: a warp per pair runs the narrowphase (Levenberg-Marquardt restated, six points a
+// round, lmder2 Superquadrics_Ig2.cpp:1057-1354, with its restart rules
+// :2013-2053; five lanes a point), precompute (Superquadrics.cpp:1030-1050)
 // and the law (:1209-1361); one thread per body gathers forces in a fixed order and integrates
 // (NewtonIntegrator.cpp:99-304, 391-429).  The state is checkpointed every `checkpoint_every`
 // steps.

@@ -5,7 +5,7 @@
 // each ~18 pow + 4 atan2 + 6 sincos.  These kernels measure, on the device itself:
 //   * the FP64 and FP32 fused multiply-add rates (independent FMA chains, 2 flops each);
 //   * the rate of FP64 Disfunction evaluations when every lane of a full grid evaluates
-//     independent points (the evaluation-mix peak that bounds k_contacts_lm).
+//     independent points (the evaluation-mix peak that bounds the FP64 searches).
 // No counterpart in the reference.  Compiled with --fmad=false like the engine; the FMA loops
 // use explicit fma() / fmaf() so they still issue fused multiply-adds.
 #include <cuda_runtime.h>
