@@ -57,7 +57,7 @@ __device__ __forceinline__ D3 mulG(const Rot& R, D3 v) {
             R.m[6] * v.x + (R.m[7] * v.y + R.m[8] * v.z));
 }
 // R^T * v == rot_mat2local * v (same coefficients, same order)
-__device__ __forceinline__ D3 mulL(const Rot& R, D3 v) {
+__host__ __device__ __forceinline__ D3 mulL(const Rot& R, D3 v) {
   return d3(R.m[0] * v.x + (R.m[3] * v.y + R.m[6] * v.z),
             R.m[1] * v.x + (R.m[4] * v.y + R.m[7] * v.z),
             R.m[2] * v.x + (R.m[5] * v.y + R.m[8] * v.z));
@@ -100,10 +100,31 @@ __device__ __forceinline__ D3 supportLocal(const SqShape& s, D3 n) {
   return r;
 }
 // Superquadrics::isInside (Superquadrics.cpp:103-108); p is relative to the centre.
-__device__ __forceinline__ bool isInside(const SqShape& s, D3 p) {
+__host__ __device__ __forceinline__ bool isInside(const SqShape& s, D3 p) {
   p = mulL(s.R, p);
   return 1 > pow(pow(fabs(p.x / s.rx), 2.0 / s.e1) + pow(fabs(p.y / s.ry), 2.0 / s.e1), s.e1 / s.e2) +
                  pow(fabs(p.z / s.rz), 2.0 / s.e2);
+}
+// isInside decided in FP32 where its value is far from 1: 1 inside, 0 outside, -1 for the FP64 test
+// (six pow, four divisions: some 40,000 cycles of the FP64 pipe; here the 15 products and sums of the
+// local coordinates and 8 conversions).  With x, y, z the local coordinates over the radii, m the larger
+// and n the smaller of |x|, |y|, the value is
+//   (m (1 + (n/m)^(2/eps1))^(eps1/2))^(2/eps2) + |z|^(2/eps2)
+// where the bracket's second factor is between 1 and 2 and only (n/m)^(2/eps1) can underflow before the
+// last power, beside the 1.  For eps >= 0.01 the value near 1 is off by less than 2e-4: three roundings
+// in each of x, y, z, one more in n/m, two powf of at most 4 ulp, a sum and a product in the bracket,
+// 8.5e-7 in all, raised to 2/eps2 <= 200.  isInside's own |x|^(2/eps1) underflows below |x| = 0.029 at
+// eps1 = 0.01, which takes up to 0.029 off its value.  Both are within the band: a point is decided where
+// the value is outside [0.9, 1.1].
+__host__ __device__ __forceinline__ int insideFast(const SqShape& s, D3 p) {
+  const float e1 = (float)s.e1, e2 = (float)s.e2, rx = (float)s.rx, ry = (float)s.ry, rz = (float)s.rz;
+  if (!(e1 >= 0.01f && e2 >= 0.01f)) return -1;
+  if (!(fminf(rx, fminf(ry, rz)) >= 1e-25f && fmaxf(rx, fmaxf(ry, rz)) <= 1e25f)) return -1;   // FP32's own range
+  p = mulL(s.R, p);
+  const float x = fabsf((float)p.x / rx), y = fabsf((float)p.y / ry), z = fabsf((float)p.z / rz);
+  const float m = x > y ? x : y, t = m > 0.f ? (x > y ? y : x) / m : 0.f;   // (NaN in either stays NaN)
+  const float v = powf(m * powf(1.f + powf(t, 2.f / e1), 0.5f * e1), 2.f / e2) + powf(z, 2.f / e2);
+  return v < 0.9f ? 1 : v > 1.1f ? 0 : -1;   // NaN: the FP64 test
 }
 
 // Disfunction, 9-argument form (pkg/dem/Superquadrics_Ig2.cpp:622-687).

@@ -1752,21 +1752,6 @@ __device__ __forceinline__ bool angleTest(double sep, double nrmf, const D3& c) 
   return fabs(sep / (nrmf * nrm(c))) > 0.95;
 }
 
-// isInside (Superquadrics.cpp:103-108) of p relative to the centre, decided in FP32 where it is far
-// from its threshold: 1 inside, 0 outside, -1 for the FP64 test (six pow).  The FP32 value is off by
-// some 1e-6 times its exponents (2/eps1, 2/eps2 up to 200 here); a point is decided outside [0.9, 1.1].
-__device__ __forceinline__ int insideFast(const SqShape& s, D3 p) {
-  const float e1 = (float)s.e1, e2 = (float)s.e2;
-  if (!(e1 >= 0.01f && e2 >= 0.01f)) return -1;
-  const float px = (float)p.x, py = (float)p.y, pz = (float)p.z;
-  const float x = (float)s.R.m[0] * px + (float)s.R.m[3] * py + (float)s.R.m[6] * pz;
-  const float y = (float)s.R.m[1] * px + (float)s.R.m[4] * py + (float)s.R.m[7] * pz;
-  const float z = (float)s.R.m[2] * px + (float)s.R.m[5] * py + (float)s.R.m[8] * pz;
-  const float v = powf(powf(fabsf(x / (float)s.rx), 2.f / e1) + powf(fabsf(y / (float)s.ry), 2.f / e1), e1 / e2) +
-                  powf(fabsf(z / (float)s.rz), 2.f / e2);
-  return v < 0.9f ? 1 : v > 1.1f ? 0 : -1;   // NaN: the FP64 test
-}
-
 #include "sq_wave_search.cuh"
 #include "sq_warp_search.cuh"
 
