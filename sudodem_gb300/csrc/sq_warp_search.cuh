@@ -21,6 +21,8 @@
 // search's results do not depend on the schedule: speculative points that it does not come to are
 // dropped.
 
+#include "sq_warp_plan.cuh"
+
 static const int WS_LANES = 5, WS_POINTS = 6;
 
 // sgn(n) * y for y >= 0 (0 when n is 0, where y is 0 in every use), without the multiplication
@@ -297,18 +299,9 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
         more = false;
         resume = false;
         for (;;) {   // damping loop: the step for mu, and those that follow its rejections
-          // Twelve points: four trials with their probes.  Six: a slow search divides mu by three at
-          // every accepted trial, until trials are rejected (two to five in a row, mu times 2, 4, 8
-          // ...) and mu is above the level again below which it was rejected last, muRej, which moves
-          // little: so the trials up to the first above that level take a group each, and that
-          // one's probes two more.  plan: the trial whose probes are evaluated with it (0: those of
-          // every trial; 4: none).
-          int rej = 0;
-          if (W == 1) for (double m = mu; rej < 4 && m <= muRej; rej++) m *= (double)(2 << rej) * 0.5 * nu;
-          const int plan = rej < 2 ? 0 : rej;
-          const int trial = !real ? 0 : plan == 0 ? grp / 3 : plan == 2 ? (grp < 2 ? grp : grp < 5 ? 2 : 3) : plan == 3 ? min(grp, 3) : grp;
-          const int role = plan == 0 ? grp % 3 : plan == 4 ? 0 : max(0, min(2, grp - plan)) * (grp < plan + 3 ? 1 : 0);
-          const int trials = plan == 0 ? 2 * W : plan == 4 ? WS_POINTS : 4;
+          const int plan = wsPlan<W>(mu, muRej, nu);
+          const int trial = real ? wsTrial(plan, grp) : 0, role = wsRole(plan, grp);
+          const int trials = wsTrials<W>(plan);
           double myMu = mu;
           for (int j = 0, m = nu; j < trial; j++, m = (int)((unsigned)m << 1)) myMu *= m;
           const double bo = (odd ? diag0 : diag1) + myMu, bx = (odd ? diag1 : diag0) + myMu;   // even lanes: Dp0, odd lanes: Dp1
@@ -329,7 +322,7 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
           ev64 += WS_POINTS * W;
           bool ended = false, accepted = false;
           for (int a = 0; a < trials; a++) {
-            const int g = plan == 0 ? 3 * a : plan == 2 && a == 3 ? 5 : a;
+            const int g = wsGroup(plan, a);
             const WSlot& o = q[g];
             if (a > 0 && (o.bits & (WB_SMALL | WB_HUGE))) {   // the step after the last rejection ends the call
               end((o.bits & WB_SMALL) ? 2 : 4);
@@ -350,7 +343,7 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
               more = outer();
               accepted = true;
               // the probes at the accepted trial: in this round's groups, or a round of their own
-              const bool have = plan == 0 || a == plan;
+              const bool have = wsProbed(plan, a);
               probe0 = have ? g + 1 : 0; probe1 = have ? g + 2 : 1;
               if (more && !have) {
                 round(grp == 0 ? p0 + Dp0 : p0, grp == 1 ? p1 + Dp1 : p1, false, 0, 0, 0, 0, 0, 0, 0, 0, 0u);
