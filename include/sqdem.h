@@ -103,17 +103,22 @@ typedef struct {
   long long collider_runs;    /* collider passes executed */
   long long steps;            /* timesteps executed */
   long long evals_fp32;       /* Disfunction evaluations on the FP32 pipes (double-float, mixed form) */
-  long long evals_fp64;       /* Disfunction evaluations in FP64 */
-  long long lm_rounds_max;    /* longest contact among those searched one per warp, in its rounds of up
-                                 to six evaluations (the critical path of the contact stage), max over
-                                 steps */
+  long long evals_fp64;       /* Disfunction evaluations in FP64, those made ahead for points that the
+                                 search then did not ask for included */
+  long long lm_rounds_max;    /* longest FP64 search, in rounds one after another (the critical path of
+                                 the contact stage), max over steps.  A round is one evaluation in the
+                                 kernels that advance lists of searches, one launch at a time (in
+                                 k_nm_round up to four), and up to six evaluations where a warp runs a
+                                 search, twelve where two do */
   long long fallback_fp64;    /* mixed form: searches deferred to the FP64 kernel (a decision
                                  inside its rounding band, itmax reached, or an evaluation it does
                                  not reproduce) */
-  long long lm_rounds_max_ff; /* mixed form: longest search in rounds of the double-float kernel
-                                 (lm_rounds_max: of the FP64 kernel) */
-  long long long_queue;       /* searches that ran long at the previous step (mixed form: 32+
-                                 iterations; FP64 form: 8+, in a batch 16+), run one per warp in FP64 */
+  long long lm_rounds_max_ff; /* mixed form: longest double-float search, in rounds of one evaluation in
+                                 the list kernels and up to sixteen where a warp runs a search */
+  long long long_queue;       /* searches that ran long at the previous step and were run from the start
+                                 by a warp or two each, in FP64: 32+ iterations in the mixed form, 8+ in
+                                 the FP64 form (16+ in a batch; of those below 32 at most 6,000 a step),
+                                 32+ evaluations in the Hertz-Mindlin model */
 } sqdem_report;
 
 /* Record layouts shared with the CPU oracle (doubles per record). */

@@ -61,7 +61,7 @@ __device__ __forceinline__ void ffLoad(const Dev& d, int i, LMF& L) {
   const unsigned f = (unsigned)c.z;
   L.k = c.x; L.nu = c.y; L.iters = (unsigned)c.w; L.stop = 0; L.touching = true;
   L.phase = (int)(f & 7u); L.fromCenter = f & WF_FROMCENTER; L.isNew = f & WF_NEW; L.stopFlag = f & WF_STOPFLAG;
-  L.calls = (f >> 8) & 15u; L.maxit = (f >> 12) & 15u; L.rounds = 0;
+  L.calls = (f >> 8) & 15u; L.maxit = (f >> 12) & 15u; L.rounds = f >> 16;
   const double2 p = B.angle[i];
   const double4 n = B.normal[i], s = B.shear[i], g = B.nforce[i], h = B.phys[i];
   L.p0 = ffUnpack(p.x); L.p1 = ffUnpack(p.y);
@@ -75,7 +75,8 @@ __device__ __forceinline__ void ffLoad(const Dev& d, int i, LMF& L) {
 __device__ __forceinline__ void ffStore(const Dev& d, int i, const LMF& L) {
   const Table& B = d.B;
   const unsigned f = (unsigned)L.phase | (L.fromCenter ? WF_FROMCENTER : 0u) | (L.isNew ? WF_NEW : 0u) |
-                     (L.stopFlag ? WF_STOPFLAG : 0u) | (L.st == LMF_ST_INIT ? WF_INIT : 0u) | (L.calls << 8) | (L.maxit << 12);
+                     (L.stopFlag ? WF_STOPFLAG : 0u) | (L.st == LMF_ST_INIT ? WF_INIT : 0u) | (L.calls << 8) | (L.maxit << 12) |
+                     (L.rounds << 16);
   B.owner[i] = L.e;
   B.cd[i] = make_int4(L.k, L.nu, (int)f, (int)L.iters);
   B.angle[i] = make_double2(ffPack(L.p0), ffPack(L.p1));
@@ -92,7 +93,7 @@ __device__ __forceinline__ void ffFinal(const Dev& d, int i, const LMF& L) {
   B.p1[i] = make_double4(ffPack(L.P1[0]), ffPack(L.P1[1]), ffPack(L.P1[2]), 0);
   B.p2[i] = make_double4(ffPack(L.P2[0]), ffPack(L.P2[1]), ffPack(L.P2[2]), 0);
   B.phys[i] = make_double4(ffPack(L.c[0]), ffPack(L.c[1]), ffPack(L.c[2]), 0);
-  B.cd[i] = make_int4((int)L.calls, (int)L.iters, (int)L.maxit, L.touching ? 1 : 0);
+  B.cd[i] = make_int4((int)L.calls, (int)L.iters, (int)L.maxit, (int)(L.rounds << 1) | (L.touching ? 1 : 0));
 }
 __device__ __forceinline__ int mainEntry(const Dev& d, int j) {
   const int nFront = d.S->lmCount;
@@ -127,7 +128,11 @@ __device__ __forceinline__ void ffRoute(const Dev& d, int i, bool mine, int r, c
   if (mine) {
     if (r == LMF_END) ffFinal(d, i, L);
     else if (r == LMF_MORE) ffStore(d, i, L);
-    else { d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = L.e; deferred++; }
+    else {
+      d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = L.e;
+      deferred++;
+      atomicMax(&d.S->err[E_ROUNDS_MAX_FF], (unsigned long long)L.rounds);
+    }
   }
   const bool more = mine && r == LMF_MORE;
   waveAppend(more && L.st == LMF_ST_PROBE0, i, d.waveP, &d.Q->nP[round]);
@@ -181,6 +186,7 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_trial(Dev d, int round) {
     int r = LMF_DEFER;
     if (mine) {
       ev++;
+      L.rounds++;
       r = lmfConsume(L, v);
       if (r == LMF_END) r = lmfCallEnd(d, L, id1, id2, pB);
     }
@@ -228,6 +234,7 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_probe(Dev d, int round) {
     ffPairEval(s, isB, pB, L.q0, L.q1, v);
     if (mine) {
       ev += 2;
+      L.rounds += 2;
       if (r == LMF_MORE) r = lmfConsume(L, v);
       if (r == LMF_END) r = lmfCallEnd(d, L, id1, id2, pB);
     }
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_warp(Dev d, int tail, int round
     L.E = E;
     bool resume = tail && L.st != LMF_ST_INIT;   // the call goes on at the pending trial
     int r = LMF_MORE;
-    unsigned nr = 0;
+    unsigned nr = L.rounds;
     // every lane carries the whole state; L holds it between calls
     do {   // one lmder2 call
       ff p0 = L.p0, p1 = L.p1, mu = L.mu, Dp0 = L.Dp0, Dp1 = L.Dp1, pfL2 = L.pfL2;
@@ -411,6 +418,7 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_warp(Dev d, int tail, int round
         resume = false;
       }
     } while (r == LMF_MORE);
+    L.rounds = nr;
     if (lane == 0) {
       if (r == LMF_END) { ffFinal(d, i, L); d.waveF[atomicAdd(&d.Q->nF, 1)] = i; }
       else { d.deferQueue[atomicAdd(&d.S->fbCount, 1)] = e; deferred++; }

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_
     int phase = 0;
     unsigned calls = 0, iters = 0, maxit = 0, rounds = 0;
     bool touching = true;
-    if (mode == WS_TAIL) { contact = w.contact; phase = (int)w.phase; calls = w.calls; iters = w.iters; maxit = w.maxit; }
+    if (mode == WS_TAIL) { contact = w.contact; phase = (int)w.phase; calls = w.calls; iters = w.iters; maxit = w.maxit; rounds = w.rounds; }
     WSlot* q = slots[own][flip];   // the last round's points
     // evaluates the lane's group's point into the round's slots; the other trial fields are the caller's
     auto round = [&](double q0, double q1, bool trial, double D0, double D1, double t0, double t1, double myMu, double pfL2,

@@ -20,14 +20,15 @@
 // Search time of a jammed cell of 200,000: 24.4 -> 18 ms, of 43,011: 11.4 -> 5.8.  Values, decisions
 // and results per search are those of k_search_warp, bit for bit.
 
-static const unsigned WF_FROMCENTER = 8u, WF_NEW = 16u, WF_STOPFLAG = 32u, WF_INIT = 64u;   // with phase in bits 0-2
+// flag word of a slot: phase in bits 0-2, these, calls from bit 8, maxit from 12, rounds so far from 16
+static const unsigned WF_FROMCENTER = 8u, WF_NEW = 16u, WF_STOPFLAG = 32u, WF_INIT = 64u;
 
 // A search's state between launches, slot i of table B.
 struct WaveState {
   double p0, p1, mu, D0, D1, pfL2, diag0, diag1, j01, jt0, jt1;
   D3 pf, contact;
   int e, k, nu;
-  unsigned phase, calls, iters, maxit;
+  unsigned phase, calls, iters, maxit, rounds;   // rounds: evaluations one after another, for the report
   bool fromCenter, isNew, stopFlag, init;
 };
 __device__ __forceinline__ void waveLoad(const Dev& d, int i, WaveState& w) {
@@ -37,7 +38,7 @@ __device__ __forceinline__ void waveLoad(const Dev& d, int i, WaveState& w) {
   const unsigned f = (unsigned)c.z;
   w.k = c.x; w.nu = c.y; w.iters = (unsigned)c.w;
   w.phase = f & 7u; w.fromCenter = f & WF_FROMCENTER; w.isNew = f & WF_NEW; w.stopFlag = f & WF_STOPFLAG; w.init = f & WF_INIT;
-  w.calls = (f >> 8) & 15u; w.maxit = (f >> 12) & 15u;
+  w.calls = (f >> 8) & 15u; w.maxit = (f >> 12) & 15u; w.rounds = f >> 16;
   const double2 p = B.angle[i];
   const double4 n = B.normal[i], s = B.shear[i], g = B.nforce[i], h = B.phys[i];
   w.p0 = p.x; w.p1 = p.y;
@@ -49,7 +50,7 @@ __device__ __forceinline__ void waveLoad(const Dev& d, int i, WaveState& w) {
 __device__ __forceinline__ void waveStore(const Dev& d, int i, const WaveState& w) {
   const Table& B = d.B;
   const unsigned f = w.phase | (w.fromCenter ? WF_FROMCENTER : 0u) | (w.isNew ? WF_NEW : 0u) | (w.stopFlag ? WF_STOPFLAG : 0u) |
-                     (w.init ? WF_INIT : 0u) | (w.calls << 8) | (w.maxit << 12);
+                     (w.init ? WF_INIT : 0u) | (w.calls << 8) | (w.maxit << 12) | (w.rounds << 16);
   B.owner[i] = w.e;
   B.cd[i] = make_int4(w.k, w.nu, (int)f, (int)w.iters);
   B.angle[i] = make_double2(w.p0, w.p1);
@@ -62,7 +63,7 @@ __device__ __forceinline__ void waveStore(const Dev& d, int i, const WaveState& 
 __device__ __forceinline__ void waveFinal(const Dev& d, int i, const WaveState& w, bool touching, D3 P1, D3 P2) {
   const Table& B = d.B;
   B.owner[i] = w.e;
-  B.cd[i] = make_int4((int)w.calls, (int)w.iters, (int)w.maxit, touching ? 1 : 0);
+  B.cd[i] = make_int4((int)w.calls, (int)w.iters, (int)w.maxit, (int)(w.rounds << 1) | (touching ? 1 : 0));
   B.angle[i] = make_double2(w.p0, w.p1);
   B.phys[i] = dd4(w.contact, 0);
   B.p1[i] = dd4(P1, 0); B.p2[i] = dd4(P2, 0);
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(LM_BS, 3) k_wave_trial(Dev d, int round) {
       w.e = j < nFront ? d.lmQueue[j] : d.lmQueue[d.qCap - 1 - (j - nFront)];
       w.isNew = !(d.A.flags[w.e] & F_GEOM);
       w.fromCenter = w.isNew; w.init = true; w.stopFlag = false;
-      w.phase = 0; w.calls = 0; w.iters = 0; w.maxit = 0;
+      w.phase = 0; w.calls = 0; w.iters = 0; w.maxit = 0; w.rounds = 0;
       w.jt0 = w.jt1 = w.j01 = w.diag0 = w.diag1 = 0;
       w.contact = d3(0, 0, 0);
     } else waveLoad(d, i, w);
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(LM_BS, 3) k_wave_trial(Dev d, int round) {
     double sep;
     pairEval(l, q0, q1, c, P1, P2, f, sep);
     if (valid && !(lane & 1)) ev64++;
+    w.rounds++;
     const double fl2 = nrm(f);
     if (sep > 0) w.stopFlag = true;
     int stop = 0;
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(LM_BS, 3) k_wave_probe(Dev d, int round) {
     pairEval(l, w.p0, w.p1 + w.D1, c, P1, P2, f2, sep);
     if (sep > 0) w.stopFlag = true;
     if (valid && !odd) ev64 += 2;
+    w.rounds += 2;
     // even lane: column 0 of the Jacobian, odd lane: column 1
     const D3 g = odd ? f2 : f1;
     const double D = odd ? w.D1 : w.D0;
@@ -346,6 +349,7 @@ __global__ void __launch_bounds__(LM_BS, 3) k_wave_probe(Dev d, int round) {
 __global__ void __launch_bounds__(128) k_wave_finish(Dev d) {
   const int n = d.Q->nF;
   Counters cnt = {0, 0, 0, 0, 0};
+  unsigned roundsMax = 0;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const int i = d.waveF[j], e = d.B.owner[i];
     const int4 c = d.B.cd[i];
@@ -353,8 +357,10 @@ __global__ void __launch_bounds__(128) k_wave_finish(Dev d) {
     const unsigned fl = d.A.flags[e];
     int id1, id2;
     entryIds(d, e, fl, id1, id2);
-    finishSearch(d, e, fl, id1, id2, !(fl & F_GEOM), p.x, p.y, c.w != 0, xyz(d.B.p1[i]), xyz(d.B.p2[i]), xyz(d.B.phys[i]),
+    roundsMax = max(roundsMax, (unsigned)c.w >> 1);
+    finishSearch(d, e, fl, id1, id2, !(fl & F_GEOM), p.x, p.y, (c.w & 1) != 0, xyz(d.B.p1[i]), xyz(d.B.p2[i]), xyz(d.B.phys[i]),
                  (unsigned)c.x, (unsigned)c.y, (unsigned)c.z, cnt);
   }
   flushCounters(d, cnt);
+  flushRounds(d, E_ROUNDS_MAX, roundsMax);
 }

@@ -1221,6 +1221,11 @@ __device__ __forceinline__ void flushCounters(const Dev& d, Counters c) {
     if (c.nanF) atomicAdd(&d.S->err[E_NAN_FORCE], c.nanF);
   }
 }
+// the longest search of a finish kernel's threads, in rounds (word: E_ROUNDS_MAX or E_ROUNDS_MAX_FF)
+__device__ __forceinline__ void flushRounds(const Dev& d, int word, unsigned rounds) {
+  rounds = __reduce_max_sync(0xffffffffu, rounds);
+  if ((threadIdx.x & 31) == 0 && rounds) atomicMax(&d.S->err[word], (unsigned long long)rounds);
+}
 
 // Ip2_SuperquadricsMat2_SuperquadricsMat2_HertzMindlinPhys::go (Superquadrics.cpp:1118-1160) and
 // SuperquadricsLaw2::go (Superquadrics.cpp:1367-1557) for one entry whose geometry g was just
@@ -1957,11 +1962,13 @@ __global__ void __launch_bounds__(128) k_ff_finish(Dev d) {
   const double dt = d.prm->dt;
   Counters cnt = {0, 0, 0, 0, 0};
   unsigned long long deferred = 0;
+  unsigned roundsMax = 0;
   for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
     if (i0 + threadIdx.x >= n) continue;
     const int i = d.waveF[i0 + threadIdx.x];
     const int e = d.B.owner[i];
     const int4 info = d.B.cd[i];
+    roundsMax = max(roundsMax, (unsigned)info.w >> 1);
     const unsigned fl = d.A.flags[e];
     int id1, id2;
     entryIds(d, e, fl, id1, id2);
@@ -1975,7 +1982,7 @@ __global__ void __launch_bounds__(128) k_ff_finish(Dev d) {
     const double2 an = d.B.angle[i];
     g.ang0 = ffToD(ffUnpack(an.x)); g.ang1 = ffToD(ffUnpack(an.y)); g.angSet = true;
     bool ok = true;
-    if (!info.w) {
+    if (!(info.w & 1)) {
       g.precomputed = false; g.depth = 0; g.isShearNew = true;
     } else {
       const D3 P1 = b1.pos + unpack(d.B.p1[i]), P2 = b1.pos + unpack(d.B.p2[i]);
@@ -2003,6 +2010,7 @@ __global__ void __launch_bounds__(128) k_ff_finish(Dev d) {
     }
   }
   flushCounters(d, cnt);
+  flushRounds(d, E_ROUNDS_MAX_FF, roundsMax);
   if (deferred) atomicAdd(&d.S->err[E_FALLBACK], deferred);
 }
 

@@ -139,3 +139,29 @@ def test_more_long_searches_than_warps_take_at_once(gpu):
     assert np.array_equal(b.scenes[0].interactions(True), e.interactions(True))
     assert np.array_equal(b.scenes[0].body_state(), e.body_state())
     b.close()
+
+
+@pytest.mark.parametrize("precision,small,large", [("fp64", 250, 15800), ("mixed", 250, 7800)])
+def test_report_counts_the_rounds_of_every_search(gpu, precision, small, large):
+    """The report's longest search counts what was run in rounds over lists as well as what a warp ran.
+    Alone, both scenes give each search a warp, several evaluations a round; in the batch the first four (FP64)
+    or three rounds, a trial and two probes each, run over lists, one evaluation a round, which takes a
+    search no fewer rounds."""
+    ss = [assemblies.cubic_specimen(n, seed=41 + i, eps_range=(0.3, 1.7), spacing=2.1e-3, wall_gap=0.0)
+          for i, n in enumerate((small, large))]
+    word = "lm_rounds_max" if precision == "fp64" else "lm_rounds_max_ff"
+    alone = []
+    for spec in ss:
+        e = Engine(precision=precision)
+        e.load(spec)
+        e.step(1)
+        alone.append(e.sync()[word])
+    b = Batch(2, precision=precision)
+    b.load(ss)
+    b.step(1)
+    rep = b.sync()
+    b.close()
+    # a search that goes on to the warps has been through all of the lists' rounds
+    lists = 3 * (4 if precision == "fp64" else 3)
+    assert max(alone) > lists
+    assert rep[word] >= max(alone)
