@@ -158,17 +158,20 @@ sqdem_status sqdem_set_bodies(sqdem_ctx* ctx, int n, const int* kind, const doub
                               const double* state);
 sqdem_status sqdem_set_params(sqdem_ctx* ctx, const sqdem_params* p);
 
-/* Launch shapes of the contact stage: resident blocks per SM of the search kernel (at most
- * what its occupancy allows) and grid-stride blocks per SM of the first contact pass; 0 keeps
- * the default.  Shapes change no result, only the time. */
+/* Launch shapes of the contact stage: resident blocks per SM of the search kernels (at most
+ * what their occupancy allows) and grid-stride blocks per SM of the first contact pass; 0 keeps
+ * the default.  Shapes change no result, only the time.  The search blocks have an effect in the
+ * mixed form, and for more than 16,000 particles (in the Hertz-Mindlin model 10,000; of the scene or
+ * of the batch it steps in) in the FP64 form; smaller scenes give every search a warp, in grids of a fixed size. */
 sqdem_status sqdem_set_launch_shape(sqdem_ctx* ctx, int search_blocks_per_sm, int pass1_blocks_per_sm);
 typedef struct {
   int search_blocks_per_sm, pass1_blocks_per_sm;   /* the shape chosen and set */
   double ms_per_step;                               /* its device time per step */
   int candidates;                                   /* shapes timed */
 } sqdem_tune;
-/* Autotuner: times each candidate shape (search blocks per SM 1..occupancy x pass-1 blocks
- * per SM 4/8/16/32) for `steps` timesteps on the scene itself, twice, and sets the fastest.
+/* Autotuner: times each candidate shape (search blocks per SM 1..occupancy, where they have an
+ * effect, x pass-1 blocks per SM 4/8/16/32) for `steps` timesteps on the scene itself, twice, and
+ * sets the fastest; search blocks without an effect are left as they are.
  * The tuning steps are ordinary timesteps (shapes change no result): the scene advances by
  * candidates x (2 x steps + 1) steps.  No counterpart in the reference. */
 sqdem_status sqdem_autotune(sqdem_ctx* ctx, int steps, sqdem_tune* out);

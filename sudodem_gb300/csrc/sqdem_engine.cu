@@ -2726,6 +2726,13 @@ static int nmRounds(const sqdem_ctx* c, const Dev& d) {
   return n <= NM_WARP_MAX ? 0 : 6;
 }
 
+// Whether the contact stage of this scene has kernels whose grid searchBlocksPerSM gives: the rounds'
+// and the double-float ones.
+static bool searchShapeUsed(const sqdem_ctx* c, const Dev& d) {
+  if (c->contactModel == SQDEM_CONTACT_HERTZ_MINDLIN) return nmRounds(c, d) > 0;
+  return c->precision == SQDEM_MIXED || std::max(c->load, d.NP) > WARP_SEARCH_MAX;
+}
+
 // shared memory of a k_search_warp<W> block: the trial points of its searches, two rounds of them
 static size_t wsShared(int W, int threads) { return sizeof(WSlot) * 2 * WS_POINTS * W * (threads / (32 * W)); }
 
@@ -3821,28 +3828,31 @@ sqdem_status sqdem_set_launch_shape(sqdem_ctx* c, int search_blocks_per_sm, int 
 // Time every candidate shape on the scene itself: two rounds over the candidates, `steps`
 // timesteps each (CUDA events on the context stream), the minimum per candidate kept.  Since
 // shapes change no result these are ordinary timesteps: the scene advances by
-// candidates x (2 x steps + 1) steps, as it would with the default shape.
+// candidates x (2 x steps + 1) steps, as it would with the default shape.  Where every search has a
+// warp (searchShapeUsed) no kernel reads the search blocks: only pass 1's shapes are timed then.
 sqdem_status sqdem_autotune(sqdem_ctx* c, int steps, sqdem_tune* out) {
   if (!c || steps <= 0) return SQDEM_ERR_ARG;
   if (!c->haveBodies) return fail(c, SQDEM_ERR_STATE, "no bodies");
   const int mx = maxSearchBlocksPerSM(c);
+  const bool sweep = searchShapeUsed(c, c->d);
+  const int lo = sweep ? 1 : searchBlocksPerSM(c), hi = sweep ? mx : lo;
   const int p1s[4] = {4, 8, 16, 32};
-  std::vector<double> t(4 * (size_t)mx, 1e300);
+  std::vector<double> t(4 * (size_t)(hi - lo + 1), 1e300);
   sqdem_status s;
   for (int round = 0; round < 2; round++)
-    for (int sb = 1; sb <= mx; sb++)
+    for (int sb = lo; sb <= hi; sb++)
       for (int k = 0; k < 4; k++) {
-        if ((s = sqdem_set_launch_shape(c, sb, p1s[k]))) return s;
+        if ((s = sqdem_set_launch_shape(c, sweep ? sb : c->shapeSearch, p1s[k]))) return s;
         if (round == 0 && (s = sqdem_step(c, 1))) return s;   // graph capture outside the timing
         double ms = 0;
         if ((s = sqdem_time_steps(c, steps, &ms))) return s;
-        double& b = t[4 * (size_t)(sb - 1) + k];
+        double& b = t[4 * (size_t)(sb - lo) + k];
         b = std::min(b, ms);
       }
   size_t bi = 0;
   for (size_t i = 1; i < t.size(); i++) if (t[i] < t[bi]) bi = i;
-  const int bs = (int)(bi / 4) + 1, bp = p1s[bi % 4];
-  if ((s = sqdem_set_launch_shape(c, bs, bp))) return s;
+  const int bs = (int)(bi / 4) + lo, bp = p1s[bi % 4];
+  if ((s = sqdem_set_launch_shape(c, sweep ? bs : c->shapeSearch, bp))) return s;
   if (out) { out->search_blocks_per_sm = bs; out->pass1_blocks_per_sm = bp; out->ms_per_step = t[bi] / steps; out->candidates = (int)t.size(); }
   return SQDEM_OK;
 }

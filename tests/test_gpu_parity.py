@@ -353,6 +353,24 @@ def test_autotuned_launch_shapes_change_nothing(gpu):
         assert np.array_equal(c.body_state(), b.body_state())
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,model,swept", [("fp64", "linear", False), ("fp64", "hertz_mindlin", False),
+                                                   ("mixed", "linear", True)])
+def test_autotuner_times_only_shapes_that_are_read(gpu, precision, model, swept):
+    """A scene whose searches all have a warp reads no search blocks: four shapes of pass 1 are timed, and the
+    search blocks the caller set stay set.  The mixed form's search kernels read them."""
+    spec = assemblies.walled_lattice(64, seed=3, box=12e-3, per_side=4, spacing=2.2e-3)
+    e = Engine(device=0, precision=precision)
+    e.load(spec)
+    if model == "hertz_mindlin":
+        e.set_material_moduli([1e6] * len(spec.materials["Kn"]), [0.3] * len(spec.materials["Kn"]))
+        e.set_contact_model(model)
+    e.set_launch_shape(1, 0)
+    t = e.autotune(steps=1)
+    assert t["candidates"] > 4 if swept else (t["candidates"], t["search_blocks_per_sm"]) == (4, 1)
+    assert t["candidates"] % 4 == 0 and int(e.scalars()[0]) == 3 * t["candidates"]
+
+
 def _bed_statistics(spec, bodies, recs, slab=10e-3):
     """Packing fraction of the bottom slab (Superquadrics::Initial volumes of the particles
     whose centres lie in it, over the slab volume), coordination number (touching
