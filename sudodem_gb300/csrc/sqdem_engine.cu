@@ -91,7 +91,7 @@ static const unsigned DOF_ALL = 63u;
 struct Params {
   double dt, g[3], damping, verletDist, minSweepDistFactor, h0;
   int targetInterv, sortAxis, isSuperquadrics, exactAsphericalRot, recordFull;
-  int lmSpread;   // idle lanes evaluate the points running searches ask for next
+  int lmSpread;   // Nelder-Mead: lanes a search does not need evaluate points it may ask for next
   int contactModel;   // SQDEM_CONTACT_LINEAR or SQDEM_CONTACT_HERTZ_MINDLIN
   int periodicFix;    // sqdem_set_periodic_fix: torque arm and relative velocity of image contacts
   int vlongBucket;    // iteration bucket from which a search goes to the long-search queue
@@ -199,7 +199,7 @@ struct Dev {
   unsigned long long* bbPart;
   // boundary controller: per-wall kn sums of real contacts, per-block partial sums
   double* wallKn; double* svPart; int svBlocks;
-  int wallChunks, lmBlocks;   // grids sized to the scene
+  int wallChunks;   // sized to the scene
 };
 
 __device__ __forceinline__ unsigned long long encOrd(double x) {
@@ -2738,7 +2738,7 @@ static size_t wsShared(int W, int threads) { return sizeof(WSlot) * 2 * WS_POINT
 
 // The contact stage on c->stream: pass 1, then the searches of the selected contact model
 // (and, for Hertz-Mindlin, the finish pass of the contacts found touching).
-static void launchContactStage(sqdem_ctx* c, const Dev& d, int grid) {
+static void launchContactStage(sqdem_ctx* c, const Dev& d) {
   cudaStream_t s = c->stream;
   const int p1 = c->shapePass1 > 0 ? c->shapePass1 : PASS1_BLOCKS_PER_SM;
   const int pre = std::min(nblk(d.Pcap, 128), c->numSMs * p1);
@@ -2887,9 +2887,7 @@ static void enqueueStep(sqdem_ctx* c, bool timed) {
   // graph node around them was measured to cost as much as they do: 0.083 against 0.085 ms a step)
   enqueueCollider(c);
   if (timed) cudaEventRecord(c->ev[1], s);
-  // LM grid: all resident blocks, fewer for a small table (at most one lane per 4 entries)
-  const int lmFull = c->numSMs * searchBlocksPerSM(c);
-  launchContactStage(c, d, std::max(1, std::min(lmFull, nblk(d.Pcap, LM_BS * 4))));
+  launchContactStage(c, d);
   if (timed) cudaEventRecord(c->ev[2], s);
   k_wall_forces<<<d.W + 1, 128, 0, s>>>(d);
   c->launches++;
@@ -3645,7 +3643,7 @@ sqdem_status sqdem_time_contacts(sqdem_ctx* c, int nrep, double* ms) {
   CK(cudaEventRecord(c->ev[1], c->stream));
   for (int i = 0; i < nrep; i++) {
     k_reset_queue<<<1, 1, 0, c->stream>>>(d);
-    launchContactStage(c, d, c->numSMs * searchBlocksPerSM(c));
+    launchContactStage(c, d);
   }
   CK(cudaEventRecord(c->ev[2], c->stream));
   CK(cudaEventSynchronize(c->ev[2]));
@@ -3776,7 +3774,7 @@ sqdem_status sqdem_contacts_static_queue(sqdem_ctx* c) {
   d.qCap = SQDEM_STATIC_QUEUE_MAX;
   k_reset_queue<<<1, 1, 0, c->stream>>>(d);
   c->launches += 1;
-  launchContactStage(c, d, c->numSMs * searchBlocksPerSM(c));
+  launchContactStage(c, d);
   CK(cudaGetLastError());
   return SQDEM_OK;
 }
