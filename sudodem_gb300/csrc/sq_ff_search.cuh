@@ -151,9 +151,10 @@ __device__ __forceinline__ void ffCount(const Dev& d, unsigned long long ev, uns
 }
 
 template <bool FIRST>
-__global__ void __launch_bounds__(LM_BS, 4) k_ff_trial(Dev d, int round) {
+__global__ void __launch_bounds__(LM_BS, 4) k_ff_trial(Dev d, int round, int few) {
   __shared__ LMF sL[LM_BS / 2];
   const int n = FIRST ? d.S->lmCount + d.S->nmShort : d.Q->nT[round];
+  if (FIRST && n <= few) return;   // k_ff_warp takes them all
   const int* in = (round & 1) ? d.waveT1 : d.waveT0;
   int* next = (round & 1) ? d.waveT0 : d.waveT1;
   const int lane = threadIdx.x & 31;
@@ -245,10 +246,11 @@ __global__ void __launch_bounds__(LM_BS, 4) k_ff_probe(Dev d, int round) {
   ffCount(d, ev, deferred);
 }
 
-// One search per warp, sixteen points a round.  tail: the searches left after `rounds` rounds, else
-// the main queue.
-__global__ void __launch_bounds__(LM_BS, 4) k_ff_warp(Dev d, int tail, int rounds) {
+// One search per warp, sixteen points a round.  tail: the searches left after `rounds` rounds, unless
+// the main queue is no longer than `few`; else the main queue.
+__global__ void __launch_bounds__(LM_BS, 4) k_ff_warp(Dev d, int tail, int rounds, int few) {
   const unsigned FULL = 0xffffffffu;
+  if (tail && d.S->lmCount + d.S->nmShort <= few) tail = 0;
   const int lane = threadIdx.x & 31, grp = lane >> 1;
   const bool isB = lane & 1;
   const int trial = grp < 15 ? grp / 3 : 0, role = grp < 15 ? grp % 3 : 0;   // group 15 mirrors group 0

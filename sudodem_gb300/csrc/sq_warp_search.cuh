@@ -121,7 +121,8 @@ enum { WB_APART = 1, WB_FINITE = 2, WB_GAIN = 4, WB_SMALL = 8, WB_HUGE = 16 };
 //   WS_LONG      the long-search queue (fbQueue), its front first
 //   WS_DEFERRED  the searches the mixed form's double-float kernels deferred (deferQueue)
 //   WS_MAIN      the main queue (lmQueue), longest first
-//   WS_TAIL      the searches left after `rounds` rounds of k_wave_trial / k_wave_probe, from there on
+//   WS_TAIL      the searches left after `rounds` rounds of k_wave_trial / k_wave_probe, from there on;
+//                the main queue where it is no longer than `few`, which those leave alone
 enum { WS_LONG = 0, WS_DEFERRED = 1, WS_MAIN = 2, WS_TAIL = 3 };
 
 // W warps per search.  W = 1: blocks go to the SMs in turn, so that in blocks of one warp fewer
@@ -131,9 +132,10 @@ enum { WS_LONG = 0, WS_DEFERRED = 1, WS_MAIN = 2, WS_TAIL = 3 };
 // bound the stage and the pipes are otherwise idle (12,800 particles, mixed form: 18.3 -> 15.1 ms for
 // five steps; 1,583 in FP64: 3.46 -> 2.82 ms a step; 20,000 polydisperse: 11.1 -> 9.6 for three).
 template <int W>
-__global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_warp(Dev d, int mode, int waveRounds) {
+__global__ void __launch_bounds__(W == 1 ? LM_BS : 64, W == 1 ? 3 : 6) k_search_warp(Dev d, int mode, int waveRounds, int few) {
   const unsigned FULL = 0xffffffffu;
   const SceneState& S = *d.S;
+  if (mode == WS_TAIL && S.lmCount + S.nmShort <= few) mode = WS_MAIN;
   extern __shared__ WSlot wsSlots[];   // per search of the block: two rounds of WS_POINTS * W (wsShared)
   WSlot (*slots)[2][WS_POINTS * W] = reinterpret_cast<WSlot(*)[2][WS_POINTS * W]>(wsSlots);
   __shared__ int taken[W == 1 ? LM_BS / 32 : 1];

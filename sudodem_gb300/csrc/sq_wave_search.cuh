@@ -193,10 +193,11 @@ __device__ __forceinline__ void waveAppend(bool want, int i, int* list, int* cou
 }
 
 template <bool FIRST>
-__global__ void __launch_bounds__(LM_BS, 3) k_wave_trial(Dev d, int round) {
+__global__ void __launch_bounds__(LM_BS, 3) k_wave_trial(Dev d, int round, int few) {
   const SceneState& S = *d.S;
   const int nFront = S.lmCount;
   const int n = FIRST ? S.lmCount + S.nmShort : d.Q->nT[round];
+  if (FIRST && n <= few) return;   // k_search_warp takes them all
   const int* in = (round & 1) ? d.waveT1 : d.waveT0;
   int* next = (round & 1) ? d.waveT0 : d.waveT1;
   const int lane = threadIdx.x & 31;

@@ -2717,6 +2717,17 @@ static int ffRounds(const sqdem_ctx* c, const Dev& d) {
   return n <= FF_WARP_MAX ? 0 : std::min(WAVE_MAX_ROUNDS, (int)std::lround(std::log2(n / 1e3)));
 }
 
+// The main queue's length up to which each search takes a warp in large scenes too, decided by the
+// kernels (the rounds leave such a queue alone): one warp per scheduler holds them all at once.  A round
+// is an evaluation by two lanes, some 60 us however few searches share it, a warp's is 22.
+// Depositions, FP64: 17,000 particles, 4 searches: 0.42 ms a step in rounds, 0.24 by warps; 60,000, 23: 0.88, 0.46;
+// mixed form: 9,000, 4: 0.27, 0.21; 60,000, 23: 0.49, 0.37.  Lines at half, twice and four times this
+// length: the same within 2% there, in loose cells of 620-3,800 searches up to 6% less at four times.
+// In a batch the scene's share of it, so that all scenes' searches together are few.
+static int fewSearches(const sqdem_ctx* c, const Dev& d) {
+  return (int)(4ll * c->numSMs * d.NP / std::max(c->load, d.NP));
+}
+
 // Hertz-Mindlin model: rounds before the searches left get a warp each; none up to NM_WARP_MAX particles
 // (a packed lattice of 977: 0.86 ms a step, 1.06 in rounds; of 7,001: 1.28 and 1.40; of 20,000: 2.74
 // without rounds, 2.35 with four, 2.10 with six, 2.15 with ten).
@@ -2780,45 +2791,47 @@ static void launchContactStage(sqdem_ctx* c, const Dev& d) {
     if (c->precision == SQDEM_MIXED) {
       // the long searches in FP64 beside the double-float searches, then the searches the
       // double-float kernels deferred
-      if (n <= LONG_PAIR_MAX) k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0);
-      else k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0);
+      if (n <= LONG_PAIR_MAX) k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0, 0);
+      else k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0, 0);
       k_body_ff<<<nblk(d.N, 256), 256, 0, s>>>(d);
       const int blocks = c->numSMs * searchBlocksPerSM(c);
       const int ffw = std::min(blocks, nblk(d.Pcap, LM_BS / 32));
       const int rounds = ffRounds(c, d);
-      if (rounds == 0) k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 0, 0);
+      if (rounds == 0) k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 0, 0, 0);
       else {
         const int ff = std::min(blocks, nblk(d.Pcap, LM_BS / 2));
-        k_ff_trial<true><<<ff, LM_BS, 0, s>>>(d, 0);
+        const int few = fewSearches(c, d);
+        k_ff_trial<true><<<ff, LM_BS, 0, s>>>(d, 0, few);
         k_ff_probe<<<ff, LM_BS, 0, s>>>(d, 0);
         for (int r = 1; r < rounds; r++) {
-          k_ff_trial<false><<<ff, LM_BS, 0, s>>>(d, r);
+          k_ff_trial<false><<<ff, LM_BS, 0, s>>>(d, r, 0);
           k_ff_probe<<<ff, LM_BS, 0, s>>>(d, r);
         }
-        k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 1, rounds);
+        k_ff_warp<<<ffw, LM_BS, 0, s>>>(d, 1, rounds, few);
       }
       if (c->timingSearch) cudaEventRecord(c->ev[5], s);
       k_ff_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
-      k_search_warp<2><<<ws2, 64, wsShared(2, 64), s>>>(d, WS_DEFERRED, 0);
+      k_search_warp<2><<<ws2, 64, wsShared(2, 64), s>>>(d, WS_DEFERRED, 0, 0);
       join();
       if (c->timingSearch) cudaEventRecord(c->ev[6], s);
       c->launches += 6 + 2 * rounds;
     } else {
       if (n <= WARP_SEARCH_MAX) {
-        k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0);
-        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_MAIN, 0);
+        k_search_warp<2><<<ws2, 64, wsShared(2, 64), c->stream2>>>(d, WS_LONG, 0, 0);
+        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_MAIN, 0, 0);
         c->launches += 3;
       } else {
-        k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0);
+        k_search_warp<1><<<nblk(ws, LM_BS / 32), LM_BS, wsShared(1, LM_BS), c->stream2>>>(d, WS_LONG, 0, 0);
         const int wave = c->numSMs * searchBlocksPerSM(c);
-        k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0);
+        const int few = fewSearches(c, d);
+        k_wave_trial<true><<<wave, LM_BS, 0, s>>>(d, 0, few);
         k_wave_probe<<<wave, LM_BS, 0, s>>>(d, 0);
         const int rounds = waveRounds(c, d);
         for (int r = 1; r < rounds; r++) {
-          k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r);
+          k_wave_trial<false><<<wave, LM_BS, 0, s>>>(d, r, 0);
           k_wave_probe<<<wave, LM_BS, 0, s>>>(d, r);
         }
-        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_TAIL, rounds);
+        k_search_warp<1><<<ws, 32, wsShared(1, 32), s>>>(d, WS_TAIL, rounds, few);
         k_wave_finish<<<std::min(nblk(d.Pcap, 128), c->numSMs * 8), 128, 0, s>>>(d);
         c->launches += 4 + 2 * rounds;
       }

@@ -165,3 +165,37 @@ def test_report_counts_the_rounds_of_every_search(gpu, precision, small, large):
     lists = 3 * (4 if precision == "fp64" else 3)
     assert max(alone) > lists
     assert rep[word] >= max(alone)
+
+
+@pytest.mark.parametrize("precision,sizes", [("fp64", (700, 15400)), ("mixed", (700, 7400))])
+def test_few_searches_take_warps_in_large_scenes(gpu, precision, sizes):
+    """Loose scenes with a hundred touching pairs, in a batch above the particle line of the rounds: each search
+    takes a warp as it does in the scenes alone, so the longest takes as many rounds, with the same bits.  A
+    jammed scene beside them in the batch keeps its rounds, with the same bits too."""
+    per = 30
+    ss = [assemblies.walled_lattice(n, seed=51 + i, spacing=2.6e-3, r_range=(0.9e-3, 1.2e-3), per_side=per,
+                                    box=(per + 0.7) * 2.6e-3) for i, n in enumerate(sizes)]
+    word = "lm_rounds_max" if precision == "fp64" else "lm_rounds_max_ff"
+
+    def alone(spec, steps):
+        e = Engine(precision=precision)
+        e.load(spec)
+        e.step(steps)
+        return e.sync(), e
+
+    def together(specs, steps):
+        b = Batch(len(specs), precision=precision)
+        b.load(specs)
+        b.step(steps)
+        return b.sync(), b
+    rep, b = together(ss, 1)
+    b.close()
+    longest = max(alone(s, 1)[0][word] for s in ss)
+    assert longest > 0 and rep[word] == longest
+    ss.append(assemblies.cubic_specimen(900, seed=53, eps_range=(0.3, 1.7), spacing=2.1e-3, wall_gap=0.0))
+    _, b = together(ss, 6)
+    for i, spec in enumerate(ss):
+        _, e = alone(spec, 6)
+        assert np.array_equal(b.scenes[i].interactions(True), e.interactions(True)), i
+        assert np.array_equal(b.scenes[i].body_state(), e.body_state()), i
+    b.close()
