@@ -589,7 +589,8 @@ def run_ours(args):
                          "flops_per_evaluation": fpe,
                          "evaluation_rate": rate, "peak_evaluation_rate": peak_eval,
                          "evaluation_rate_frac": rate / peak_eval if peak_eval else None,
-                         "note": "Disfunction evaluations of the Levenberg-Marquardt searches dominate; flops per "
+                         "note": "Disfunction evaluations of the Levenberg-Marquardt searches dominate, those made ahead "
+                                 "for points a search then did not ask for included; flops per "
                                  "evaluation counted by ncu on the pipe-peak kernel that does nothing else"}
     cpu, ferr = None, None
     if rank == 0 and not args.no_cpu_baseline:

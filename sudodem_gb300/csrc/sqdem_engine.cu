@@ -2693,9 +2693,13 @@ static const int PASS1_BLOCKS_PER_SM = 16;   // grid-stride blocks of pass 1 per
 
 // FP64 form, where each search goes.  Up to WARP_SEARCH_MAX particles (of the scene, or of the batch
 // it steps in) every search takes a warp: 608 warps then run the stage in about the time of its
-// longest search (a jammed cell of 1,583 particles: 2.9 ms a step, 3.2 in rounds; of 9,000: 1.7
-// against 2.3).  Above it the rounds' full lanes win (43,011 particles: 6.3 ms against 15.5), until
-// few searches are left: a trial and a probe launch take 0.2 ms for up to some 3,500 searches, one
+// longest search (a jammed cell of 1,583 particles: 2.9 ms a step, 3.2 in rounds).  Above it the
+// rounds' full lanes win (a jammed cell of 43,011: 6.3 ms against 15.5).  The line is a compromise
+// between scenes with few searches per particle (polydisperse depositions of 9,000 and 15,800: 2.76 and
+// 2.98 ms a step by warps, 3.48 and 3.54 in rounds) and dense ones, for which it lies too high: jammed
+// cells of 4,001, 9,001 and 16,000 particles take 3.3, 4.9 and 7.6 ms by warps, 3.4, 3.8 and 4.3 in
+// rounds, servo specimens of 4,001 and 15,800 3.1 and 4.6, 3.4 and 3.7.  The rounds go on until few
+// searches are left: a trial and a probe launch take 0.2 ms for up to some 3,500 searches, one
 // warp each 0.24 ms per iteration of those, and their number falls with the iterations, so that
 // the number of rounds grows with the logarithm of the scene (43,011 particles: 6 rounds, 200,000:
 // 13; one third more or fewer rounds cost at most 2% there).
